@@ -427,122 +427,167 @@ __device__ void batch_tc_setup(Pass &ps, const dm_batch_tc_pass &bp, int n) {
     }
 }
 
-// One operation on a 64-coefficient column in shared memory (index j = d0 +
-// 4 d1 + 16 d2 over the round's digits; digit positions from the op flags),
-// in FP64: the same maps as the register rounds, with runtime digits.
+// Round r's matrix U (64 x 64 in its K-digit order) is the round's operations
+// applied to the 64 unit vectors: column k of U = ops(e_k), composed in FP64
+// in shared memory and written as the FP16 images that the MMAs read, K-major
+// (value (n%8)*8 + k%8 + (k/8)*64 + (n/8)*512 for output n, input k), with
+// Uh = fp16(U) and Ul = fp16(2**11 (U - Uh)): three images 2**11 Uh | Ul | Uh
+// for the cp.async-fed kernels, two images Uh | Ul for the TMA-fed one.
+//
+// What bounds it is the FP64 pipe (two FMAs per clock and SM) and, before
+// this form, the latency of one thread per column.  So one warp owns 8
+// columns (index j = d0 + 4 d1 + 16 d2 of column c at c * kColStride + j; no
+// block barrier between operations), its lanes sharing each operation's
+// independent groups; the 4x4 maps that come before the round's first pair
+// operation form a Kronecker product and are written as such (two products
+// per entry instead of 16 FMAs per four entries and map); and a map whose I
+// row is (1,0,0,0), whose X and Y rows take no I, costs 10 FMAs per four
+// entries instead of 16.  The 8 columns of a warp are the 8 halves of one
+// 16-byte chunk per row of an image.  Measured with one column per thread and
+// now: a recorded 20-layer circuit of 10 qubits (20 passes) 1,314 -> 612 us,
+// the 14-qubit QFT with 2 layers (24 passes) 15.63 -> 14.07 ms.
+constexpr int kColStride = 65;   // doubles per column: a warp's lanes spread over the banks
+constexpr int kColsPerWarp = 8;
+constexpr int kColBytes = 64 * kColStride * 8;   // one round's columns
+static_assert(kColBytes <= int(kSmemBytes), "one round of FP64 columns fits the pass's shared memory");
+
+// One operation on the warp's 8 columns (digit positions from the op flags).
 // Map2: 16x16 general maps too (the single-state passes; the batched plans hold none).
 template <bool Map2>
-__device__ void col_apply(double *col, const dm_op &op, const double *__restrict__ mats) {
+__device__ __forceinline__ void cols_apply(double *w, const dm_op &op, const double *__restrict__ mats, int lane) {
     const double *mg = mats + op.moff;
     const int da = (op.flags >> 8) & 3, db = (op.flags >> 12) & 3;
     if (op.kind == DM_OP_MAP1) {
         double m[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) m[i] = mg[i];
+        const bool row0 = m[0] == 1.0 && m[1] == 0.0 && m[2] == 0.0 && m[3] == 0.0;
+        const bool xy = row0 && m[4] == 0.0 && m[8] == 0.0;
         const int S = 1 << (2 * da);
-#pragma unroll 1
-        for (int o = 0; o < 16; ++o) {
-            const int j0 = ((o >> (2 * da)) << (2 * da + 2)) | (o & (S - 1));
-            double x0 = col[j0], x1 = col[j0 + S], x2 = col[j0 + 2 * S], x3 = col[j0 + 3 * S];
-            map4(m, false, x0, x1, x2, x3);
-            col[j0] = x0;
-            col[j0 + S] = x1;
-            col[j0 + 2 * S] = x2;
-            col[j0 + 3 * S] = x3;
+        const int g = lane & 15;
+        const int j0 = ((g >> (2 * da)) << (2 * da + 2)) | (g & (S - 1));
+        double *col = w + (lane >> 4) * kColStride + j0;
+#pragma unroll
+        for (int it = 0; it < kColsPerWarp / 2; ++it) {
+            double *x = col + 2 * it * kColStride;
+            double x0 = x[0], x1 = x[S], x2 = x[2 * S], x3 = x[3 * S];
+            if (xy) {
+                map4_tp_xy(m, x0, x1, x2, x3);
+            } else {
+                map4(m, row0, x0, x1, x2, x3);
+                x[0] = x0;
+            }
+            x[S] = x1;
+            x[2 * S] = x2;
+            x[3 * S] = x3;
         }
         return;
     }
+    // pair operations: lane = (column, value of the third digit)
     const int SA = 1 << (2 * da), SB = 1 << (2 * db), SC = 1 << (2 * (3 - da - db));
-    CxCoef<double> cx{1.0, 0.0, 1.0, 0.0, 0.0};
-    const bool ideal = (op.flags & DM_CX_IDEAL) != 0;
-    if (op.kind == DM_OP_CX && !ideal) cx = CxCoef<double>{mg[0], mg[1], mg[2], mg[3], mg[4]};
+    double *col = w + (lane >> 2) * kColStride + (lane & 3) * SC;
+    double x[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) x[i] = col[(i >> 2) * SA + (i & 3) * SB];
+    if (Map2 && op.kind == DM_OP_MAP2) {   // y[4 pa + pb] = sum_s mg[16 (4 pa + pb) + s] x[s]
 #pragma unroll 1
-    for (int o = 0; o < 4; ++o) {   // the four groups of the third digit
-        const int j0 = o * SC;
-        double x[16];
+        for (int i = 0; i < 16; ++i) {
+            double acc = 0.0;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) x[i] = col[j0 + (i >> 2) * SA + (i & 3) * SB];
-        if (Map2 && op.kind == DM_OP_MAP2) {   // y[4 pa + pb] = sum_s mg[16 (4 pa + pb) + s] x[s]
-#pragma unroll 1
-            for (int i = 0; i < 16; ++i) {
-                double acc = 0.0;
-#pragma unroll
-                for (int j = 0; j < 16; ++j) acc = fma(mg[16 * i + j], x[j], acc);
-                col[j0 + (i >> 2) * SA + (i & 3) * SB] = acc;
-            }
-            continue;
+            for (int j = 0; j < 16; ++j) acc = fma(mg[16 * i + j], x[j], acc);
+            col[(i >> 2) * SA + (i & 3) * SB] = acc;
         }
-        if (op.kind == DM_OP_CX) {
-            cx16(x, cx, ideal);
-        } else {   // DM_OP_DIAG2: entry (pa, pb) scaled by mg[4 pa + pb]
-#pragma unroll
-            for (int i = 0; i < 16; ++i) x[i] *= mg[i];
-        }
-#pragma unroll
-        for (int i = 0; i < 16; ++i) col[j0 + (i >> 2) * SA + (i & 3) * SB] = x[i];
+        return;
     }
+    if (op.kind == DM_OP_CX) {
+        CxCoef<double> cx{1.0, 0.0, 1.0, 0.0, 0.0};
+        const bool ideal = (op.flags & DM_CX_IDEAL) != 0;
+        if (!ideal) cx = CxCoef<double>{mg[0], mg[1], mg[2], mg[3], mg[4]};
+        cx16(x, cx, ideal);
+    } else {   // DM_OP_DIAG2: entry (pa, pb) scaled by mg[4 pa + pb]
+#pragma unroll
+        for (int i = 0; i < 16; ++i) x[i] *= mg[i];
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) col[(i >> 2) * SA + (i & 3) * SB] = x[i];
 }
 
-// Round r's matrix U (64 x 64 in its K-digit order) is the round's operations
-// applied to the 64 unit vectors: column k of U = ops(e_k), composed in FP64
-// on a column held in shared memory, one thread per column.  Written as FP16
-// images that the MMAs read, K-major (value (n%8)*8 + k%8 + (k/8)*64 +
-// (n/8)*512 for output n, input k), with Uh = fp16(U) and
-// Ul = fp16(2**11 (U - Uh)): three images 2**11 Uh | Ul | Uh for the
-// cp.async-fed kernels, two images Uh | Ul for the TMA-fed one.
-constexpr int kColStride = 65;   // doubles per column: a warp's 32 columns spread over the banks
-static_assert(2 * 64 * kColStride * 8 <= int(kSmemBytes), "two rounds of FP64 columns fit the pass's shared memory");
-
+// Columns k0 .. k0 + 7 of round r (k0 a multiple of 8) by one warp, w its 8 columns of scratch;
+// the round's images at img (three or two of them).
 template <bool Map2>
-__device__ void compose_column(const dm_batch_pass &bp, int r, int k, const double *__restrict__ mats, double *col) {
-#pragma unroll 1
-    for (int j = 0; j < 64; ++j) col[j] = j == k ? 1.0 : 0.0;
-    const int ob = r > 0 ? bp.round_end[r - 1] : 0, oe = bp.round_end[r];
-    for (int o = ob; o < oe; ++o) col_apply<Map2>(col, bp.ops[o], mats);
-}
-
-__device__ void write_column(uint16_t *__restrict__ img, int k, const double *col, bool three) {
-    const uint32_t kpos = uint32_t(k & 7) + uint32_t(k >> 3) * 64;
-    const int uh = three ? 8192 : 0;   // three: 2**11 Uh at 0, Ul at 4096, Uh at 8192; two: Uh at 0, Ul at 4096
-#pragma unroll 4
-    for (int j = 0; j < 64; ++j) {
-        const uint32_t pos = kpos + uint32_t(j & 7) * 8 + uint32_t(j >> 3) * 512;
-        const double u = col[j];
-        const __half h = __double2half(u);
-        const double hd = double(__half2float(h));
-        if (three) img[pos] = __half_as_ushort(__float2half_rn(float(hd * double(kLoScale))));
-        img[4096 + pos] = __half_as_ushort(__double2half((u - hd) * double(kLoScale)));
-        img[uh + pos] = __half_as_ushort(h);
+__device__ void compose_warp(const dm_batch_pass &bp, int r, int k0, const double *__restrict__ mats, double *w,
+                             uint16_t *__restrict__ img, bool three, int lane) {
+    int o = r > 0 ? bp.round_end[r - 1] : 0;
+    const int oe = bp.round_end[r];
+    // the leading 4x4 maps, at most one per digit: their Kronecker product
+    const double *lead[3] = {nullptr, nullptr, nullptr};
+    for (; o < oe && bp.ops[o].kind == DM_OP_MAP1; ++o) {
+        const int d = (bp.ops[o].flags >> 8) & 3;
+        if (d == 0 ? lead[0] != nullptr : d == 1 ? lead[1] != nullptr : lead[2] != nullptr) break;
+        const double *m = mats + bp.ops[o].moff;
+        if (d == 0) lead[0] = m;
+        else if (d == 1) lead[1] = m;
+        else lead[2] = m;
     }
+#pragma unroll
+    for (int it = 0; it < 2 * kColsPerWarp; ++it) {   // lane's rows j of column c
+        const int c = it >> 1, j = lane + 32 * (it & 1), k = k0 + c;
+        const double f0 = lead[0] ? lead[0][4 * (j & 3) + (k & 3)] : ((j ^ k) & 3 ? 0.0 : 1.0);
+        const double f1 = lead[1] ? lead[1][4 * ((j >> 2) & 3) + ((k >> 2) & 3)] : ((j ^ k) & 12 ? 0.0 : 1.0);
+        const double f2 = lead[2] ? lead[2][4 * (j >> 4) + (k >> 4)] : ((j ^ k) & 48 ? 0.0 : 1.0);
+        w[c * kColStride + j] = f2 * f1 * f0;
+    }
+    __syncwarp();
+    for (; o < oe; ++o) {
+        cols_apply<Map2>(w, bp.ops[o], mats, lane);
+        __syncwarp();
+    }
+    // row j of the 8 columns: one 16-byte chunk per image
+    const int uh = three ? 8192 : 0;   // three: 2**11 Uh at 0, Ul at 4096, Uh at 8192; two: Uh at 0, Ul at 4096
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        const int j = lane + 32 * half;
+        const uint32_t pos = uint32_t(k0 >> 3) * 64 + uint32_t(j & 7) * 8 + uint32_t(j >> 3) * 512;
+        uint32_t h2[4], l2[4], s2[4];
+#pragma unroll
+        for (int c = 0; c < kColsPerWarp; c += 2) {
+            const double u0 = w[c * kColStride + j], u1 = w[(c + 1) * kColStride + j];
+            const __half h0 = __double2half(u0), h1 = __double2half(u1);
+            const float f0 = __half2float(h0), f1 = __half2float(h1);
+            const __half l0 = __double2half((u0 - double(f0)) * double(kLoScale));
+            const __half l1 = __double2half((u1 - double(f1)) * double(kLoScale));
+            h2[c >> 1] = uint32_t(__half_as_ushort(h0)) | (uint32_t(__half_as_ushort(h1)) << 16);
+            l2[c >> 1] = uint32_t(__half_as_ushort(l0)) | (uint32_t(__half_as_ushort(l1)) << 16);
+            s2[c >> 1] = uint32_t(__half_as_ushort(__float2half_rn(f0 * kLoScale))) |
+                         (uint32_t(__half_as_ushort(__float2half_rn(f1 * kLoScale))) << 16);
+        }
+        if (three) *reinterpret_cast<uint4 *>(img + pos) = make_uint4(s2[0], s2[1], s2[2], s2[3]);
+        *reinterpret_cast<uint4 *>(img + 4096 + pos) = make_uint4(l2[0], l2[1], l2[2], l2[3]);
+        *reinterpret_cast<uint4 *>(img + uh + pos) = make_uint4(h2[0], h2[1], h2[2], h2[3]);
+    }
+    __syncwarp();   // the columns are read before the next round's are written
 }
 
-// All rounds of a batched pass into per-CTA scratch (three images per round),
-// 128 threads, two rounds at a time; the pass's operand and matrix regions
-// are free between passes.
+// All rounds of a batched pass into per-CTA scratch (three images per round), all threads of the
+// CTA, each warp its 8 columns; the pass's operand and matrix regions are free between passes.
+static_assert(kThreads / 32 * kColsPerWarp == 64, "the CTA's warps cover the 64 columns");
 __device__ void compose_rounds(const dm_batch_pass &bp, const double *__restrict__ mats, uint16_t *__restrict__ umats,
                                double *work) {
-    const int nr = bp.nrounds;
-    const int tid = threadIdx.x;
-    if (tid >= 128) return;
-    double *col = work + tid * kColStride;
-    for (int r0 = 0; r0 < nr; r0 += 2) {
-        const int r = r0 + (tid >> 6), k = tid & 63;
-        if (r >= nr) break;
-        compose_column<false>(bp, r, k, mats, col);
-        write_column(umats + int64_t(r) * kUHalves, k, col, true);
-    }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int r = 0; r < bp.nrounds; ++r)
+        compose_warp<false>(bp, r, warp * kColsPerWarp, mats, work + warp * kColsPerWarp * kColStride,
+                            umats + int64_t(r) * kUHalves, true, lane);
 }
 
-// One pass's round images for the single-state kernels: one CTA per round,
-// one thread per column.
-__global__ void __launch_bounds__(64)
+// One pass's round images for the single-state kernels: one warp per CTA, CTA (r, c) the columns
+// 8c .. 8c + 7 of round r, so that a pass's FP64 work spreads over 8 SMs per round.
+__global__ void __launch_bounds__(32)
     compose_pass_kernel(const __grid_constant__ dm_batch_pass bp, const double *__restrict__ mats,
                         uint16_t *__restrict__ images, int image_halves) {
-    __shared__ double cols[64 * kColStride];
-    const int r = blockIdx.x, k = threadIdx.x;
-    double *col = cols + k * kColStride;
-    compose_column<true>(bp, r, k, mats, col);
-    write_column(images + int64_t(r) * image_halves, k, col, image_halves == kUHalves);
+    __shared__ double cols[kColsPerWarp * kColStride];
+    const int r = blockIdx.x, k0 = int(blockIdx.y) * kColsPerWarp;
+    compose_warp<true>(bp, r, k0, mats, cols, images + int64_t(r) * image_halves, image_halves == kUHalves,
+                       threadIdx.x);
 }
 
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
@@ -588,7 +633,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
 // into shared memory, the round matrices composed from those coefficients,
 // then the tiles streamed.  Slot s of the program is op s of the
 // concatenated tensor-core passes; op o of a pass reads coef + 16 o.
-constexpr int kCoefOffset = 2 * 64 * kColStride * 8;   // after the two rounds of FP64 columns
+constexpr int kCoefOffset = kColBytes;   // after the round of FP64 columns
 static_assert(kCoefOffset + DM_MAX_PASS_OPS * kCoefStride * 8 <= int(kSmemBytes), "slot coefficients fit");
 
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
@@ -825,7 +870,7 @@ extern "C" int dm_compose_rounds(int format, const dm_batch_pass *pass, const do
     if (rc) return rc;
     const int halves = format == DM_IMAGE_TC ? tc::kUHalves : 2 * 4096;
     if (images_count < size_t(pass->nrounds) * size_t(halves)) return DM_ERR_ARG;
-    tc::compose_pass_kernel<<<pass->nrounds, 64, 0, as_stream(stream)>>>(*pass, mats_dev, images_dev, halves);
+    tc::compose_pass_kernel<<<dim3(pass->nrounds, 64 / tc::kColsPerWarp), 32, 0, as_stream(stream)>>>(*pass, mats_dev, images_dev, halves);
     count_launch();
     return launch_status();
 }
