@@ -18,7 +18,7 @@ CSRC = os.path.join(PKG_DIR, 'csrc')
 INCLUDE = os.path.join(REPO_DIR, 'include')
 BUILD_DIR = os.path.join(PKG_DIR, '_build')
 LIB_PATH = os.path.join(PKG_DIR, 'libdmgb300.so')
-SOURCES = ['dm_misc.cu', 'dm_pass.cu', 'dm_state.cu', 'dm_measure.cu', 'dm_tc.cu', 'dm_tma.cu', 'dm_mlp.cu',
+SOURCES = ['dm_misc.cu', 'dm_pass.cu', 'dm_noise.cu', 'dm_state.cu', 'dm_measure.cu', 'dm_tc.cu', 'dm_tma.cu', 'dm_mlp.cu',
            'dm_sample.cu', 'dm_sched.cpp']
 ARCH = ['-gencode', 'arch=compute_103a,code=sm_103a']
 NVCC_FLAGS = ['-O3', '-std=c++17', '-lineinfo', '-Xcompiler', '-fPIC', '-Xptxas', '-warn-spills',

@@ -29,21 +29,84 @@ struct Mat4 {
 
 // ---------------------------------------------------------------------------
 // single-operation sweeps
+//
+// FP32 sweeps are bound by HBM, FP64 sweeps by the FP64 pipe (two FMAs per
+// clock and SM; the dense 4x4 map's 16 FMAs per four coefficients are 2.6
+// times the sweep's HBM time).  So a map is classified by its zeros on the
+// host: a rotation neither reads nor writes the I quarter of the state (3/4
+// of the traffic) and costs 9 FMAs per four coefficients, a
+// trace-preserving unital-XY map 10.  CX leaves 4 of its 16 entries alone
+// and neither reads nor writes them.  Threads move 16-byte vectors along the
+// contiguous direction; a state that is not 16-byte aligned takes the
+// element-wise form (Vec = false).
 // ---------------------------------------------------------------------------
 
-template <typename T>
-__global__ void __launch_bounds__(256) map1_kernel(T *__restrict__ st, int log4s, int64_t ngroups,
-                                                   Mat4<T> m, int row0_id) {
+enum MapKind { kMapDense, kMapRow0, kMapTpXy, kMapRotation };
+
+static MapKind map_kind(const double *m) {
+    if (!(m[0] == 1.0 && m[1] == 0.0 && m[2] == 0.0 && m[3] == 0.0)) return kMapDense;
+    if (!(m[4] == 0.0 && m[8] == 0.0)) return kMapRow0;
+    return m[12] == 0.0 ? kMapRotation : kMapTpXy;
+}
+
+template <typename T, int Kind>
+__device__ __forceinline__ void map_kinds(const T *m, T &x0, T &x1, T &x2, T &x3) {
+    if constexpr (Kind == kMapDense || Kind == kMapRow0) {
+        map4<Kind == kMapRow0>(m, x0, x1, x2, x3);
+    } else if constexpr (Kind == kMapTpXy) {
+        map4_tp_xy(m, x0, x1, x2, x3);
+    } else {
+        const T y1 = fma(m[5], x1, fma(m[6], x2, m[7] * x3));
+        const T y2 = fma(m[9], x1, fma(m[10], x2, m[11] * x3));
+        const T y3 = fma(m[13], x1, fma(m[14], x2, m[15] * x3));
+        x1 = y1;
+        x2 = y2;
+        x3 = y3;
+    }
+}
+
+// 16 bytes of coefficients (one coefficient when the state is not aligned)
+template <typename T, bool Vec>
+struct alignas(Vec ? 16 : alignof(T)) Pack {
+    static constexpr int N = Vec ? 16 / int(sizeof(T)) : 1;
+    T v[N];
+};
+
+// Axes above the contiguous one (or any axis, element by element).
+template <typename T, int Kind, bool Vec>
+__global__ void __launch_bounds__(256) map1_kernel(T *__restrict__ st, int log4s, int64_t npacks, const Mat4<T> m) {
+    using P = Pack<T, Vec>;
     const int64_t s = int64_t(1) << (2 * log4s);
-    for (int64_t g = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; g < ngroups;
-         g += int64_t(gridDim.x) * blockDim.x) {
-        const int64_t i0 = ((g >> (2 * log4s)) << (2 * log4s + 2)) | (g & (s - 1));
-        T x0 = st[i0], x1 = st[i0 + s], x2 = st[i0 + 2 * s], x3 = st[i0 + 3 * s];
-        map4(m.m, row0_id != 0, x0, x1, x2, x3);
-        st[i0] = x0;
-        st[i0 + s] = x1;
-        st[i0 + 2 * s] = x2;
-        st[i0 + 3 * s] = x3;
+    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < npacks;
+         i += int64_t(gridDim.x) * blockDim.x) {
+        const int64_t g = i * P::N;
+        T *at = st + (((g >> (2 * log4s)) << (2 * log4s + 2)) | (g & (s - 1)));
+        P x0{}, x1, x2, x3;
+        if constexpr (Kind != kMapRotation) x0 = *reinterpret_cast<const P *>(at);
+        x1 = *reinterpret_cast<const P *>(at + s);
+        x2 = *reinterpret_cast<const P *>(at + 2 * s);
+        x3 = *reinterpret_cast<const P *>(at + 3 * s);
+#pragma unroll
+        for (int e = 0; e < P::N; ++e) map_kinds<T, Kind>(m.m, x0.v[e], x1.v[e], x2.v[e], x3.v[e]);
+        if constexpr (Kind == kMapDense) *reinterpret_cast<P *>(at) = x0;
+        *reinterpret_cast<P *>(at + s) = x1;
+        *reinterpret_cast<P *>(at + 2 * s) = x2;
+        *reinterpret_cast<P *>(at + 3 * s) = x3;
+    }
+}
+
+// The contiguous axis: a group is four adjacent coefficients.
+template <typename T, int Kind>
+__global__ void __launch_bounds__(256) map1_low_kernel(T *__restrict__ st, int64_t ngroups, const Mat4<T> m) {
+    struct alignas(16) Group {
+        T v[4];
+    };
+    Group *st4 = reinterpret_cast<Group *>(st);
+    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < ngroups;
+         i += int64_t(gridDim.x) * blockDim.x) {
+        Group x = st4[i];
+        map_kinds<T, Kind>(m.m, x.v[0], x.v[1], x.v[2], x.v[3]);
+        st4[i] = x;
     }
 }
 
@@ -52,25 +115,66 @@ __device__ __forceinline__ int64_t insert_zero_digit(int64_t g, int pos) {
     return ((g >> (2 * pos)) << (2 * pos + 2)) | low;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256) cx_kernel(T *__restrict__ st, int pos_c, int pos_t, int64_t ngroups,
-                                                 CxCoef<T> k, int ideal) {
+// entries of a CX pair group that the map changes (index 4 * control + target)
+__device__ __forceinline__ constexpr bool cx_moves(int i) { return i != 0 && i != 1 && i != 12 && i != 13; }
+
+// Both qubits above the contiguous axis (or any pair, element by element).
+template <typename T, bool Vec>
+__global__ void __launch_bounds__(256) cx_kernel(T *__restrict__ st, int pos_c, int pos_t, int64_t npacks,
+                                                 const CxCoef<T> k, int ideal) {
+    using P = Pack<T, Vec>;
     const int lo = pos_c < pos_t ? pos_c : pos_t;
     const int hi = pos_c < pos_t ? pos_t : pos_c;
     const int64_t sc = int64_t(1) << (2 * pos_c), stt = int64_t(1) << (2 * pos_t);
+    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < npacks;
+         i += int64_t(gridDim.x) * blockDim.x) {
+        T *at = st + insert_zero_digit(insert_zero_digit(i * P::N, lo), hi);
+        P x[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+            if (cx_moves(j)) x[j] = *reinterpret_cast<const P *>(at + (j >> 2) * sc + (j & 3) * stt);
+#pragma unroll
+        for (int e = 0; e < P::N; ++e) {
+            T y[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) y[j] = cx_moves(j) ? x[j].v[e] : T(0);
+            cx16(y, k, ideal != 0);
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+                if (cx_moves(j)) x[j].v[e] = y[j];
+        }
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+            if (cx_moves(j)) *reinterpret_cast<P *>(at + (j >> 2) * sc + (j & 3) * stt) = x[j];
+    }
+}
+
+// One qubit of the pair on the contiguous axis: four rows of four adjacent coefficients.
+template <typename T, bool ControlLow>
+__global__ void __launch_bounds__(256) cx_low_kernel(T *__restrict__ st, int hi, int64_t ngroups, const CxCoef<T> k,
+                                                     int ideal) {
+    struct alignas(16) Row {
+        T v[4];
+    };
+    const int64_t s = int64_t(1) << (2 * hi);
     for (int64_t g = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; g < ngroups;
          g += int64_t(gridDim.x) * blockDim.x) {
-        const int64_t i0 = insert_zero_digit(insert_zero_digit(g, lo), hi);
+        T *at = st + insert_zero_digit(insert_zero_digit(g, 0), hi);
         T x[16];
 #pragma unroll
-        for (int pc = 0; pc < 4; ++pc)
+        for (int h = 0; h < 4; ++h) {
+            const Row r = *reinterpret_cast<const Row *>(at + h * s);
 #pragma unroll
-            for (int pt = 0; pt < 4; ++pt) x[4 * pc + pt] = st[i0 + pc * sc + pt * stt];
+            for (int l = 0; l < 4; ++l) x[ControlLow ? 4 * l + h : 4 * h + l] = r.v[l];
+        }
         cx16(x, k, ideal != 0);
 #pragma unroll
-        for (int pc = 0; pc < 4; ++pc)
+        for (int h = 0; h < 4; ++h) {
+            Row r;
 #pragma unroll
-            for (int pt = 0; pt < 4; ++pt) st[i0 + pc * sc + pt * stt] = x[4 * pc + pt];
+            for (int l = 0; l < 4; ++l) r.v[l] = x[ControlLow ? 4 * l + h : 4 * h + l];
+            *reinterpret_cast<Row *>(at + h * s) = r;
+        }
     }
 }
 
@@ -101,7 +205,10 @@ __device__ void tile_map1(T *tile, int k, int r, const T *__restrict__ mg, bool 
     for (int g = threadIdx.x; g < ng; g += blockDim.x) {
         const int i0 = ((g >> (2 * r)) << (2 * r + 2)) | (g & (s - 1));
         T x0 = tile[i0], x1 = tile[i0 + s], x2 = tile[i0 + 2 * s], x3 = tile[i0 + 3 * s];
-        map4(m, row0_id, x0, x1, x2, x3);
+        if (row0_id)
+            map4<true>(m, x0, x1, x2, x3);
+        else
+            map4<false>(m, x0, x1, x2, x3);
         tile[i0] = x0;
         tile[i0 + s] = x1;
         tile[i0 + 2 * s] = x2;
@@ -531,14 +638,30 @@ extern "C" int dm_apply_pass(void *state_dev, int n, int dtype, const dm_pass *p
                        as_stream(stream));
 }
 
+template <typename T, int Kind>
+static void launch_map1(T *st, int n, int log4s, const Mat4<T> &m, cudaStream_t s) {
+    const int64_t ngroups = pow4(n - 1);
+    if (reinterpret_cast<uintptr_t>(st) & 15) {
+        map1_kernel<T, Kind, false><<<grid_for(ngroups, 256), 256, 0, s>>>(st, log4s, ngroups, m);
+    } else if (log4s == 0) {
+        map1_low_kernel<T, Kind><<<grid_for(ngroups, 256), 256, 0, s>>>(st, ngroups, m);
+    } else {
+        const int64_t npacks = ngroups / Pack<T, true>::N;
+        map1_kernel<T, Kind, true><<<grid_for(npacks, 256), 256, 0, s>>>(st, log4s, npacks, m);
+    }
+}
+
 template <typename T>
 static int do_map1(void *state_dev, int n, int q, const double *m4x4, cudaStream_t s) {
     Mat4<T> m;
     for (int i = 0; i < 16; ++i) m.m[i] = T(m4x4[i]);
-    const bool row0_id = m4x4[0] == 1.0 && m4x4[1] == 0.0 && m4x4[2] == 0.0 && m4x4[3] == 0.0;
-    const int64_t ngroups = pow4(n - 1);
-    map1_kernel<T><<<grid_for(ngroups, 256), 256, 0, s>>>(static_cast<T *>(state_dev), n - 1 - q, ngroups, m,
-                                                          row0_id ? 1 : 0);
+    T *st = static_cast<T *>(state_dev);
+    switch (map_kind(m4x4)) {
+        case kMapRotation: launch_map1<T, kMapRotation>(st, n, n - 1 - q, m, s); break;
+        case kMapTpXy: launch_map1<T, kMapTpXy>(st, n, n - 1 - q, m, s); break;
+        case kMapRow0: launch_map1<T, kMapRow0>(st, n, n - 1 - q, m, s); break;
+        default: launch_map1<T, kMapDense>(st, n, n - 1 - q, m, s); break;
+    }
     count_launch();
     return launch_status();
 }
@@ -567,9 +690,19 @@ static int do_cx(void *state_dev, int n, int qc, int qt, const double *err, cuda
     bool ideal;
     cx_coefficients(err, c5, &ideal);
     CxCoef<T> k{T(c5[0]), T(c5[1]), T(c5[2]), T(c5[3]), T(c5[4])};
+    T *st = static_cast<T *>(state_dev);
+    const int pc = n - 1 - qc, pt = n - 1 - qt;
     const int64_t ngroups = pow4(n - 2);
-    cx_kernel<T><<<grid_for(ngroups, 256), 256, 0, s>>>(static_cast<T *>(state_dev), n - 1 - qc, n - 1 - qt,
-                                                        ngroups, k, ideal ? 1 : 0);
+    if (reinterpret_cast<uintptr_t>(st) & 15) {
+        cx_kernel<T, false><<<grid_for(ngroups, 256), 256, 0, s>>>(st, pc, pt, ngroups, k, ideal ? 1 : 0);
+    } else if (pc == 0) {
+        cx_low_kernel<T, true><<<grid_for(ngroups, 256), 256, 0, s>>>(st, pt, ngroups, k, ideal ? 1 : 0);
+    } else if (pt == 0) {
+        cx_low_kernel<T, false><<<grid_for(ngroups, 256), 256, 0, s>>>(st, pc, ngroups, k, ideal ? 1 : 0);
+    } else {
+        const int64_t npacks = ngroups / Pack<T, true>::N;
+        cx_kernel<T, true><<<grid_for(npacks, 256), 256, 0, s>>>(st, pc, pt, npacks, k, ideal ? 1 : 0);
+    }
     count_launch();
     return launch_status();
 }
@@ -580,18 +713,6 @@ extern "C" int dm_apply_cx(void *state_dev, int n, int dtype, int qc, int qt, co
     DM_CHECK_ARG(n >= 2 && qc >= 0 && qt >= 0 && qc < n && qt < n && qc != qt);
     return dtype == DM_F64 ? do_cx<double>(state_dev, n, qc, qt, tsp_err2, as_stream(stream))
                            : do_cx<float>(state_dev, n, qc, qt, tsp_err2, as_stream(stream));
-}
-
-extern "C" int dm_apply_memory_noise(void *state_dev, int n, int dtype, double f, double p, double g,
-                                     void *stream) {
-    DM_CHECK_ARG(state_dev && valid_n(n) && valid_dtype(dtype));
-    const double k = sqrt(g) * f, d = (1 - g) * (2 * p - 1);
-    const double m[16] = {1, 0, 0, 0, 0, k, 0, 0, 0, 0, k, 0, d, 0, 0, g};
-    for (int q = 0; q < n; ++q) {
-        int rc = dm_apply_map1(state_dev, n, dtype, q, m, stream);
-        if (rc) return rc;
-    }
-    return DM_OK;
 }
 
 // ---------------------------------------------------------------------------

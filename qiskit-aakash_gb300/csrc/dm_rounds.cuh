@@ -14,9 +14,11 @@ struct CxCoef {
     T c, s, c2, s2, cs;
 };
 
-template <typename T>
-__device__ __forceinline__ void map4(const T *m, bool row0_id, T &x0, T &x1, T &x2, T &x3) {
-    T y0 = row0_id ? x0 : fma(m[0], x0, fma(m[1], x1, fma(m[2], x2, m[3] * x3)));
+// Row0: row 0 of the map is (1,0,0,0).  A compile-time choice: as a run-time one the compiler
+// computes row 0 anyway and selects, a quarter of the map's FP64 operations.
+template <bool Row0, typename T>
+__device__ __forceinline__ void map4(const T *m, T &x0, T &x1, T &x2, T &x3) {
+    const T y0 = Row0 ? x0 : fma(m[0], x0, fma(m[1], x1, fma(m[2], x2, m[3] * x3)));
     T y1 = fma(m[4], x0, fma(m[5], x1, fma(m[6], x2, m[7] * x3)));
     T y2 = fma(m[8], x0, fma(m[9], x1, fma(m[10], x2, m[11] * x3)));
     T y3 = fma(m[12], x0, fma(m[13], x1, fma(m[14], x2, m[15] * x3)));
@@ -90,10 +92,18 @@ __device__ __forceinline__ void reg_map1(T (&v)[1 << (2 * R)], const T *__restri
         }
         return;
     }
+    if (row0_id) {
+#pragma unroll
+        for (int o = 0; o < (1 << (2 * (R - 1))); ++o) {
+            const int j0 = ((o >> (2 * D)) << (2 * D + 2)) | (o & (S - 1));
+            map4<true>(m, v[j0], v[j0 + S], v[j0 + 2 * S], v[j0 + 3 * S]);
+        }
+        return;
+    }
 #pragma unroll
     for (int o = 0; o < (1 << (2 * (R - 1))); ++o) {
         const int j0 = ((o >> (2 * D)) << (2 * D + 2)) | (o & (S - 1));
-        map4(m, row0_id, v[j0], v[j0 + S], v[j0 + 2 * S], v[j0 + 3 * S]);
+        map4<false>(m, v[j0], v[j0 + S], v[j0 + 2 * S], v[j0 + 3 * S]);
     }
 }
 

@@ -473,8 +473,10 @@ __device__ __forceinline__ void cols_apply(double *w, const dm_op &op, const dou
             double x0 = x[0], x1 = x[S], x2 = x[2 * S], x3 = x[3 * S];
             if (xy) {
                 map4_tp_xy(m, x0, x1, x2, x3);
+            } else if (row0) {
+                map4<true>(m, x0, x1, x2, x3);
             } else {
-                map4(m, row0, x0, x1, x2, x3);
+                map4<false>(m, x0, x1, x2, x3);
                 x[0] = x0;
             }
             x[S] = x1;
