@@ -282,7 +282,8 @@ def time_replays(torch, state, steps):
 
 
 PASS_KERNELS = {'dm_apply_pass': 'pass_pipe_kernel', 'dm_apply_pass_tc': 'pass_tc_kernel',
-                'dm_apply_pass_tma': 'pass_tma_kernel', 'dm_compose_rounds': 'compose_pass_kernel'}
+                'dm_apply_pass_tma': 'pass_tma_kernel', 'dm_compose_rounds': 'compose_pass_kernel',
+                'dm_compose_passes': 'compose_passes_kernel'}
 
 
 def pass_kernel_profile(torch, state):
@@ -341,7 +342,7 @@ def tile_pattern_ceiling(torch, N, state, entry):
 
 def all_durations(by_kernel):
     """Durations of the pass launches (the round-matrix composition launches are listed apart)."""
-    return [d for k, v in by_kernel.items() if k != 'compose_pass_kernel' for d in v]
+    return [d for k, v in by_kernel.items() if not k.startswith('compose_') for d in v]
 
 
 def fp64_peak(torch, N, seconds=0.5):

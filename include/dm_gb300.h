@@ -291,6 +291,24 @@ typedef struct dm_batch_pass {
 int dm_compose_rounds(int format, const dm_batch_pass *pass, const double *mats_dev, size_t mats_count,
                       uint16_t *images_dev, size_t images_count, void *stream);
 
+/* dm_compose_rounds for the rounds of several passes in one launch: entry i
+ * of the round table composes round `round` of pass `pass`, whose moff are
+ * relative to mats_dev + mats_off, into the images at images_dev + image_off
+ * (8 FP16 values aligned).  The tables are passed twice: host copies
+ * (validated here) and the identical device copies the kernel reads. */
+typedef struct dm_compose_round {
+    int32_t pass, round;
+    int32_t format;                    /* DM_IMAGE_TC or DM_IMAGE_TMA */
+    int32_t pad;
+    int64_t mats_off;                  /* doubles */
+    int64_t image_off;                 /* FP16 values */
+} dm_compose_round;
+
+int dm_compose_passes(const dm_batch_pass *passes_host, const dm_batch_pass *passes_dev, int npasses,
+                      const dm_compose_round *rounds_host, const dm_compose_round *rounds_dev, int nrounds,
+                      const double *mats_dev, size_t mats_count, uint16_t *images_dev, size_t images_count,
+                      void *stream);
+
 /* One independent circuit instance of a batched program. */
 typedef struct dm_batch_instance {
     int32_t n;                         /* qubits */

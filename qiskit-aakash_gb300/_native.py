@@ -122,6 +122,11 @@ class DmBatchTcPass(ctypes.Structure):
     _fields_ = [('ops', DmBatchPass), ('tables', DmTcPass)]
 
 
+class DmComposeRound(ctypes.Structure):
+    _fields_ = [('pass_', ctypes.c_int32), ('round', ctypes.c_int32), ('format', ctypes.c_int32),
+                ('pad', ctypes.c_int32), ('mats_off', ctypes.c_int64), ('image_off', ctypes.c_int64)]
+
+
 class DmBatchInstance(ctypes.Structure):
     _fields_ = [('n', ctypes.c_int32), ('npasses', ctypes.c_int32), ('pass_begin', ctypes.c_int32),
                 ('pad', ctypes.c_int32), ('state_off', ctypes.c_int64), ('prob_off', ctypes.c_int64),
@@ -181,6 +186,8 @@ SIGNATURES = {
     'dm_apply_pass_tc': (_i, [_vp, _i, ctypes.POINTER(DmTcPass), _vp, _sz, _vp, _vp]),
     'dm_apply_pass_tma': (_i, [_vp, _i, ctypes.POINTER(DmTcPass), _vp, _sz, _vp, _vp]),
     'dm_compose_rounds': (_i, [_i, ctypes.POINTER(DmBatchPass), _vp, _sz, _vp, _sz, _vp]),
+    'dm_compose_passes': (_i, [ctypes.POINTER(DmBatchPass), _vp, _i, ctypes.POINTER(DmComposeRound), _vp, _i, _vp,
+                               _sz, _vp, _sz, _vp]),
     'dm_max_abs_diff': (_i, [_vp, _i, _vp, _i, _i, _vp, _vp]),
     'dm_tile_copy_probe': (_i, [_vp, _i, _vp, _vp]),
     'dm_fp64_fma_probe_threads': (_i, []),

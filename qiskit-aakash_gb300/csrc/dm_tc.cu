@@ -434,26 +434,25 @@ __device__ void batch_tc_setup(Pass &ps, const dm_batch_tc_pass &bp, int n) {
 // Uh = fp16(U) and Ul = fp16(2**11 (U - Uh)): three images 2**11 Uh | Ul | Uh
 // for the cp.async-fed kernels, two images Uh | Ul for the TMA-fed one.
 //
-// What bounds it is the FP64 pipe (two FMAs per clock and SM) and, before
-// this form, the latency of one thread per column.  So one warp owns 8
+// What bounds it is the FP64 pipe: two FMAs per clock and SM, one warp
+// instruction per 64 cycles on each of its four quarters.  So one warp owns C
 // columns (index j = d0 + 4 d1 + 16 d2 of column c at c * kColStride + j; no
 // block barrier between operations), its lanes sharing each operation's
-// independent groups; the 4x4 maps that come before the round's first pair
+// independent groups: 8 columns in the batched sweeps, where a CTA composes a
+// whole pass and the pair operations then fill the lanes, and 2 in the
+// single-state launches, whose rounds have the chip to themselves and spread
+// over 32 warps each.  The 4x4 maps that come before the round's first pair
 // operation form a Kronecker product and are written as such (two products
 // per entry instead of 16 FMAs per four entries and map); and a map whose I
 // row is (1,0,0,0), whose X and Y rows take no I, costs 10 FMAs per four
-// entries instead of 16.  The 8 columns of a warp are the 8 halves of one
-// 16-byte chunk per row of an image.  Measured with one column per thread and
-// now: a recorded 20-layer circuit of 10 qubits (20 passes) 1,314 -> 612 us,
-// the 14-qubit QFT with 2 layers (24 passes) 15.63 -> 14.07 ms.
+// entries instead of 16.
 constexpr int kColStride = 65;   // doubles per column: a warp's lanes spread over the banks
-constexpr int kColsPerWarp = 8;
 constexpr int kColBytes = 64 * kColStride * 8;   // one round's columns
 static_assert(kColBytes <= int(kSmemBytes), "one round of FP64 columns fits the pass's shared memory");
 
-// One operation on the warp's 8 columns (digit positions from the op flags).
+// One operation on the warp's C columns (digit positions from the op flags).
 // Map2: 16x16 general maps too (the single-state passes; the batched plans hold none).
-template <bool Map2>
+template <bool Map2, int C>
 __device__ __forceinline__ void cols_apply(double *w, const dm_op &op, const double *__restrict__ mats, int lane) {
     const double *mg = mats + op.moff;
     const int da = (op.flags >> 8) & 3, db = (op.flags >> 12) & 3;
@@ -468,7 +467,7 @@ __device__ __forceinline__ void cols_apply(double *w, const dm_op &op, const dou
         const int j0 = ((g >> (2 * da)) << (2 * da + 2)) | (g & (S - 1));
         double *col = w + (lane >> 4) * kColStride + j0;
 #pragma unroll
-        for (int it = 0; it < kColsPerWarp / 2; ++it) {
+        for (int it = 0; it < C / 2; ++it) {
             double *x = col + 2 * it * kColStride;
             double x0 = x[0], x1 = x[S], x2 = x[2 * S], x3 = x[3 * S];
             if (xy) {
@@ -486,6 +485,7 @@ __device__ __forceinline__ void cols_apply(double *w, const dm_op &op, const dou
         return;
     }
     // pair operations: lane = (column, value of the third digit)
+    if (lane >= 4 * C) return;
     const int SA = 1 << (2 * da), SB = 1 << (2 * db), SC = 1 << (2 * (3 - da - db));
     double *col = w + (lane >> 2) * kColStride + (lane & 3) * SC;
     double x[16];
@@ -514,9 +514,9 @@ __device__ __forceinline__ void cols_apply(double *w, const dm_op &op, const dou
     for (int i = 0; i < 16; ++i) col[(i >> 2) * SA + (i & 3) * SB] = x[i];
 }
 
-// Columns k0 .. k0 + 7 of round r (k0 a multiple of 8) by one warp, w its 8 columns of scratch;
+// Columns k0 .. k0 + C - 1 of round r (k0 a multiple of C) by one warp, w its C columns of scratch;
 // the round's images at img (three or two of them).
-template <bool Map2>
+template <bool Map2, int C>
 __device__ void compose_warp(const dm_batch_pass &bp, int r, int k0, const double *__restrict__ mats, double *w,
                              uint16_t *__restrict__ img, bool three, int lane) {
     int o = r > 0 ? bp.round_end[r - 1] : 0;
@@ -532,7 +532,7 @@ __device__ void compose_warp(const dm_batch_pass &bp, int r, int k0, const doubl
         else lead[2] = m;
     }
 #pragma unroll
-    for (int it = 0; it < 2 * kColsPerWarp; ++it) {   // lane's rows j of column c
+    for (int it = 0; it < 2 * C; ++it) {   // lane's rows j of column c
         const int c = it >> 1, j = lane + 32 * (it & 1), k = k0 + c;
         const double f0 = lead[0] ? lead[0][4 * (j & 3) + (k & 3)] : ((j ^ k) & 3 ? 0.0 : 1.0);
         const double f1 = lead[1] ? lead[1][4 * ((j >> 2) & 3) + ((k >> 2) & 3)] : ((j ^ k) & 12 ? 0.0 : 1.0);
@@ -541,55 +541,74 @@ __device__ void compose_warp(const dm_batch_pass &bp, int r, int k0, const doubl
     }
     __syncwarp();
     for (; o < oe; ++o) {
-        cols_apply<Map2>(w, bp.ops[o], mats, lane);
+        cols_apply<Map2, C>(w, bp.ops[o], mats, lane);
         __syncwarp();
     }
-    // row j of the 8 columns: one 16-byte chunk per image
+    // row j of the C columns: one chunk of C halves per image (16 bytes of 8 columns)
     const int uh = three ? 8192 : 0;   // three: 2**11 Uh at 0, Ul at 4096, Uh at 8192; two: Uh at 0, Ul at 4096
+    struct alignas(2 * C) Chunk {
+        uint32_t v[C / 2];
+    };
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
         const int j = lane + 32 * half;
-        const uint32_t pos = uint32_t(k0 >> 3) * 64 + uint32_t(j & 7) * 8 + uint32_t(j >> 3) * 512;
-        uint32_t h2[4], l2[4], s2[4];
+        const uint32_t pos = uint32_t(k0 >> 3) * 64 + uint32_t(k0 & 7) + uint32_t(j & 7) * 8 + uint32_t(j >> 3) * 512;
+        Chunk h2, l2, s2;
 #pragma unroll
-        for (int c = 0; c < kColsPerWarp; c += 2) {
+        for (int c = 0; c < C; c += 2) {
             const double u0 = w[c * kColStride + j], u1 = w[(c + 1) * kColStride + j];
             const __half h0 = __double2half(u0), h1 = __double2half(u1);
             const float f0 = __half2float(h0), f1 = __half2float(h1);
             const __half l0 = __double2half((u0 - double(f0)) * double(kLoScale));
             const __half l1 = __double2half((u1 - double(f1)) * double(kLoScale));
-            h2[c >> 1] = uint32_t(__half_as_ushort(h0)) | (uint32_t(__half_as_ushort(h1)) << 16);
-            l2[c >> 1] = uint32_t(__half_as_ushort(l0)) | (uint32_t(__half_as_ushort(l1)) << 16);
-            s2[c >> 1] = uint32_t(__half_as_ushort(__float2half_rn(f0 * kLoScale))) |
-                         (uint32_t(__half_as_ushort(__float2half_rn(f1 * kLoScale))) << 16);
+            h2.v[c >> 1] = uint32_t(__half_as_ushort(h0)) | (uint32_t(__half_as_ushort(h1)) << 16);
+            l2.v[c >> 1] = uint32_t(__half_as_ushort(l0)) | (uint32_t(__half_as_ushort(l1)) << 16);
+            s2.v[c >> 1] = uint32_t(__half_as_ushort(__float2half_rn(f0 * kLoScale))) |
+                           (uint32_t(__half_as_ushort(__float2half_rn(f1 * kLoScale))) << 16);
         }
-        if (three) *reinterpret_cast<uint4 *>(img + pos) = make_uint4(s2[0], s2[1], s2[2], s2[3]);
-        *reinterpret_cast<uint4 *>(img + 4096 + pos) = make_uint4(l2[0], l2[1], l2[2], l2[3]);
-        *reinterpret_cast<uint4 *>(img + uh + pos) = make_uint4(h2[0], h2[1], h2[2], h2[3]);
+        if (three) *reinterpret_cast<Chunk *>(img + pos) = s2;
+        *reinterpret_cast<Chunk *>(img + 4096 + pos) = l2;
+        *reinterpret_cast<Chunk *>(img + uh + pos) = h2;
     }
     __syncwarp();   // the columns are read before the next round's are written
 }
 
 // All rounds of a batched pass into per-CTA scratch (three images per round), all threads of the
-// CTA, each warp its 8 columns; the pass's operand and matrix regions are free between passes.
-static_assert(kThreads / 32 * kColsPerWarp == 64, "the CTA's warps cover the 64 columns");
+// CTA, each warp 8 columns; the pass's operand and matrix regions are free between passes.
+constexpr int kBatchCols = 64 / (kThreads / 32);
 __device__ void compose_rounds(const dm_batch_pass &bp, const double *__restrict__ mats, uint16_t *__restrict__ umats,
                                double *work) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int r = 0; r < bp.nrounds; ++r)
-        compose_warp<false>(bp, r, warp * kColsPerWarp, mats, work + warp * kColsPerWarp * kColStride,
-                            umats + int64_t(r) * kUHalves, true, lane);
+        compose_warp<false, kBatchCols>(bp, r, warp * kBatchCols, mats, work + warp * kBatchCols * kColStride,
+                                        umats + int64_t(r) * kUHalves, true, lane);
 }
 
-// One pass's round images for the single-state kernels: one warp per CTA, CTA (r, c) the columns
-// 8c .. 8c + 7 of round r, so that a pass's FP64 work spreads over 8 SMs per round.
-__global__ void __launch_bounds__(32)
+// The single-state launches: CTA (r, c) takes the columns 8c .. 8c + 7 of a round, 2 per warp.
+constexpr int kComposeWarps = 4, kComposeCols = 2, kComposeGrid = 64 / (kComposeWarps * kComposeCols);
+
+// One pass's round images (CTA x = round of the pass).
+__global__ void __launch_bounds__(32 * kComposeWarps)
     compose_pass_kernel(const __grid_constant__ dm_batch_pass bp, const double *__restrict__ mats,
                         uint16_t *__restrict__ images, int image_halves) {
-    __shared__ double cols[kColsPerWarp * kColStride];
-    const int r = blockIdx.x, k0 = int(blockIdx.y) * kColsPerWarp;
-    compose_warp<true>(bp, r, k0, mats, cols, images + int64_t(r) * image_halves, image_halves == kUHalves,
-                       threadIdx.x);
+    __shared__ double cols[kComposeWarps * kComposeCols * kColStride];
+    const int r = blockIdx.x, warp = threadIdx.x >> 5;
+    compose_warp<true, kComposeCols>(bp, r, (int(blockIdx.y) * kComposeWarps + warp) * kComposeCols, mats,
+                                     cols + warp * kComposeCols * kColStride, images + int64_t(r) * image_halves,
+                                     image_halves == kUHalves, threadIdx.x & 31);
+}
+
+// The round images of several passes (CTA x = entry of the round table).  A pass's composition alone
+// is a launch of a few microseconds on a few dozen warps; one launch for many passes fills the chip.
+__global__ void __launch_bounds__(32 * kComposeWarps)
+    compose_passes_kernel(const dm_batch_pass *__restrict__ passes, const dm_compose_round *__restrict__ rounds,
+                          const double *__restrict__ mats, uint16_t *__restrict__ images) {
+    __shared__ double cols[kComposeWarps * kComposeCols * kColStride];
+    const dm_compose_round e = rounds[blockIdx.x];
+    const int warp = threadIdx.x >> 5;
+    compose_warp<true, kComposeCols>(passes[e.pass], e.round, (int(blockIdx.y) * kComposeWarps + warp) * kComposeCols,
+                                     mats + e.mats_off, cols + warp * kComposeCols * kColStride, images + e.image_off,
+                                     e.format == DM_IMAGE_TC, threadIdx.x & 31);
 }
 
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
@@ -872,7 +891,36 @@ extern "C" int dm_compose_rounds(int format, const dm_batch_pass *pass, const do
     if (rc) return rc;
     const int halves = format == DM_IMAGE_TC ? tc::kUHalves : 2 * 4096;
     if (images_count < size_t(pass->nrounds) * size_t(halves)) return DM_ERR_ARG;
-    tc::compose_pass_kernel<<<dim3(pass->nrounds, 64 / tc::kColsPerWarp), 32, 0, as_stream(stream)>>>(*pass, mats_dev, images_dev, halves);
+    tc::compose_pass_kernel<<<dim3(pass->nrounds, tc::kComposeGrid), 32 * tc::kComposeWarps, 0, as_stream(stream)>>>(
+        *pass, mats_dev, images_dev, halves);
+    count_launch();
+    return launch_status();
+}
+
+extern "C" int dm_compose_passes(const dm_batch_pass *passes_host, const dm_batch_pass *passes_dev, int npasses,
+                                 const dm_compose_round *rounds_host, const dm_compose_round *rounds_dev, int nrounds,
+                                 const double *mats_dev, size_t mats_count, uint16_t *images_dev, size_t images_count,
+                                 void *stream) {
+    DM_CHECK_ARG(passes_host && passes_dev && rounds_host && rounds_dev && mats_dev && images_dev && npasses >= 1 &&
+                 nrounds >= 1);
+    if (reinterpret_cast<uintptr_t>(images_dev) & 15 || reinterpret_cast<uintptr_t>(mats_dev) & 7) return DM_ERR_ARG;
+    if (mats_count > size_t(INT32_MAX)) return DM_ERR_RANGE;
+    for (int i = 0; i < nrounds; ++i) {
+        const dm_compose_round &e = rounds_host[i];
+        if (e.pass < 0 || e.pass >= npasses) return DM_ERR_ARG;
+        if (e.format != DM_IMAGE_TC && e.format != DM_IMAGE_TMA) return DM_ERR_ARG;
+        if (e.mats_off < 0 || size_t(e.mats_off) > mats_count) return DM_ERR_ARG;
+        // the rounds of a pass follow one another with one coefficient offset: the pass is checked once
+        if (i == 0 || e.pass != rounds_host[i - 1].pass || e.mats_off != rounds_host[i - 1].mats_off) {
+            const int rc = validate_round_ops(passes_host[e.pass], int64_t(mats_count) - e.mats_off, true);
+            if (rc) return rc;
+        }
+        if (e.round < 0 || e.round >= passes_host[e.pass].nrounds) return DM_ERR_PROGRAM;
+        const int64_t halves = e.format == DM_IMAGE_TC ? tc::kUHalves : 2 * 4096;
+        if (e.image_off < 0 || (e.image_off & 7) || size_t(e.image_off + halves) > images_count) return DM_ERR_ARG;
+    }
+    tc::compose_passes_kernel<<<dim3(nrounds, tc::kComposeGrid), 32 * tc::kComposeWarps, 0, as_stream(stream)>>>(
+        passes_dev, rounds_dev, mats_dev, images_dev);
     count_launch();
     return launch_status();
 }

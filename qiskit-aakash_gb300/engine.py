@@ -27,6 +27,9 @@ DEFAULT_LOW_AXES = 2
 # launched (the rest of the queue waits for later operations or a read-out).
 STREAM_OPS = 4096
 
+# Tensor-core passes whose round matrices one launch composes (groups double up to this).
+COMPOSE_PASSES = 16
+
 # Copy-out of large states: 32 Mi coefficients (256 MB FP64) per chunk, two
 # device and two pinned host buffers per device, host copies in 16 MB slices.
 _COPY_CHUNK = 1 << 25
@@ -181,11 +184,12 @@ class DeviceState:
         if compose not in ('device', 'host'):
             raise BasicAerError("compose must be 'device' or 'host'")
         # where the tensor-core rounds' 64x64 matrices are composed in FP64:
-        # 'device' (dm_compose_rounds from the ops' coefficients) or 'host' (numpy, FP16 images uploaded)
+        # 'device' (dm_compose_passes from the ops' coefficients) or 'host' (numpy, FP16 images uploaded)
         self.compose = compose
         self.passes_by_kernel = {'tma': 0, 'tc': 0, 'cuda_cores': 0}
         self.composed_on = {'device': 0, 'host': 0}
-        self._images = None       # device round images of the pass in flight (DM_MAX_ROUNDS x 12288 FP16)
+        self._images = None       # device round images of the group of passes in flight
+        self._group = 1           # passes of the next group composed in one launch
         self.status = torch.zeros(1, dtype=torch.int32, device=self.device) if self.tensor_cores else None
         self.kmax = min(tile_axes or DEFAULT_TILE_AXES[precision], N.DM_MAX_TILE_AXES)
         self.low = low_axes
@@ -306,7 +310,7 @@ class DeviceState:
         fit a 5-dimensional tensor map; other passes run on the cp.async-fed
         kernel; a pass with more rounds than a descriptor holds, on neither.
         With compose='device' the round matrices are composed by
-        dm_compose_rounds from the ops' FP64 coefficients; a pass with more
+        dm_compose_passes from the ops' FP64 coefficients; a pass with more
         ops than its table holds is composed on the host."""
         kernels = (('tma', 'dm_apply_pass_tma', encode_pass_tma),) if self.tma else ()
         kernels += (('tc', 'dm_apply_pass_tc', encode_pass_tc),)
@@ -327,54 +331,97 @@ class DeviceState:
                 continue
         return None
 
-    def _image_buffer(self):
-        if self._images is None:
-            torch = _torch()
-            self._images = torch.empty(N.DM_MAX_ROUNDS * 3 * 4096, dtype=torch.int16, device=self.device)
-        return self._images
-
     def _run_passes_tc(self, passes):
-        """Encode and launch pass by pass: the host plans pass i+1 while the GPU runs pass i.
+        """Encode and launch the passes in groups: the host plans the next group while the GPU runs one.
 
-        Device composition: the ops' coefficients go up (a few KB), one
-        dm_compose_rounds launch writes the round images into one device
-        buffer, and the pass reads them; the stream orders each pass's
-        composition after the previous pass's reads."""
-        torch = _torch()
-        sp = ctypes.c_void_p(self.status.data_ptr())
+        Device composition: a group's op tables and coefficients go up in one
+        copy, one dm_compose_passes launch writes its round images and the
+        passes read them.  A composition alone is a few dozen warps for
+        several microseconds, so groups double from one pass (the device
+        starts at once) up to COMPOSE_PASSES; the stream orders a group's
+        composition after the previous group's reads of the image buffer."""
         keep = []
+        ran = 0
+        group = []
         for p in passes:
             enc = self._encode_tc(p)
-            if enc is None:
-                self._run_passes([p])     # more rounds than a descriptor holds: the CUDA-core pass
-                self.passes_by_kernel['cuda_cores'] += 1
-                continue
-            name, d, bp, data = enc
+            if enc is None or enc[2] is None:
+                self._run_group(group, keep)
+                group = []
+                if enc is None:               # more rounds than a descriptor holds: the CUDA-core pass
+                    self._run_passes([p])
+                    self.passes_by_kernel['cuda_cores'] += 1
+                    keep.append(self._keep)
+                    continue
+                self._run_host_composed(enc, keep)
+            else:
+                group.append(enc)
+                if len(group) >= self._group:
+                    self._group = min(2 * self._group, COMPOSE_PASSES)
+                    self._run_group(group, keep)
+                    group = []
+            ran += 1
+        self._run_group(group, keep)
+        self.passes_run += ran
+        self._keep = keep        # until the next flush
+
+    def _run_host_composed(self, enc, keep):
+        torch = _torch()
+        name, d, _, data = enc
+        host = np.concatenate(data).view(np.int16)      # FP16 bit patterns
+        h = torch.from_numpy(host).pin_memory()
+        dev = h.to(self.device, non_blocking=True)
+        self.h2d_bytes += host.nbytes
+        self._call(name, self.ptr, self.n, ctypes.byref(d), ctypes.c_void_p(dev.data_ptr()),
+                   ctypes.c_size_t(host.size), ctypes.c_void_p(self.status.data_ptr()), self.stream, keep=(d, dev))
+        self.passes_by_kernel['tma' if name == 'dm_apply_pass_tma' else 'tc'] += 1
+        self.composed_on['host'] += 1
+        keep.append((h, dev, d))
+
+    def _run_group(self, group, keep):
+        """One composition launch for the group's passes, then the passes."""
+        if not group:
+            return
+        torch = _torch()
+        tables = (N.DmBatchPass * len(group))(*[bp for _, _, bp, _ in group])
+        nrounds = sum(bp.nrounds for _, _, bp, _ in group)
+        rounds = (N.DmComposeRound * nrounds)()
+        coefs, images = [], []
+        i = mats = size = 0
+        for k, (name, _, bp, data) in enumerate(group):
+            tma = name == 'dm_apply_pass_tma'
+            halves = 2 * 4096 if tma else 3 * 4096
+            images.append((size, halves * bp.nrounds))
+            for r in range(bp.nrounds):
+                e = rounds[i]
+                e.pass_, e.round, e.format = k, r, N.DM_IMAGE_TMA if tma else N.DM_IMAGE_TC
+                e.mats_off, e.image_off = mats, size
+                size += halves
+                i += 1
+            coefs += data
+            mats += sum(c.size for c in data)
+        # one upload: coefficients (8-byte values first, so that every part is aligned), round and pass tables
+        block = np.concatenate(coefs) if coefs else np.zeros(1)
+        raw = block.tobytes() + bytes(rounds) + bytes(tables)
+        h = torch.from_numpy(np.frombuffer(raw, dtype=np.uint8).copy()).pin_memory()
+        dev = h.to(self.device, non_blocking=True)
+        self.h2d_bytes += len(raw)
+        if self._images is None or self._images.numel() < size:
+            self._images = torch.empty(size, dtype=torch.int16, device=self.device)
+        img = self._images
+        at = dev.data_ptr()
+        at_rounds = at + block.nbytes
+        at_passes = at_rounds + ctypes.sizeof(rounds)
+        self._call('dm_compose_passes', tables, ctypes.c_void_p(at_passes), len(group), rounds,
+                   ctypes.c_void_p(at_rounds), nrounds, ctypes.c_void_p(at), ctypes.c_size_t(block.size),
+                   ctypes.c_void_p(img.data_ptr()), ctypes.c_size_t(size), self.stream, keep=(tables, rounds, dev, img))
+        sp = ctypes.c_void_p(self.status.data_ptr())
+        for (name, d, _, _), (off, count) in zip(group, images):
+            self._call(name, self.ptr, self.n, ctypes.byref(d), ctypes.c_void_p(img.data_ptr() + 2 * off),
+                       ctypes.c_size_t(count), sp, self.stream, keep=(d,))
             self.passes_by_kernel['tma' if name == 'dm_apply_pass_tma' else 'tc'] += 1
-            if bp is not None:
-                host = np.concatenate(data) if data else np.zeros(1)
-                h = torch.from_numpy(host).pin_memory()
-                dev = h.to(self.device, non_blocking=True)
-                self.h2d_bytes += host.nbytes
-                img = self._image_buffer()
-                fmt = N.DM_IMAGE_TMA if name == 'dm_apply_pass_tma' else N.DM_IMAGE_TC
-                ip, isz = ctypes.c_void_p(img.data_ptr()), ctypes.c_size_t(img.numel())
-                self._call('dm_compose_rounds', fmt, ctypes.byref(bp), ctypes.c_void_p(dev.data_ptr()),
-                           ctypes.c_size_t(host.size), ip, isz, self.stream, keep=(bp, dev))
-                self._call(name, self.ptr, self.n, ctypes.byref(d), ip, isz, sp, self.stream, keep=(d,))
-                self.composed_on['device'] += 1
-                keep.append((h, dev, d, bp))
-                continue
-            host = np.concatenate(data).view(np.int16)      # FP16 bit patterns
-            h = torch.from_numpy(host).pin_memory()
-            dev = h.to(self.device, non_blocking=True)
-            self.h2d_bytes += host.nbytes
-            self._call(name, self.ptr, self.n, ctypes.byref(d), ctypes.c_void_p(dev.data_ptr()),
-                       ctypes.c_size_t(host.size), sp, self.stream, keep=(d, dev))
-            self.composed_on['host'] += 1
-            keep.append((h, dev, d))
-        self.passes_run += len(keep)
-        self._keep = keep
+            self.composed_on['device'] += 1
+        keep.append((h, dev, img, group))
 
     def _run_passes(self, passes):
         torch = _torch()
