@@ -26,126 +26,159 @@ struct SubLattice {
     double scale;                    // 2**(n-m)
 };
 
-template <typename T>
-__global__ void __launch_bounds__(256) sublattice_gather(const T *__restrict__ st, const __grid_constant__ SubLattice L,
-                                                         double *__restrict__ out) {
-    const int64_t total = int64_t(1) << L.m;
-    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < total;
-         i += int64_t(gridDim.x) * blockDim.x) {
-        int64_t idx = 0;
-        int pop = 0;
-        for (int j = 0; j < L.m; ++j)
-            if ((i >> (L.m - 1 - j)) & 1) {
-                idx += L.stride[j];
-                ++pop;
-            }
-        out[i] = double(st[idx]) * L.errpow[pop] * L.scale;
-    }
-}
+// Walsh-Hadamard butterflies over bits [lo, lo + nb) of the 2**m vector, the
+// first sweep (lo = 0) gathering and scaling the sub-lattice as it loads.
+// FP64 additions bound a CTA (two per clock and SM: a CTA of 2,048 elements
+// and 11 bits took 13.6 us at n = 12), so a CTA takes 1,024 elements: all bits
+// of a vector up to 2**10, else at most 7 of them, as 2**nb rows of
+// 2**(10 - nb) contiguous elements (lo > 0) or 2**(10 - nb) whole blocks of
+// 2**nb (lo = 0).  Measured at n = 12: 16 us for the whole read-out, gather
+// included, 23 us before.
+constexpr int kWhtBits = 7, kWhtTileLog = 10;
 
-// In-place unnormalised Walsh-Hadamard butterflies over bits [lo, lo+nb) of
-// a 2**m vector; each CTA transforms one tile of 2**nb elements in shared
-// memory.
-constexpr int kWhtTileBits = 11;
-
-__global__ void __launch_bounds__(256) wht_kernel(double *__restrict__ v, int m, int lo, int nb) {
-    __shared__ double tile[1 << kWhtTileBits];
-    const int tsize = 1 << nb;
-    const int64_t ntiles = int64_t(1) << (m - nb);
-    const int64_t lomask = (int64_t(1) << lo) - 1;
-    for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const int64_t base = (t & lomask) | ((t >> lo) << (lo + nb));
-        for (int e = threadIdx.x; e < tsize; e += blockDim.x) tile[e] = v[base | (int64_t(e) << lo)];
-        __syncthreads();
-        for (int b = 0; b < nb; ++b) {
-            for (int p = threadIdx.x; p < tsize / 2; p += blockDim.x) {
-                const int i0 = ((p >> b) << (b + 1)) | (p & ((1 << b) - 1));
-                const int i1 = i0 | (1 << b);
-                const double x = tile[i0], y = tile[i1];
-                tile[i0] = x + y;
-                tile[i1] = x - y;
-            }
-            __syncthreads();
+template <typename T, bool Gather>
+__global__ void __launch_bounds__(256) wht_kernel(const T *__restrict__ st, const __grid_constant__ SubLattice L,
+                                                  double *__restrict__ v, int lo, int nb, int tlog) {
+    __shared__ double tile[1 << kWhtTileLog];
+    const int tsize = 1 << tlog;
+    const int rlog = tlog - nb;              // lo > 0: log2 of the contiguous run of a row
+    const int64_t b = blockIdx.x;
+    const int runs_log = lo - rlog;
+    const int64_t base = Gather ? b << tlog
+                                : ((b >> runs_log) << (lo + nb)) | ((b & ((int64_t(1) << runs_log) - 1)) << rlog);
+    auto at = [&](int e) { return Gather ? base + e : base + (int64_t(e >> rlog) << lo) + (e & ((1 << rlog) - 1)); };
+    for (int e = threadIdx.x; e < tsize; e += blockDim.x) {
+        if constexpr (Gather) {
+            const int64_t i = base + e;
+            int64_t idx = 0;
+            int pop = 0;
+            for (int j = 0; j < L.m; ++j)
+                if ((i >> (L.m - 1 - j)) & 1) {
+                    idx += L.stride[j];
+                    ++pop;
+                }
+            tile[e] = double(st[idx]) * L.errpow[pop] * L.scale;
+        } else {
+            tile[e] = v[at(e)];
         }
-        for (int e = threadIdx.x; e < tsize; e += blockDim.x) v[base | (int64_t(e) << lo)] = tile[e];
+    }
+    __syncthreads();
+    const int s0 = Gather ? 0 : rlog;        // log2 of the first bit's element stride
+    for (int k = 0; k < nb; ++k) {
+        const int sb = s0 + k;
+        for (int p = threadIdx.x; p < tsize / 2; p += blockDim.x) {
+            const int i0 = ((p >> sb) << (sb + 1)) | (p & ((1 << sb) - 1));
+            const int i1 = i0 | (1 << sb);
+            const double x = tile[i0], y = tile[i1];
+            tile[i0] = x + y;
+            tile[i1] = x - y;
+        }
         __syncthreads();
     }
+    for (int e = threadIdx.x; e < tsize; e += blockDim.x) v[at(e)] = tile[e];
 }
 
-static int wht_inplace(double *v, int m, cudaStream_t s) {
-    for (int lo = 0; lo < m; lo += kWhtTileBits) {
-        const int nb = (m - lo) < kWhtTileBits ? (m - lo) : kWhtTileBits;
-        const int64_t ntiles = int64_t(1) << (m - nb);
-        const int grid = int(ntiles < int64_t(sm_count()) * 4 ? ntiles : int64_t(sm_count()) * 4);
-        wht_kernel<<<grid, 256, 0, s>>>(v, m, lo, nb);
+template <typename T>
+static int axis_probs(const T *st, const SubLattice &L, double *v, cudaStream_t s) {
+    // the bits of a sweep; above the first one a row's run is 2**(kWhtTileLog - nb) elements
+    const int sweeps = L.m <= kWhtTileLog ? 1 : (L.m + kWhtBits - 1) / kWhtBits;
+    int lo = 0;
+    for (int i = 0; i < sweeps; ++i) {
+        const int nb = (L.m - lo + sweeps - 1 - i) / (sweeps - i);
+        const int tlog = L.m < kWhtTileLog ? L.m : kWhtTileLog;
+        const unsigned grid = unsigned(int64_t(1) << (L.m - tlog));
+        if (i == 0)
+            wht_kernel<T, true><<<grid, 256, 0, s>>>(st, L, v, lo, nb, tlog);
+        else
+            wht_kernel<T, false><<<grid, 256, 0, s>>>(st, L, v, lo, nb, tlog);
         count_launch();
-        int rc = launch_status();
+        const int rc = launch_status();
         if (rc) return rc;
+        lo += nb;
     }
     return DM_OK;
 }
 
 // --- basis N: contraction of every axis with the rows [1, +-err n] ----------
+//
+// One axis: d = err (nx X + ny Y + nz Z), then I + d and I - d: 5 FP64
+// operations per four values (the FP64 pipe is the bound, 67 us at n = 12).
+// The lowest 6 axes of a 4**6 tile are contracted in shared memory, the rest
+// three axes at a time in registers over contiguous runs.  Measured at n = 12
+// in FP64: 83 + 19 us, where three axes per thread through local memory and
+// one launch per further axis took 182 + 50 us.
 
 struct NRows {
-    double w[2][4];
+    double w[3];
 };
 
-// Contract the lowest t axes (contiguous 4**t block per thread) into 2**t values.
-template <typename T>
-__global__ void __launch_bounds__(256) contract_low(const T *__restrict__ st, int t, int64_t outer,
-                                                    const __grid_constant__ NRows R, double *__restrict__ out) {
-    const int blk = 1 << (2 * t);
-    for (int64_t o = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; o < outer;
-         o += int64_t(gridDim.x) * blockDim.x) {
-        double v[64];
-        for (int e = 0; e < blk; ++e) v[e] = double(st[o * blk + e]);
-        // contract axes from the fastest: shape (4^(t-j), 2^j) -> (4^(t-j-1), 2^(j+1))
-        int rows4 = blk >> 2;   // number of 4-groups on the current fastest 4-axis
-        int inner = 1;          // 2^j
-        for (int j = 0; j < t; ++j) {
-            // current layout: index = (h * 4 + p) * inner + i, h < rows4/inner... use a temp
-            double w[64];
-            const int outer_h = rows4 / inner;
-            for (int h = 0; h < outer_h; ++h)
-                for (int i = 0; i < inner; ++i) {
-                    double acc0 = 0.0, acc1 = 0.0;
-                    for (int p = 0; p < 4; ++p) {
-                        const double x = v[(h * 4 + p) * inner + i];
-                        acc0 = fma(R.w[0][p], x, acc0);
-                        acc1 = fma(R.w[1][p], x, acc1);
-                    }
-                    w[(h * 2 + 0) * inner + i] = acc0;
-                    w[(h * 2 + 1) * inner + i] = acc1;
-                }
-            inner *= 2;
-            rows4 /= 2;
-            const int cnt = outer_h * 2 * (inner / 2);
-            for (int e = 0; e < cnt; ++e) v[e] = w[e];
-        }
-        const int nout = 1 << t;
-        for (int e = 0; e < nout; ++e) out[o * nout + e] = v[e];
-    }
+__device__ __forceinline__ void contract(const NRows &R, double i, double x, double y, double z, double &p, double &q) {
+    const double d = fma(R.w[2], z, fma(R.w[1], y, R.w[0] * x));
+    p = i + d;
+    q = i - d;
 }
 
-// (outer, 4, inner) -> (outer, 2, inner)
-__global__ void __launch_bounds__(256) contract_axis(const double *__restrict__ in, int64_t outer, int64_t inner,
-                                                     const __grid_constant__ NRows R, double *__restrict__ out) {
-    const int64_t total = outer * inner;
-    for (int64_t g = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; g < total;
-         g += int64_t(gridDim.x) * blockDim.x) {
-        const int64_t o = g / inner, i = g - o * inner;
-        const double *src = in + o * 4 * inner + i;
-        double acc0 = 0.0, acc1 = 0.0;
-#pragma unroll
-        for (int p = 0; p < 4; ++p) {
-            const double x = src[p * inner];
-            acc0 = fma(R.w[0][p], x, acc0);
-            acc1 = fma(R.w[1][p], x, acc1);
-        }
-        out[o * 2 * inner + i] = acc0;
-        out[o * 2 * inner + inner + i] = acc1;
+constexpr int kNLow = 6, kNHigh = 3;
+
+// (tiles, 4**t) -> (tiles, 2**t), one tile per CTA.
+template <typename T>
+__global__ void __launch_bounds__(256) contract_low(const T *__restrict__ st, int t, const __grid_constant__ NRows R,
+                                                    double *__restrict__ out) {
+    constexpr int kHalf = 1 << (2 * kNLow - 1);
+    __shared__ double buf[kHalf + kHalf / 2];
+    // the fastest axis as the tile loads; then buf holds rows of 2**j values per remaining index
+    const T *src = st + (int64_t(blockIdx.x) << (2 * t));
+    for (int g = threadIdx.x; g < 1 << (2 * (t - 1)); g += blockDim.x) {
+        double p, q;
+        contract(R, double(src[4 * g]), double(src[4 * g + 1]), double(src[4 * g + 2]), double(src[4 * g + 3]), p, q);
+        buf[2 * g] = p;
+        buf[2 * g + 1] = q;
     }
+    __syncthreads();
+    double *in = buf, *to = buf + kHalf;
+    for (int j = 1; j < t; ++j) {            // (h, 4, 2**j) -> (h, 2, 2**j)
+        const int count = 1 << (2 * (t - 1 - j) + j);
+        for (int g = threadIdx.x; g < count; g += blockDim.x) {
+            const int i = g & ((1 << j) - 1), h = g >> j;
+            const double *x = in + ((h << 2) << j) + i;
+            double p, q;
+            contract(R, x[0], x[1 << j], x[2 << j], x[3 << j], p, q);
+            to[((h << 1) << j) + i] = p;
+            to[((h << 1 | 1) << j) + i] = q;
+        }
+        __syncthreads();
+        double *tmp = in;
+        in = to;
+        to = tmp;
+    }
+    for (int e = threadIdx.x; e < 1 << t; e += blockDim.x) out[(int64_t(blockIdx.x) << t) + e] = in[e];
+}
+
+// (outer, 4**K, inner) -> (outer, 2**K, inner), inner = 2**inner_log: one thread per (outer, inner).
+template <int K>
+__global__ void __launch_bounds__(128) contract_high(const double *__restrict__ in, int64_t count, int inner_log,
+                                                     const __grid_constant__ NRows R, double *__restrict__ out) {
+    const int64_t g = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+    if (g >= count) return;
+    const int64_t o = g >> inner_log, i = g & ((int64_t(1) << inner_log) - 1);
+    double v[1 << (2 * K)];
+    const double *src = in + ((o << (2 * K)) << inner_log) + i;
+#pragma unroll
+    for (int e = 0; e < 1 << (2 * K); ++e) v[e] = src[int64_t(e) << inner_log];
+#pragma unroll
+    for (int j = 0; j < K; ++j)              // (h, 4, 2**j) -> (h, 2, 2**j), in place front to back
+#pragma unroll
+        for (int e = 0; e < 1 << (2 * (K - 1 - j) + j); ++e) {
+            const int r = e & ((1 << j) - 1), h = e >> j;
+            double p, q;
+            contract(R, v[(4 * h << j) + r], v[((4 * h + 1) << j) + r], v[((4 * h + 2) << j) + r],
+                     v[((4 * h + 3) << j) + r], p, q);
+            v[(2 * h << j) + r] = p;
+            v[((2 * h + 1) << j) + r] = q;
+        }
+    double *dst = out + ((o << K) << inner_log) + i;
+#pragma unroll
+    for (int e = 0; e < 1 << K; ++e) dst[int64_t(e) << inner_log] = v[e];
 }
 
 }  // namespace dmg
@@ -165,17 +198,8 @@ extern "C" int dm_axis_probs(const void *state_dev, int n, int dtype, const int 
     for (int j = 1; j <= DM_MAX_QUBITS; ++j) L.errpow[j] = L.errpow[j - 1] * err;
     L.scale = ldexp(1.0, n - L.m);
     cudaStream_t s = as_stream(stream);
-    const int64_t total = int64_t(1) << L.m;
-    if (dtype == DM_F64)
-        sublattice_gather<double><<<grid_for(total, 256), 256, 0, s>>>(static_cast<const double *>(state_dev), L,
-                                                                       out_dev);
-    else
-        sublattice_gather<float><<<grid_for(total, 256), 256, 0, s>>>(static_cast<const float *>(state_dev), L,
-                                                                      out_dev);
-    count_launch();
-    int rc = launch_status();
-    if (rc || L.m == 0) return rc;
-    return wht_inplace(out_dev, L.m, s);
+    return dtype == DM_F64 ? axis_probs(static_cast<const double *>(state_dev), L, out_dev, s)
+                           : axis_probs(static_cast<const float *>(state_dev), L, out_dev, s);
 }
 
 static int low_axes(int n) { return n < 3 ? n : 3; }
@@ -188,42 +212,48 @@ extern "C" size_t dm_nbasis_probs_scratch_bytes(int n) {
     return (first + first / 2) * sizeof(double);
 }
 
+// The contractions of dm_nbasis_probs and dm_nbasis_probs_noalloc.  scratch: the two buffers of
+// dm_nbasis_probs_scratch_bytes (sized for a three-axis first step; this one contracts up to six).
+static int nbasis(const void *state_dev, int n, int dtype, const double *nvec3, double err, double *out_dev,
+                  double *scratch, cudaStream_t s) {
+    NRows R;
+    for (int c = 0; c < 3; ++c) R.w[c] = err * nvec3[c];
+    const int t = n < kNLow ? n : kNLow;
+    double *bufA = scratch;
+    double *bufB = scratch ? scratch + (size_t(pow4(n - low_axes(n))) << low_axes(n)) : nullptr;
+    double *dst = t == n ? out_dev : bufA;
+    const unsigned tiles = unsigned(pow4(n - t));
+    if (dtype == DM_F64)
+        contract_low<double><<<tiles, 256, 0, s>>>(static_cast<const double *>(state_dev), t, R, dst);
+    else
+        contract_low<float><<<tiles, 256, 0, s>>>(static_cast<const float *>(state_dev), t, R, dst);
+    count_launch();
+    int rc = launch_status();
+    const double *src = dst;
+    for (int done = t; !rc && done < n;) {
+        const int K = n - done < kNHigh ? n - done : kNHigh;
+        const int64_t count = pow4(n - done - K) << done;
+        double *d = done + K == n ? out_dev : (src == bufA ? bufB : bufA);
+        const unsigned grid = unsigned((count + 127) / 128);
+        if (K == 3)
+            contract_high<3><<<grid, 128, 0, s>>>(src, count, done, R, d);
+        else if (K == 2)
+            contract_high<2><<<grid, 128, 0, s>>>(src, count, done, R, d);
+        else
+            contract_high<1><<<grid, 128, 0, s>>>(src, count, done, R, d);
+        count_launch();
+        rc = launch_status();
+        src = d;
+        done += K;
+    }
+    return rc;
+}
+
 extern "C" int dm_nbasis_probs(const void *state_dev, int n, int dtype, const double *nvec3, double err,
                                double *out_dev, void *scratch_dev, void *stream) {
     DM_CHECK_ARG(state_dev && nvec3 && out_dev && valid_n(n) && valid_dtype(dtype));
-    const int t = low_axes(n);
-    DM_CHECK_ARG(t == n || scratch_dev);
-    NRows R;
-    R.w[0][0] = R.w[1][0] = 1.0;
-    for (int c = 0; c < 3; ++c) {
-        R.w[0][c + 1] = err * nvec3[c];
-        R.w[1][c + 1] = -err * nvec3[c];
-    }
-    cudaStream_t s = as_stream(stream);
-    const size_t first = size_t(pow4(n - t)) << t;
-    double *bufA = static_cast<double *>(scratch_dev);
-    double *bufB = bufA ? bufA + first : nullptr;
-    double *dst = (t == n) ? out_dev : bufA;
-    const int64_t outer = pow4(n - t);
-    if (dtype == DM_F64)
-        contract_low<double><<<grid_for(outer, 256), 256, 0, s>>>(static_cast<const double *>(state_dev), t, outer,
-                                                                  R, dst);
-    else
-        contract_low<float><<<grid_for(outer, 256), 256, 0, s>>>(static_cast<const float *>(state_dev), t, outer, R,
-                                                                 dst);
-    count_launch();
-    int rc = launch_status();
-    if (rc || t == n) return rc;
-    const double *src = bufA;
-    for (int q = n - t - 1; q >= 0; --q) {
-        const int64_t o = pow4(q), inner = int64_t(1) << (n - 1 - q);
-        double *d = (q == 0) ? out_dev : (src == bufA ? bufB : bufA);
-        contract_axis<<<grid_for(o * inner, 256), 256, 0, s>>>(src, o, inner, R, d);
-        count_launch();
-        if ((rc = launch_status())) return rc;
-        src = d;
-    }
-    return DM_OK;
+    DM_CHECK_ARG(low_axes(n) == n || scratch_dev);
+    return nbasis(state_dev, n, dtype, nvec3, err, out_dev, static_cast<double *>(scratch_dev), as_stream(stream));
 }
 
 // ---------------------------------------------------------------------------
@@ -316,37 +346,7 @@ extern "C" int dm_nbasis_probs_noalloc(const void *state_dev, int n, int dtype, 
         int rc = noalloc_scratch(&scratch);
         if (rc) return rc;
     }
-    NRows R;
-    R.w[0][0] = R.w[1][0] = 1.0;
-    for (int c = 0; c < 3; ++c) {
-        R.w[0][c + 1] = err * nvec3[c];
-        R.w[1][c + 1] = -err * nvec3[c];
-    }
-    cudaStream_t s = as_stream(stream);
-    // Every buffer element read below is written earlier in the same call,
-    // so the array's contents from a previous call never leak into a result.
-    const size_t first = size_t(pow4(n - t)) << t;
-    double *bufA = scratch;
-    double *bufB = scratch ? scratch + first : nullptr;
-    double *dst = (t == n) ? out_dev : bufA;
-    const int64_t outer = pow4(n - t);
-    if (dtype == DM_F64)
-        contract_low<double><<<grid_for(outer, 256), 256, 0, s>>>(static_cast<const double *>(state_dev), t, outer,
-                                                                  R, dst);
-    else
-        contract_low<float><<<grid_for(outer, 256), 256, 0, s>>>(static_cast<const float *>(state_dev), t, outer, R,
-                                                                 dst);
-    count_launch();
-    int rc = launch_status();
-    if (rc || t == n) return rc;
-    const double *src = bufA;
-    for (int q = n - t - 1; q >= 0; --q) {
-        const int64_t o = pow4(q), inner = int64_t(1) << (n - 1 - q);
-        double *d = (q == 0) ? out_dev : (src == bufA ? bufB : bufA);
-        contract_axis<<<grid_for(o * inner, 256), 256, 0, s>>>(src, o, inner, R, d);
-        count_launch();
-        if ((rc = launch_status())) return rc;
-        src = d;
-    }
-    return DM_OK;
+    // Every buffer element read is written earlier in the same call, so the array's contents from a
+    // previous call never leak into a result.
+    return nbasis(state_dev, n, dtype, nvec3, err, out_dev, scratch, as_stream(stream));
 }
