@@ -15,6 +15,8 @@
 // operations per coefficient instead of n.  Defer needs c to stay small (the
 // unscaled Z grows like g**-n), so it is used for g >= 1/2, which every
 // physical decay factor per cycle is; below that each axis is scaled at once.
+// Measured for all qubits: n = 13 FP64 672 us in three sweeps (6.8 ms as 13),
+// n = 14 FP32 1.32 ms in three (4.5 ms as 14, each at the HBM roof).
 #include <math.h>
 
 #include "dm_common.cuh"

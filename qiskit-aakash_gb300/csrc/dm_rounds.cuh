@@ -15,7 +15,8 @@ struct CxCoef {
 };
 
 // Row0: row 0 of the map is (1,0,0,0).  A compile-time choice: as a run-time one the compiler
-// computes row 0 anyway and selects, a quarter of the map's FP64 operations.
+// computes row 0 anyway and selects, a quarter of the map's FP64 operations
+// (a fused FP64 pass at n = 13: 3.58 -> 2.94 ms).
 template <bool Row0, typename T>
 __device__ __forceinline__ void map4(const T *m, T &x0, T &x1, T &x2, T &x3) {
     const T y0 = Row0 ? x0 : fma(m[0], x0, fma(m[1], x1, fma(m[2], x2, m[3] * x3)));

@@ -599,7 +599,9 @@ __global__ void __launch_bounds__(32 * kComposeWarps)
 }
 
 // The round images of several passes (CTA x = entry of the round table).  A pass's composition alone
-// is a launch of a few microseconds on a few dozen warps; one launch for many passes fills the chip.
+// is a launch of a few microseconds on a few dozen warps; one launch for many passes fills the chip
+// (20 passes of 10 qubits: 18-25 us each alone, 52 us together; 24 passes of the 14-qubit QFT: 20 us
+// per launch of up to 16).
 __global__ void __launch_bounds__(32 * kComposeWarps)
     compose_passes_kernel(const dm_batch_pass *__restrict__ passes, const dm_compose_round *__restrict__ rounds,
                           const double *__restrict__ mats, uint16_t *__restrict__ images) {
