@@ -350,8 +350,9 @@ typedef struct dm_batch_tc_pass {
     dm_tc_pass tables;
 } dm_batch_tc_pass;
 
-/* Device scratch dm_batch_run_tc needs for the round matrices it composes
- * (DM_MAX_ROUNDS FP16 image sets per CTA). */
+/* Device scratch dm_batch_run_tc needs: the round matrices it composes
+ * (DM_MAX_ROUNDS FP16 image sets per CTA), template coefficients and the
+ * counters of the groups of CTAs that share an instance. */
 size_t dm_batch_tc_scratch_bytes(void);
 
 /* dm_batch_run for FP32 instances of 7..12 qubits with every pass on the
@@ -359,7 +360,8 @@ size_t dm_batch_tc_scratch_bytes(void);
  * CTA composes the pass's round matrices from the instance's FP64
  * coefficient block (the ops applied to the 64 unit vectors, in FP64) into
  * its slice of scratch_dev as the 3-way FP16 split images, then streams the
- * instance's tiles.  status_dev is set to 1 if a bounded tensor-core wait
+ * instance's tiles.  Large instances of an uneven batch, and batches too small
+ * for the chip, run on several CTAs each (one or two launches).  status_dev is set to 1 if a bounded tensor-core wait
  * gives up. */
 int dm_batch_run_tc(float *states_dev, size_t states_count, double *probs_dev, size_t probs_count,
                     const double *mats_dev, size_t mats_count, const dm_batch_instance *insts_host,

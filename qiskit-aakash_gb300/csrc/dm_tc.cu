@@ -39,6 +39,7 @@
 // that the epilogue adds); warps 0-3 own the rows of M block 0 and warps 4-7
 // those of M block 1, one row per thread (TMEM lane quadrant = warp % 4).
 #include <cuda_fp16.h>
+#include <math.h>
 
 #include <mutex>
 
@@ -138,7 +139,7 @@ __device__ __forceinline__ void tc_teardown(TcCta &c) {
 // of the CTA); round r's images are at umats + p.rounds[r].umoff.  Returns
 // false when a bounded wait gave up (*status is then set).
 __device__ __forceinline__ bool tc_pass_tiles(float *__restrict__ st, const Pass &p,
-                                              const uint16_t *__restrict__ umats, int64_t t0, int64_t dt, TcCta &c,
+                                              const uint16_t *__restrict__ umats, int t0, int dt, TcCta &c,
                                               int *status) {
     unsigned char *AH = c.AH, *AL = c.AL, *B = c.B;
     uint64_t &mbar = *c.mbar;
@@ -148,21 +149,21 @@ __device__ __forceinline__ bool tc_pass_tiles(float *__restrict__ st, const Pass
     uint32_t phase = c.phase;
     bool pending = c.pending;
     const int tid = threadIdx.x, warp = tid >> 5;
-    const int64_t ntiles = int64_t(1) << (2 * p.m);
+    const int ntiles = 1 << (2 * p.m);   // at most 4**10
     const int64_t off_tid = tile_offset(p, 4 * tid);
     __syncthreads();   // earlier readers of hi_off are done
     for (int i = tid; i < kTile / 4 / kThreads; i += kThreads) hi_off[i] = tile_offset(p, 4 * kThreads * i);
     __syncthreads();
 
-    auto tile_base = [&](int64_t t) {
+    auto tile_base = [&](int t) {
         int64_t base = 0;
         for (int u = 0; u < p.m; ++u) {
-            base += (t & 3) * p.nonres_stride[u];
+            base += int64_t(t & 3) * p.nonres_stride[u];
             t >>= 2;
         }
         return base;
     };
-    auto load_tile = [&](int64_t t) {   // natural layout into AH / AL (64 KB)
+    auto load_tile = [&](int t) {   // natural layout into AH / AL (64 KB)
         const float *src = st + tile_base(t) + off_tid;
 #pragma unroll 8
         for (int i = 0; i < kTile / 4 / kThreads; ++i)
@@ -181,7 +182,7 @@ __device__ __forceinline__ bool tc_pass_tiles(float *__restrict__ st, const Pass
 
     load_u(0);
     bool loaded = false;   // the tile's load went out during the previous tile's last round
-    for (int64_t t = t0; t < ntiles; t += dt) {
+    for (int t = t0; t < ntiles; t += dt) {
         if (!loaded) load_tile(t);
         loaded = false;
         cp_async_wait_all();
@@ -385,46 +386,48 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
 // batched sweeps on the tensor cores
 // ---------------------------------------------------------------------------
 
-constexpr int64_t kScratchHalves = int64_t(DM_MAX_ROUNDS) * kUHalves;   // round images per CTA
+constexpr int64_t kScratchHalves = int64_t(DM_MAX_ROUNDS) * kUHalves;   // a pass's round images
 
-// Kernel parameters of one batched pass (thread 0 the scalars, all threads the rounds).
+// Kernel parameters of one batched pass, each field by a thread of its own (the pass table is in
+// global memory: one thread reading it field by field takes microseconds).
+static_assert(sizeof(Round) == sizeof(dm_tc_round), "a round's table is copied as words");
 __device__ void batch_tc_setup(Pass &ps, const dm_batch_tc_pass &bp, int n) {
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int nr = bp.ops.nrounds;
+    // the digit positions of the resident axes (local axis r = the r-th lowest)
+    unsigned resident = 0;
+#pragma unroll
+    for (int r = 0; r < kAxes; ++r) resident |= 1u << (n - 1 - bp.ops.axes[r]);
     if (tid == 0) {
         ps.n = n;
         ps.m = n - kAxes;
-        int low = 0;
-        while (low < kAxes && bp.ops.axes[low] == n - 1 - low) ++low;
-        ps.low = low;
-        ps.nrounds = bp.ops.nrounds;
+        ps.low = __ffs(~resident) - 1;
+        ps.nrounds = nr;
         ps.vec0 = bp.tables.vec0 == 0 ? 0 : -1;
         ps.direct = bp.tables.direct_last ? 1 : 0;
         ps.up = ldexpf(1.0f, n);
         ps.down = ldexpf(1.0f, -n);
-        unsigned resident = 0;
-        for (int r = 0; r < kAxes; ++r) {
-            resident |= 1u << bp.ops.axes[r];
-            ps.res_stride[r] = int64_t(1) << (2 * (n - 1 - bp.ops.axes[r]));
-        }
-        int m = 0;
-        for (int q = n - 1; q >= 0; --q)
-            if (!((resident >> q) & 1)) ps.nonres_stride[m++] = int64_t(1) << (2 * (n - 1 - q));
-        for (int i = 0; i < 8; ++i) ps.natrow[i] = bp.tables.natrow[i];
-        for (int i = 0; i < 6; ++i) ps.natk[i] = bp.tables.natk[i];
-        if (ps.direct) {
-            const dm_tc_round &L = bp.tables.rounds[bp.ops.nrounds - 1];
-            direct_offsets(ps, L.rowc, L.kc);
+    } else if (tid >= 32 && tid < 64) {
+        if (lane < kAxes) ps.res_stride[lane] = int64_t(1) << (2 * (n - 1 - bp.ops.axes[lane]));
+        // the lane-th lowest position that is not resident
+        if (lane < n && !((resident >> lane) & 1))
+            ps.nonres_stride[lane - __popc(resident & ((1u << lane) - 1))] = int64_t(1) << (2 * lane);
+    } else if (tid >= 64 && tid < 96) {
+        if (lane < 8) ps.natrow[lane] = bp.tables.natrow[lane];
+        else if (lane < 14) ps.natk[lane - 8] = bp.tables.natk[lane - 8];
+    } else if (tid >= 96 && tid < 128) {
+        if (lane < 14 && bp.tables.direct_last) {
+            // direct last round: the offset 2**b of tile bit b, bit b % 2 of local axis b / 2
+            const dm_tc_round &L = bp.tables.rounds[nr - 1];
+            const int bit = __ffs(lane < 8 ? L.rowc[lane] : L.kc[lane - 8]) - 1;
+            ps.lastg[lane] = (int64_t(1) << (2 * (n - 1 - bp.ops.axes[bit >> 1]))) << (bit & 1);
         }
     }
-    for (int r = tid; r < bp.ops.nrounds; r += kThreads) {
-        const dm_tc_round &in = bp.tables.rounds[r];
-        Round &o = ps.rounds[r];
-        for (int i = 0; i < 3; ++i) o.digits[i] = in.digits[i];
-        o.vec = in.vec;
-        o.umoff = int32_t(r * kUHalves);
-        for (int i = 0; i < 8; ++i) o.rowc[i] = in.rowc[i];
-        for (int i = 0; i < 6; ++i) o.kc[i] = in.kc[i];
-    }
+    const uint32_t *in = reinterpret_cast<const uint32_t *>(bp.tables.rounds);
+    uint32_t *out = reinterpret_cast<uint32_t *>(ps.rounds);
+    constexpr int kWords = sizeof(Round) / 4;
+    for (int i = tid; i < nr * kWords; i += kThreads)
+        out[i] = i % kWords == 1 ? uint32_t(i / kWords * kUHalves) : in[i];   // word 1: umoff
 }
 
 // Round r's matrix U (64 x 64 in its K-digit order) is the round's operations
@@ -453,8 +456,7 @@ static_assert(kColBytes <= int(kSmemBytes), "one round of FP64 columns fits the 
 // One operation on the warp's C columns (digit positions from the op flags).
 // Map2: 16x16 general maps too (the single-state passes; the batched plans hold none).
 template <bool Map2, int C>
-__device__ __forceinline__ void cols_apply(double *w, const dm_op &op, const double *__restrict__ mats, int lane) {
-    const double *mg = mats + op.moff;
+__device__ __forceinline__ void cols_apply(double *w, const dm_op &op, const double *__restrict__ mg, int lane) {
     const int da = (op.flags >> 8) & 3, db = (op.flags >> 12) & 3;
     if (op.kind == DM_OP_MAP1) {
         double m[16];
@@ -514,19 +516,19 @@ __device__ __forceinline__ void cols_apply(double *w, const dm_op &op, const dou
     for (int i = 0; i < 16; ++i) col[(i >> 2) * SA + (i & 3) * SB] = x[i];
 }
 
-// Columns k0 .. k0 + C - 1 of round r (k0 a multiple of C) by one warp, w its C columns of scratch;
-// the round's images at img (three or two of them).
-template <bool Map2, int C>
-__device__ void compose_warp(const dm_batch_pass &bp, int r, int k0, const double *__restrict__ mats, double *w,
+// Columns k0 .. k0 + C - 1 (k0 a multiple of C) of the round of operations ops[o] .. ops[oe - 1] by
+// one warp, w its C columns of scratch; the round's images at img (three or two of them).  Packed: op
+// o's coefficients are at mats + kCoefStride * o instead of mats + moff.
+template <bool Map2, bool Packed, int C>
+__device__ void compose_warp(const dm_op *ops, int o, int oe, int k0, const double *__restrict__ mats, double *w,
                              uint16_t *__restrict__ img, bool three, int lane) {
-    int o = r > 0 ? bp.round_end[r - 1] : 0;
-    const int oe = bp.round_end[r];
+    auto coef = [&](int i) { return mats + (Packed ? kCoefStride * i : ops[i].moff); };
     // the leading 4x4 maps, at most one per digit: their Kronecker product
     const double *lead[3] = {nullptr, nullptr, nullptr};
-    for (; o < oe && bp.ops[o].kind == DM_OP_MAP1; ++o) {
-        const int d = (bp.ops[o].flags >> 8) & 3;
+    for (; o < oe && ops[o].kind == DM_OP_MAP1; ++o) {
+        const int d = (ops[o].flags >> 8) & 3;
         if (d == 0 ? lead[0] != nullptr : d == 1 ? lead[1] != nullptr : lead[2] != nullptr) break;
-        const double *m = mats + bp.ops[o].moff;
+        const double *m = coef(o);
         if (d == 0) lead[0] = m;
         else if (d == 1) lead[1] = m;
         else lead[2] = m;
@@ -541,7 +543,7 @@ __device__ void compose_warp(const dm_batch_pass &bp, int r, int k0, const doubl
     }
     __syncwarp();
     for (; o < oe; ++o) {
-        cols_apply<Map2, C>(w, bp.ops[o], mats, lane);
+        cols_apply<Map2, C>(w, ops[o], coef(o), lane);
         __syncwarp();
     }
     // row j of the C columns: one chunk of C halves per image (16 bytes of 8 columns)
@@ -573,15 +575,206 @@ __device__ void compose_warp(const dm_batch_pass &bp, int r, int k0, const doubl
     __syncwarp();   // the columns are read before the next round's are written
 }
 
-// All rounds of a batched pass into per-CTA scratch (three images per round), all threads of the
-// CTA, each warp 8 columns; the pass's operand and matrix regions are free between passes.
-constexpr int kBatchCols = 64 / (kThreads / 32);
-__device__ void compose_rounds(const dm_batch_pass &bp, const double *__restrict__ mats, uint16_t *__restrict__ umats,
-                               double *work) {
+// This CTA's share of a batched pass's round images (three per round): the group's ranks take the
+// (round, columns) items in turn, warp by warp; the operand region is free between passes.  Alone a
+// CTA takes 8 columns per warp, which fills the lanes in pair operations; in a group 2, which spreads
+// a round over all SM quarters (one FP64 warp instruction per 64 cycles each).
+struct ComposeShared {                // behind the columns in the operand region
+    double coefs[DM_MAX_PASS_OPS * kCoefStride];
+    dm_op ops[DM_MAX_PASS_OPS];
+    int16_t round_end[DM_MAX_ROUNDS];
+};
+static_assert(kColBytes + sizeof(ComposeShared) <= kSmemBytes, "columns and operations fit the pass's shared memory");
+
+template <int C>
+__device__ void compose_items(const ComposeShared &cs, int nrounds, uint16_t *__restrict__ umats, double *work,
+                              int rank, int G) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int r = 0; r < bp.nrounds; ++r)
-        compose_warp<false, kBatchCols>(bp, r, warp * kBatchCols, mats, work + warp * kBatchCols * kColStride,
-                                        umats + int64_t(r) * kUHalves, true, lane);
+    for (int i = rank + G * warp; i < nrounds * (64 / C); i += G * (kThreads / 32)) {
+        const int r = i / (64 / C), k0 = i % (64 / C) * C;
+        compose_warp<false, true, C>(cs.ops, r > 0 ? cs.round_end[r - 1] : 0, cs.round_end[r], k0, cs.coefs,
+                                     work + warp * C * kColStride, umats + int64_t(r) * kUHalves, true, lane);
+    }
+}
+
+// The pass's operations and coefficients are copied to shared memory first: an operation's own read
+// from global memory would cost every warp a round trip per operation.
+__device__ __noinline__ void compose_share(const dm_batch_pass &bp, const double *mats, uint16_t *umats,
+                                           unsigned char *smem, int rank, int G) {
+    ComposeShared &cs = *reinterpret_cast<ComposeShared *>(smem + kColBytes);
+    const int nops = bp.nops, nr = bp.nrounds;
+    for (int i = threadIdx.x; i < nops * kCoefStride; i += kThreads) {
+        const dm_op &op = bp.ops[i / kCoefStride];
+        if (op.kind != DM_OP_CX || i % kCoefStride < 5) cs.coefs[i] = mats[op.moff + i % kCoefStride];
+    }
+    for (int i = threadIdx.x; i < nops * 4; i += kThreads)
+        reinterpret_cast<uint32_t *>(cs.ops)[i] = reinterpret_cast<const uint32_t *>(bp.ops)[i];
+    for (int i = threadIdx.x; i < nr; i += kThreads) cs.round_end[i] = bp.round_end[i];
+    __syncthreads();
+    double *work = reinterpret_cast<double *>(smem);
+    if (G < 8)
+        compose_items<8>(cs, nr, umats, work, rank, G);
+    else
+        compose_items<2>(cs, nr, umats, work, rank, G);
+}
+static_assert(sizeof(dm_op) == 16, "operations are copied as words");
+
+// ---------------------------------------------------------------------------
+// groups of CTAs
+//
+// G CTAs (a group) run one instance together: each takes every G-th tile of a
+// pass and its share of the round-matrix composition, with one barrier among
+// the group per pass.  One CTA per instance leaves a sweep waiting for its
+// largest instance (a 12-qubit, 47-layer one takes a CTA 0.4 s) and keeps 304
+// states in flight, far more than L2 holds; with groups the tail is a G-th of
+// that and up to 10 qubits the states in flight stay in L2 (19 groups of 16
+// CTAs x 4 MB).  Measured: a batch of 576 instances of 6-12 qubits whose
+// largest ones are the longest, 511 -> 362 ms; 1,024 points of a 10-qubit
+// template, 3.4 waves of CTAs, 79.5 -> 78.0 ms.  A pass costs a group about
+// 20 us beside its tiles (16 us each where two CTAs share an SM), so work that
+// fills the chip evenly stays at one CTA per instance.
+//
+// A cooperative launch does not take two CTAs per SM of a kernel that
+// allocates tensor memory, so groups form among CTAs that run already: a CTA
+// joins the group of its ticket, and the first member closes the group when it
+// is full or, with the chip shared and CTAs still to come, after kJoinNs with
+// the members it has (later ones leave).  A group therefore only ever waits
+// for running CTAs.  Every wait is bounded and ends in *status = 1.
+// ---------------------------------------------------------------------------
+
+struct GroupSync {
+    unsigned joined;                  // members so far, kClosed once the first member closed the group
+    unsigned size;                    // members of the closed group
+    unsigned arrived;                 // barrier arrivals since the launch began
+    int inst;                         // instance the group runs next
+    unsigned pad[28];                 // one 128-byte line per group
+};
+constexpr unsigned kClosed = 0x80000000u;
+constexpr uint64_t kJoinNs = 1000000;
+
+constexpr int kSegSlots = 512;        // template coefficients composed at a time (>= DM_MAX_PASS_OPS)
+constexpr int kMaxGroup = 32;
+constexpr int kBigQubits = 11, kBigGroup = 8;   // instances that several CTAs share in an uneven batch
+
+// The scratch buffer: round images (two sets per group, or one when a CTA is its own group),
+// template coefficients, group counters, the CTA tickets and the launch's abort flag.
+struct GroupScratch {
+    uint16_t *images;
+    double *coefs;
+    GroupSync *sync;
+    unsigned *tickets;
+    int *abort;
+};
+__host__ __device__ inline size_t scratch_images_bytes(int ctas) { return size_t(ctas) * size_t(kScratchHalves) * 2; }
+__host__ __device__ inline size_t scratch_coefs_bytes(int ctas) { return size_t(ctas) * kSegSlots * kCoefStride * 8; }
+__host__ __device__ inline size_t scratch_sync_bytes(int ctas) { return (size_t(ctas) + 1) * sizeof(GroupSync); }
+__host__ __device__ inline GroupScratch group_scratch(unsigned char *p, int ctas) {
+    GroupScratch g;
+    g.images = reinterpret_cast<uint16_t *>(p);
+    g.coefs = reinterpret_cast<double *>(p + scratch_images_bytes(ctas));
+    g.sync = reinterpret_cast<GroupSync *>(p + scratch_images_bytes(ctas) + scratch_coefs_bytes(ctas));
+    g.tickets = &(g.sync + ctas)->joined;
+    g.abort = &(g.sync + ctas)->inst;
+    return g;
+}
+
+// One CTA's place in its group (rank < 0: the group was closed without it).
+struct Group {
+    int id, G, rank;
+    GroupSync *sync;
+    int *abort;                       // set by any CTA whose wait gave up
+    unsigned epoch;                   // barriers passed
+};
+
+// Bounded wait of one thread for *word, read with acquire, to satisfy pred.
+template <typename Pred>
+__device__ __forceinline__ bool group_wait(const unsigned *word, const int *abort, uint64_t limit_ns, Pred pred) {
+    const uint64_t t0 = tcg::global_ns();
+    for (uint32_t it = 1;; ++it) {
+        unsigned v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
+        if (pred(v)) return true;
+        if ((it & 15) == 0) {
+            if (*static_cast<const volatile int *>(abort) != 0 || tcg::global_ns() - t0 > limit_ns ||
+                it >= tcg::kWaitPollCap)
+                return false;
+            __nanosleep(32);
+        }
+    }
+}
+
+// Joins a group of up to G CTAs (all threads; g in shared memory), or stays alone.
+template <bool Grouped>
+__device__ __forceinline__ void group_join(const GroupScratch &gs, int G, Group &g) {
+    if (threadIdx.x == 0 && !Grouped) {
+        g = Group{int(blockIdx.x), 1, 0, gs.sync + blockIdx.x, gs.abort, 0};
+    } else if (threadIdx.x == 0) {
+        const int id = int(atomicAdd(gs.tickets, 1u)) / G;
+        GroupSync *sync = gs.sync + id;
+        const unsigned old = atomicAdd(&sync->joined, 1u);
+        int rank = old & kClosed ? -1 : int(old), size = 0;
+        if (rank == 0) {
+            const bool full = group_wait(&sync->joined, gs.abort, kJoinNs, [&](unsigned v) { return v >= unsigned(G); });
+            const unsigned members = full ? unsigned(G) : atomicOr(&sync->joined, kClosed);
+            size = int(members < unsigned(G) ? members : unsigned(G));
+            __threadfence();
+            atomicExch(&sync->size, unsigned(size));
+        } else if (rank > 0) {
+            if (group_wait(&sync->size, gs.abort, tcg::kWaitLimitNs, [](unsigned v) { return v != 0; }))
+                size = int(*static_cast<volatile unsigned *>(&sync->size));
+            else
+                rank = -2;
+        }
+        g = Group{id, size, rank, sync, gs.abort, 0};
+    }
+    __syncthreads();
+}
+
+// Barrier of the group (all threads): what its CTAs wrote before is visible after.  False when a wait
+// gave up here or in another CTA of the launch.
+template <bool Grouped>
+__device__ __forceinline__ bool group_barrier(Group &g, int *ok_s) {
+    __syncthreads();
+    if (!Grouped) return true;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(&g.sync->arrived, 1u);
+        const unsigned want = (g.epoch += 1) * unsigned(g.G);
+        const bool ok = group_wait(&g.sync->arrived, g.abort, tcg::kWaitLimitNs,
+                                   [=](unsigned v) { return int(v - want) >= 0; });
+        __threadfence();
+        *ok_s = ok ? 1 : 0;
+    }
+    __syncthreads();
+    return *ok_s != 0;
+}
+
+// The group's next instance (all threads), or -1 when none is left, -2 when a wait gave up.
+template <bool Grouped>
+__device__ __forceinline__ int group_next(Group &g, int *counter, int ninst, int *inst_s, int *ok_s) {
+    if (threadIdx.x == 0 && (!Grouped || g.rank == 0)) {
+        const int i = atomicAdd(counter, 1);
+        if (Grouped) *static_cast<volatile int *>(&g.sync->inst) = i;
+        *inst_s = i;
+    }
+    if (!group_barrier<Grouped>(g, ok_s)) return -2;
+    if (Grouped) {
+        if (threadIdx.x == 0) *inst_s = *static_cast<volatile int *>(&g.sync->inst);
+        __syncthreads();
+    }
+    const int i = *inst_s;
+    return i < ninst ? i : -1;
+}
+
+// This CTA's part of |0...0>: 2**-n where every digit is I or Z.
+__device__ __forceinline__ void group_init_zero(float *st, int n, int rank, int G) {
+    const int64_t total = int64_t(1) << (2 * n);
+    const float amp = ldexpf(1.0f, -n);
+    for (int64_t e = (int64_t(rank) * kThreads + threadIdx.x) * 4; e < total; e += int64_t(G) * kThreads * 4) {
+        const uint64_t x = uint64_t(e) ^ (uint64_t(e) >> 1);
+        const float v = (x & 0x5555555555555554ull) == 0 ? amp : 0.0f;   // digit 0 of the four values: I, X, Y, Z
+        *reinterpret_cast<float4 *>(st + e) = make_float4(v, 0.0f, 0.0f, v);
+    }
 }
 
 // The single-state launches: CTA (r, c) takes the columns 8c .. 8c + 7 of a round, 2 per warp.
@@ -593,9 +786,10 @@ __global__ void __launch_bounds__(32 * kComposeWarps)
                         uint16_t *__restrict__ images, int image_halves) {
     __shared__ double cols[kComposeWarps * kComposeCols * kColStride];
     const int r = blockIdx.x, warp = threadIdx.x >> 5;
-    compose_warp<true, kComposeCols>(bp, r, (int(blockIdx.y) * kComposeWarps + warp) * kComposeCols, mats,
-                                     cols + warp * kComposeCols * kColStride, images + int64_t(r) * image_halves,
-                                     image_halves == kUHalves, threadIdx.x & 31);
+    compose_warp<true, false, kComposeCols>(bp.ops, r > 0 ? bp.round_end[r - 1] : 0, bp.round_end[r],
+                                            (int(blockIdx.y) * kComposeWarps + warp) * kComposeCols, mats,
+                                            cols + warp * kComposeCols * kColStride, images + int64_t(r) * image_halves,
+                                            image_halves == kUHalves, threadIdx.x & 31);
 }
 
 // The round images of several passes (CTA x = entry of the round table).  A pass's composition alone
@@ -608,101 +802,197 @@ __global__ void __launch_bounds__(32 * kComposeWarps)
     __shared__ double cols[kComposeWarps * kComposeCols * kColStride];
     const dm_compose_round e = rounds[blockIdx.x];
     const int warp = threadIdx.x >> 5;
-    compose_warp<true, kComposeCols>(passes[e.pass], e.round, (int(blockIdx.y) * kComposeWarps + warp) * kComposeCols,
-                                     mats + e.mats_off, cols + warp * kComposeCols * kColStride, images + e.image_off,
-                                     e.format == DM_IMAGE_TC, threadIdx.x & 31);
+    const dm_batch_pass &bp = passes[e.pass];
+    compose_warp<true, false, kComposeCols>(bp.ops, e.round > 0 ? bp.round_end[e.round - 1] : 0, bp.round_end[e.round],
+                                            (int(blockIdx.y) * kComposeWarps + warp) * kComposeCols, mats + e.mats_off,
+                                            cols + warp * kComposeCols * kColStride, images + e.image_off,
+                                            e.format == DM_IMAGE_TC, threadIdx.x & 31);
 }
 
+// Shared memory of the batched kernels beside the operand and matrix regions.  In a group the tile
+// routine is a call of its own (one per pass): inlined into the group's loops it has too few registers
+// and spills in the tile loop (10 % of a sweep); with the constants of a lone CTA it has enough.
+struct BatchShared {
+    Pass ps;
+    int64_t hi_off[kTile / 4 / kThreads];
+    uint64_t mbar;
+    uint32_t tmem, phase;
+    int pending, abort_s;
+};
+constexpr uint32_t kBatchSmemBytes = kSmemBytes + (sizeof(BatchShared) + 15) / 16 * 16;
+
+__device__ __forceinline__ bool batch_tiles_inline(float *st, const uint16_t *umats, int t0, int dt, int *status) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    BatchShared &b = *reinterpret_cast<BatchShared *>(smem + kSmemBytes);
+    TcCta c{smem, smem + kABytes, smem + 2 * kABytes, &b.mbar, b.hi_off, &b.abort_s, b.tmem, b.phase, b.pending != 0};
+    const bool ok = tc_pass_tiles(st, b.ps, umats, t0, dt, c, status);
+    __syncthreads();      // every thread has read phase and pending
+    if (threadIdx.x == 0) {
+        b.phase = c.phase;
+        b.pending = c.pending ? 1 : 0;
+    }
+    __syncthreads();
+    return ok;
+}
+
+__device__ __noinline__ bool batch_tiles_call(float *st, const uint16_t *umats, int t0, int dt, int *status) {
+    return batch_tiles_inline(st, umats, t0, dt, status);
+}
+
+template <bool Grouped>
+__device__ __forceinline__ bool batch_tiles(float *st, const uint16_t *umats, const Group &g, int *status) {
+    if constexpr (Grouped)
+        return batch_tiles_call(st, umats, g.rank, g.G, status);
+    else
+        return batch_tiles_inline(st, umats, 0, 1, status);
+}
+
+__device__ __forceinline__ BatchShared &batch_setup(unsigned char *smem) {
+    BatchShared &b = *reinterpret_cast<BatchShared *>(smem + kSmemBytes);
+    TcCta c{smem, smem + kABytes, smem + 2 * kABytes, &b.mbar, b.hi_off, &b.abort_s, 0, 0, false};
+    tc_setup(c, &b.tmem);
+    if (threadIdx.x == 0) b.phase = b.pending = 0;
+    __syncthreads();
+    return b;
+}
+
+__device__ __forceinline__ void batch_teardown(unsigned char *smem) {
+    BatchShared &b = *reinterpret_cast<BatchShared *>(smem + kSmemBytes);
+    __syncthreads();
+    TcCta c{smem, smem + kABytes, smem + 2 * kABytes, &b.mbar, b.hi_off, &b.abort_s, b.tmem, b.phase, b.pending != 0};
+    tc_teardown(c);
+}
+
+// Grouped: groups of up to G CTAs per instance; otherwise one CTA per instance (G = 1).
+template <bool Grouped>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
     batch_tc_kernel(float *__restrict__ states, double *__restrict__ probs, const double *__restrict__ mats,
                     const dm_batch_instance *__restrict__ insts, int ninst, const dm_batch_tc_pass *__restrict__ passes,
-                    int *counter, uint16_t *__restrict__ scratch, int *status) {
+                    int *counter, unsigned char *__restrict__ scratch, int ctas, int G, int *status) {
     extern __shared__ __align__(1024) unsigned char smem[];
-    __shared__ __align__(8) uint64_t mbar;
-    __shared__ uint32_t tmem_base_s;
-    __shared__ int64_t hi_off[kTile / 4 / kThreads];
-    __shared__ int abort_s;
-    __shared__ int inst_s;
-    __shared__ Pass ps;
-    TcCta c{smem, smem + kABytes, smem + 2 * kABytes, &mbar, hi_off, &abort_s, 0, 0, false};
-    tc_setup(c, &tmem_base_s);
-    uint16_t *umats = scratch + int64_t(blockIdx.x) * kScratchHalves;
-    const int tid = threadIdx.x;
-    for (;;) {
-        if (tid == 0) inst_s = atomicAdd(counter, 1);
+    __shared__ int inst_s, ok_s;
+    __shared__ Group g;
+    __shared__ dm_batch_instance I;
+    __shared__ unsigned npass_s;
+    BatchShared &b = batch_setup(smem);
+    group_join<Grouped>(group_scratch(scratch, ctas), G, g);
+    if (threadIdx.x == 0) npass_s = 0;
+    bool ok = g.rank != -2;
+    while (g.rank >= 0) {
+        const int ii = group_next<Grouped>(g, counter, ninst, &inst_s, &ok_s);
+        if (ii < 0) {
+            ok = ii == -1;
+            break;
+        }
+        if (threadIdx.x == 0) I = insts[ii];
         __syncthreads();
-        const int ii = inst_s;
-        if (ii >= ninst) break;
-        const dm_batch_instance I = insts[ii];
+        const int rank = Grouped ? g.rank : 0, members = Grouped ? g.G : 1;
         float *st = states + I.state_off;
-        batch_init_zero<float, kThreads>(st, I.n);
-        bool ok = true;
+        group_init_zero(st, I.n, rank, members);
         for (int pi = 0; pi < I.npasses && ok; ++pi) {
             const dm_batch_tc_pass &bp = passes[I.pass_begin + pi];
-            batch_tc_setup(ps, bp, I.n);
-            compose_rounds(bp.ops, mats + I.mats_off, umats, reinterpret_cast<double *>(smem));
-            __threadfence_block();
-            __syncthreads();
-            ok = tc_pass_tiles(st, ps, umats, 0, 1, c, status);
+            // in a group the next pass's images are composed while this one's are read: two sets
+            uint16_t *umats = group_scratch(scratch, ctas).images +
+                              int64_t(Grouped ? g.id * G + int(npass_s & 1) : g.id) * kScratchHalves;
+            batch_tc_setup(b.ps, bp, I.n);
+            compose_share(bp.ops, mats + I.mats_off, umats, smem, rank, members);
+            ok = group_barrier<Grouped>(g, &ok_s);
+            if (Grouped && threadIdx.x == 0) npass_s += 1;
+            if (ok) ok = batch_tiles<Grouped>(st, umats, g, status);
         }
+        if (ok) ok = group_barrier<Grouped>(g, &ok_s);
         if (!ok) break;
-        batch_z_readout<float, kThreads>(st, I.n, I.meas_err, probs + I.prob_off, reinterpret_cast<double *>(smem));
+        if (rank == 0)
+            batch_z_readout<float, kThreads>(st, I.n, I.meas_err, probs + I.prob_off, reinterpret_cast<double *>(smem));
     }
-    tc_teardown(c);
+    if (!ok && threadIdx.x == 0) {
+        atomicExch(g.abort, 1);
+        atomicExch(status, 1);
+    }
+    batch_teardown(smem);
 }
 
-// Template sweeps on the tensor cores: per instance and pass, the slots'
-// recipe chains are composed in FP64 (as in the CUDA-core template kernel)
-// into shared memory, the round matrices composed from those coefficients,
-// then the tiles streamed.  Slot s of the program is op s of the
-// concatenated tensor-core passes; op o of a pass reads coef + 16 o.
-constexpr int kCoefOffset = kColBytes;   // after the round of FP64 columns
-static_assert(kCoefOffset + DM_MAX_PASS_OPS * kCoefStride * 8 <= int(kSmemBytes), "slot coefficients fit");
-
+// Template sweeps on the tensor cores: per instance the slots' recipe chains
+// are composed in FP64, up to kSegSlots of them at a time and shared among the
+// group's threads, the round matrices from those coefficients, then the tiles
+// streamed.  Slot s of the program is op s of the concatenated tensor-core
+// passes; op o of a pass reads 16 coefficients at 16 o.
+template <bool Grouped>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
     batch_param_tc_kernel(float *__restrict__ states, double *__restrict__ probs, const dm_param_program P,
                           const dm_batch_tc_pass *__restrict__ passes, const double *__restrict__ params,
-                          int params_stride, int ninst, int *counter, uint16_t *__restrict__ scratch, int *status) {
+                          int params_stride, int ninst, int *counter, unsigned char *__restrict__ scratch, int ctas,
+                          int G, int *status) {
     extern __shared__ __align__(1024) unsigned char smem[];
-    __shared__ __align__(8) uint64_t mbar;
-    __shared__ uint32_t tmem_base_s;
-    __shared__ int64_t hi_off[kTile / 4 / kThreads];
-    __shared__ int abort_s;
-    __shared__ int inst_s;
-    __shared__ Pass ps;
+    __shared__ int inst_s, ok_s;
     __shared__ double prm[DM_PARAMS_MIN_STRIDE];
-    TcCta c{smem, smem + kABytes, smem + 2 * kABytes, &mbar, hi_off, &abort_s, 0, 0, false};
-    tc_setup(c, &tmem_base_s);
-    uint16_t *umats = scratch + int64_t(blockIdx.x) * kScratchHalves;
-    double *coef = reinterpret_cast<double *>(smem + kCoefOffset);
+    __shared__ Group g;
+    __shared__ int slot, seg_begin, seg_end;          // the pass's first slot; slots in coefs
+    __shared__ unsigned npass_s;
+    BatchShared &b = batch_setup(smem);
+    group_join<Grouped>(group_scratch(scratch, ctas), G, g);
     const int tid = threadIdx.x;
-    const int n = P.n;
-    for (;;) {
-        if (tid == 0) inst_s = atomicAdd(counter, 1);
-        __syncthreads();
-        const int ii = inst_s;
-        if (ii >= ninst) break;
+    if (tid == 0) npass_s = 0;
+    bool ok = g.rank != -2;
+    while (g.rank >= 0) {
+        const int ii = group_next<Grouped>(g, counter, ninst, &inst_s, &ok_s);
+        if (ii < 0) {
+            ok = ii == -1;
+            break;
+        }
         if (tid < DM_PARAMS_MIN_STRIDE) prm[tid] = params[int64_t(ii) * params_stride + tid];
-        float *st = states + (int64_t(ii) << (2 * n));
-        batch_init_zero<float, kThreads>(st, n);   // its barriers also publish prm
-        bool ok = true;
-        int slot_base = 0;
+        if (tid == 0) slot = seg_begin = seg_end = 0;
+        __syncthreads();
+        const int rank = Grouped ? g.rank : 0, members = Grouped ? g.G : 1;
+        float *st = states + (int64_t(ii) << (2 * P.n));
+        group_init_zero(st, P.n, rank, members);
         for (int pi = 0; pi < P.npasses && ok; ++pi) {
             const dm_batch_tc_pass &bp = passes[pi];
-            batch_tc_setup(ps, bp, n);
-            for (int o = tid; o < bp.ops.nops; o += kThreads)
-                compose_slot(P, slot_base + o, prm, coef + o * kCoefStride);
-            __syncthreads();
-            compose_rounds(bp.ops, coef, umats, reinterpret_cast<double *>(smem));
-            __threadfence_block();
-            __syncthreads();
-            ok = tc_pass_tiles(st, ps, umats, 0, 1, c, status);
-            slot_base += bp.ops.nops;
+            double *coefs = group_scratch(scratch, ctas).coefs + int64_t(g.id) * kSegSlots * kCoefStride;
+            if (slot + bp.ops.nops > seg_end) {
+                // the next passes' slots; the last barrier lies after every read of the previous ones
+                __syncthreads();
+                if (tid == 0) {
+                    int end = slot;
+                    for (int q = pi; q < P.npasses && end + passes[q].ops.nops - slot <= kSegSlots; ++q)
+                        end += passes[q].ops.nops;
+                    seg_begin = slot;
+                    seg_end = end;
+                }
+                __syncthreads();
+                for (int i = seg_begin + rank * kThreads + tid; i < seg_end; i += members * kThreads)
+                    compose_slot(P, i, prm, coefs + (i - seg_begin) * kCoefStride);
+                if (!(ok = group_barrier<Grouped>(g, &ok_s))) break;
+            }
+            uint16_t *umats = group_scratch(scratch, ctas).images +
+                              int64_t(Grouped ? g.id * G + int(npass_s & 1) : g.id) * kScratchHalves;
+            batch_tc_setup(b.ps, bp, P.n);
+            compose_share(bp.ops, coefs + (slot - seg_begin) * kCoefStride, umats, smem, rank, members);
+            ok = group_barrier<Grouped>(g, &ok_s);
+            if (tid == 0) {
+                npass_s += 1;
+                slot += bp.ops.nops;
+            }
+            if (ok) ok = batch_tiles<Grouped>(st, umats, g, status);
         }
+        if (ok) ok = group_barrier<Grouped>(g, &ok_s);
         if (!ok) break;
-        batch_z_readout<float, kThreads>(st, n, prm[11], probs + (int64_t(ii) << n), reinterpret_cast<double *>(smem));
+        if (rank == 0)
+            batch_z_readout<float, kThreads>(st, P.n, prm[11], probs + (int64_t(ii) << P.n),
+                                             reinterpret_cast<double *>(smem));
     }
-    tc_teardown(c);
+    if (!ok && tid == 0) {
+        atomicExch(g.abort, 1);
+        atomicExch(status, 1);
+    }
+    batch_teardown(smem);
+}
+
+// The largest power of two of CTAs per instance, up to kMaxGroup, that ninst instances keep busy.
+static int spread_group(int ctas, int ninst) {
+    int G = 1;
+    while (2 * G <= kMaxGroup && 2 * G * ninst <= ctas) G *= 2;
+    return G;
 }
 
 }  // namespace tc
@@ -818,7 +1108,22 @@ extern "C" int dm_apply_pass_tc(void *state_dev, int n, const dm_tc_pass *pass, 
 }
 
 extern "C" size_t dm_batch_tc_scratch_bytes(void) {
-    return size_t(sm_count()) * tc::kCtasPerSm * size_t(tc::kScratchHalves) * sizeof(uint16_t);
+    const int ctas = sm_count() * tc::kCtasPerSm;
+    return tc::scratch_images_bytes(ctas) + tc::scratch_coefs_bytes(ctas) + tc::scratch_sync_bytes(ctas);
+}
+
+// Clears the work counter and the group counters and launches a batched kernel on whole groups of CTAs.
+template <typename Kernel, typename... Args>
+static int launch_groups(Kernel kernel, int G, int ctas, int *counter_dev, void *scratch_dev, cudaStream_t s,
+                         Args... args) {
+    if (ensure_max_dynamic_smem(reinterpret_cast<const void *>(kernel), int(tc::kBatchSmemBytes)) != cudaSuccess)
+        return DM_ERR_CUDA;
+    DM_CUDA_TRY(cudaMemsetAsync(counter_dev, 0, sizeof(int), s));
+    DM_CUDA_TRY(cudaMemsetAsync(tc::group_scratch(static_cast<unsigned char *>(scratch_dev), ctas).sync, 0,
+                                tc::scratch_sync_bytes(ctas), s));
+    kernel<<<ctas / G * G, tc::kThreads, tc::kBatchSmemBytes, s>>>(args...);
+    count_launch();
+    return launch_status();
 }
 
 // The rounds and operations of a tensor-core pass (round_axes[r][0..2] the
@@ -949,17 +1254,33 @@ extern "C" int dm_batch_run_tc(float *states_dev, size_t states_count, double *p
         }
     }
     if (scratch_bytes < dm_batch_tc_scratch_bytes()) return DM_ERR_ARG;
-    if (ensure_max_dynamic_smem(reinterpret_cast<const void *>(tc::batch_tc_kernel), int(tc::kSmemBytes)) !=
-        cudaSuccess)
-        return DM_ERR_CUDA;
-    cudaStream_t s = as_stream(stream);
-    DM_CUDA_TRY(cudaMemsetAsync(counter_dev, 0, sizeof(int), s));
-    const int grid = sm_count() * tc::kCtasPerSm;
-    tc::batch_tc_kernel<<<grid, tc::kThreads, tc::kSmemBytes, s>>>(states_dev, probs_dev, mats_dev, insts_dev, ninst,
-                                                                     passes_dev, counter_dev,
-                                                                     static_cast<uint16_t *>(scratch_dev), status_dev);
-    count_launch();
-    return launch_status();
+    // One CTA per instance is the faster form while the work is even: a batch then takes its total over
+    // the CTAs.  It cannot take less than its largest instance, so where that is the longer of the two
+    // (4096 mixed instances: 0.65 of the total's share; 576: 1.8) the leading large ones (the caller
+    // orders them largest first) run on groups of kBigGroup; and what does not fill the chip, on
+    // groups that do.
+    const int ctas = sm_count() * tc::kCtasPerSm;
+    double total = 0, largest = 0;
+    int big = 0;
+    for (int i = 0; i < ninst; ++i) {
+        const double w = ldexp(double(insts_host[i].npasses), 2 * insts_host[i].n);
+        total += w;
+        largest = w > largest ? w : largest;
+        if (big == i && insts_host[i].n >= tc::kBigQubits) ++big;
+    }
+    if (largest * ctas <= total) big = 0;
+    for (int part = 0; part < 2; ++part) {
+        const int begin = part ? big : 0, count = part ? ninst - big : big;
+        if (count == 0) continue;
+        int G = tc::spread_group(ctas, count);
+        if (!part && G < tc::kBigGroup) G = tc::kBigGroup;
+        const int e = launch_groups(G > 1 ? tc::batch_tc_kernel<true> : tc::batch_tc_kernel<false>, G, ctas, counter_dev,
+                                    scratch_dev, as_stream(stream), states_dev, probs_dev, mats_dev, insts_dev + begin,
+                                    count, passes_dev, counter_dev, static_cast<unsigned char *>(scratch_dev), ctas, G,
+                                    status_dev);
+        if (e) return e;
+    }
+    return DM_OK;
 }
 
 extern "C" int dm_batch_run_params_tc(const dm_param_program *host, const dm_param_program *dev,
@@ -991,15 +1312,19 @@ extern "C" int dm_batch_run_params_tc(const dm_param_program *host, const dm_par
     if (size_t(ninst) * (size_t(1) << (2 * P.n)) > states_count) return DM_ERR_ARG;
     if (size_t(ninst) * (size_t(1) << P.n) > probs_count) return DM_ERR_ARG;
     if (scratch_bytes < dm_batch_tc_scratch_bytes()) return DM_ERR_ARG;
-    if (ensure_max_dynamic_smem(reinterpret_cast<const void *>(tc::batch_param_tc_kernel), int(tc::kSmemBytes)) !=
-        cudaSuccess)
-        return DM_ERR_CUDA;
-    cudaStream_t s = as_stream(stream);
-    DM_CUDA_TRY(cudaMemsetAsync(counter_dev, 0, sizeof(int), s));
-    const int grid = sm_count() * tc::kCtasPerSm;
-    tc::batch_param_tc_kernel<<<grid, tc::kThreads, tc::kSmemBytes, s>>>(
-        states_dev, probs_dev, *dev, passes_dev, params_dev, params_stride, ninst, counter_dev,
-        static_cast<uint16_t *>(scratch_dev), status_dev);
-    count_launch();
-    return launch_status();
+    // whole waves of one instance per CTA, then what is left on groups that fill the chip
+    const int ctas = sm_count() * tc::kCtasPerSm;
+    const int whole = tc::spread_group(ctas, ninst % ctas) > 1 ? ninst / ctas * ctas : ninst;
+    for (int part = 0; part < 2; ++part) {
+        const int begin = part ? whole : 0, count = part ? ninst - whole : whole;
+        if (count == 0) continue;
+        const int G = part ? tc::spread_group(ctas, count) : 1;
+        const int e = launch_groups(
+            G > 1 ? tc::batch_param_tc_kernel<true> : tc::batch_param_tc_kernel<false>, G, ctas, counter_dev, scratch_dev, as_stream(stream),
+            states_dev + (int64_t(begin) << (2 * P.n)), probs_dev + (int64_t(begin) << P.n), *dev, passes_dev,
+            params_dev + int64_t(begin) * params_stride, params_stride, count, counter_dev,
+            static_cast<unsigned char *>(scratch_dev), ctas, G, status_dev);
+        if (e) return e;
+    }
+    return DM_OK;
 }
