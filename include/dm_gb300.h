@@ -507,6 +507,44 @@ int dm_mlp_gather(const float *features, int nfeat, const float *targets, int no
                   const int32_t *index, int rows, int members, int width, uint16_t *x, uint16_t *xt, float *t,
                   void *stream);
 
+/* The surrogate network as a whole: `members` networks 64 -> 256 -> 256 ->
+ * 256 -> nout (nout % 256 == 0, nout <= 4096) with their buffers for
+ * minibatches of up to `batch` rows (batch % 128 == 0).  Device pointers, each
+ * 16-byte aligned; every buffer is [members][...] and a member's rows lie
+ * `batch` rows apart whatever the call's row count.  count is a member's
+ * parameter count (W1 b1 ... W4 b4, W row-major [out x in]); wb / wtb the BF16
+ * copies that dm_mlp_adam keeps.  Inference needs params, wb, x, h, logits
+ * and status; training all but probs, which may be NULL. */
+typedef struct dm_mlp_net {
+    int32_t members, batch, nout, pad;
+    int64_t count;
+    float *params, *grads, *m, *v;
+    uint16_t *wb, *wtb;
+    uint16_t *x, *xt;                  /* [batch][64], [64][batch] */
+    float *pre[3];                     /* [batch][256] */
+    uint16_t *h[3], *ht[3];            /* [batch][256], [256][batch] */
+    float *logits, *t;                 /* [batch][nout] */
+    uint16_t *dz, *dzt;                /* [batch][nout], [nout][batch] */
+    uint16_t *du[3], *dut[3];          /* [batch][256], [256][batch] */
+    float *loss_rows, *probs;          /* [batch], [batch][nout] */
+    int *status;
+} dm_mlp_net;
+
+/* Logits of the first `rows` rows of x; train != 0 also keeps pre, ht. */
+int dm_mlp_forward(const dm_mlp_net *net, int rows, int train, void *stream);
+/* grads from dz / dzt and the forward pass's buffers (rows % 64 == 0). */
+int dm_mlp_backward(const dm_mlp_net *net, int rows, void *stream);
+/* Forward pass, softmax with the mean KL loss against t, backward pass. */
+int dm_mlp_loss_and_grads(const dm_mlp_net *net, int rows, void *stream);
+/* One training step on the minibatch index [members][batch]: dm_mlp_gather,
+ * dm_mlp_loss_and_grads and dm_mlp_adam (step >= 1). */
+int dm_mlp_train_step(const dm_mlp_net *net, const float *features, int nfeat, const float *targets,
+                      int64_t samples, const int32_t *index, float lr, float beta1, float beta2, float eps,
+                      int step, void *stream);
+/* Member distributions out[members][samples][nout] of every feature row. */
+int dm_mlp_predict(const dm_mlp_net *net, const float *features, int nfeat, int64_t samples, float *out,
+                   void *stream);
+
 /* Ensemble statistics of probs [members][rows][nout]: mean [rows][nout],
  * spread[r] = mean over members of TV(q_member, mean) and, with ref
  * [rows][nout], tv_ref[r] = TV(mean, ref).  members <= 8. */

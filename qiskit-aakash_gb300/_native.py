@@ -166,6 +166,16 @@ class DmMlpGemm(ctypes.Structure):
                 ('out_t', ctypes.c_void_p), ('ld_t', ctypes.c_int64), ('t_ms', ctypes.c_int64)]
 
 
+class DmMlpNet(ctypes.Structure):
+    _fields_ = [('members', ctypes.c_int32), ('batch', ctypes.c_int32), ('nout', ctypes.c_int32),
+                ('pad', ctypes.c_int32), ('count', ctypes.c_int64)] + \
+        [(f, ctypes.c_void_p) for f in ('params', 'grads', 'm', 'v', 'wb', 'wtb', 'x', 'xt')] + \
+        [('pre', ctypes.c_void_p * 3), ('h', ctypes.c_void_p * 3), ('ht', ctypes.c_void_p * 3)] + \
+        [(f, ctypes.c_void_p) for f in ('logits', 't', 'dz', 'dzt')] + \
+        [('du', ctypes.c_void_p * 3), ('dut', ctypes.c_void_p * 3)] + \
+        [(f, ctypes.c_void_p) for f in ('loss_rows', 'probs', 'status')]
+
+
 DM_MLP_EPI_GELU_FWD, DM_MLP_EPI_BIAS_F32, DM_MLP_EPI_GELU_BWD, DM_MLP_EPI_F32 = 0, 1, 2, 3
 
 _vp = ctypes.c_void_p
@@ -213,6 +223,12 @@ SIGNATURES = {
     'dm_mlp_adam': (_i, [_vp, _vp, _vp, _vp, ctypes.c_int64, _i, ctypes.POINTER(ctypes.c_int32), _i, ctypes.c_float,
                          ctypes.c_float, ctypes.c_float, ctypes.c_float, _i, _vp, _vp, _vp]),
     'dm_mlp_gather': (_i, [_vp, _i, _vp, _i, ctypes.c_int64, _vp, _i, _i, _i, _vp, _vp, _vp, _vp]),
+    'dm_mlp_forward': (_i, [ctypes.POINTER(DmMlpNet), _i, _i, _vp]),
+    'dm_mlp_backward': (_i, [ctypes.POINTER(DmMlpNet), _i, _vp]),
+    'dm_mlp_loss_and_grads': (_i, [ctypes.POINTER(DmMlpNet), _i, _vp]),
+    'dm_mlp_train_step': (_i, [ctypes.POINTER(DmMlpNet), _vp, _i, _vp, ctypes.c_int64, _vp, ctypes.c_float,
+                               ctypes.c_float, ctypes.c_float, ctypes.c_float, _i, _vp]),
+    'dm_mlp_predict': (_i, [ctypes.POINTER(DmMlpNet), _vp, _i, ctypes.c_int64, _vp, _vp]),
     'dm_mlp_ensemble': (_i, [_vp, _i, _i, _i, _vp, _vp, _vp, _vp, _vp]),
     'dm_axis_probs': (_i, [_vp, _i, _i, _ip, _d, _vp, _vp]),
     'dm_nbasis_probs_scratch_bytes': (_sz, [_i]),

@@ -150,8 +150,8 @@ class MLPEnsemble:
         K = self.nout
         self.logits, self.t = z(M, B, K), z(M, B, K)
         self.dz, self.dzt = z(M, B, K, dt=bf), z(M, K, B, dt=bf)
-        self.du = [z(M, B, 256, dt=bf) for _ in range(2)]
-        self.dut = [z(M, 256, B, dt=bf) for _ in range(2)]
+        self.du = [z(M, B, 256, dt=bf) for _ in range(3)]
+        self.dut = [z(M, 256, B, dt=bf) for _ in range(3)]
         self.loss_rows = z(M, B)
         self.probs = z(M, B, K)
 
@@ -191,27 +191,16 @@ class MLPEnsemble:
         import torch
         return ctypes.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)
 
-    def _gemm(self, epi, M, Nn, K, A, lda, a_ms, Bm, ldb, b_ms, bias=None, pre=None, out_f32=None, ld_f32=0,
-              f32_ms=0, out_bf16=None, out_t=None):
-        g = N.DmMlpGemm()
-        g.epi, g.M, g.N, g.K, g.members = epi, M, Nn, K, self.M
-        g.A, g.lda, g.a_ms = A, lda, a_ms
-        g.B, g.ldb, g.b_ms = Bm, ldb, b_ms
-        if bias is not None:
-            g.bias, g.bias_ms = bias, self.P
-        if pre is not None:
-            g.pre, g.ld_pre, g.pre_ms = pre.data_ptr(), pre.shape[2], pre.shape[1] * pre.shape[2]
-        if out_f32 is not None:
-            g.out_f32, g.ld_f32, g.f32_ms = out_f32, ld_f32, f32_ms
-        if out_bf16 is not None:
-            g.out_bf16, g.ld_bf16, g.bf16_ms = out_bf16.data_ptr(), out_bf16.shape[2], out_bf16.shape[1] * out_bf16.shape[2]
-        if out_t is not None:
-            g.out_t, g.ld_t, g.t_ms = out_t.data_ptr(), out_t.shape[2], out_t.shape[1] * out_t.shape[2]
-        N.call('dm_mlp_gemm_run', ctypes.byref(g), ctypes.c_void_p(self.status.data_ptr()), self._stream())
-
-    def _w(self, li, transposed=False):
-        base = (self.wtb if transposed else self.wb).data_ptr()
-        return base + 2 * self.layers[li][0]
+    def _net(self):
+        """The network's description for the library, from the buffers as they are now."""
+        net = N.DmMlpNet()
+        net.members, net.batch, net.nout, net.count = self.M, self.bufB, self.nout, self.P
+        for f in ('params', 'grads', 'm', 'v', 'wb', 'wtb', 'x', 'xt', 'logits', 't', 'dz', 'dzt', 'loss_rows',
+                  'probs', 'status'):
+            setattr(net, f, getattr(self, f).data_ptr())
+        for f in ('pre', 'h', 'ht', 'du', 'dut'):
+            setattr(net, f, (ctypes.c_void_p * 3)(*[b.data_ptr() for b in getattr(self, f)]))
+        return ctypes.byref(net)
 
     def _adam(self, step, lr, beta1=0.9, beta2=0.999, eps=1e-8):
         vp = ctypes.c_void_p
@@ -222,44 +211,11 @@ class MLPEnsemble:
 
     def forward(self, rows, train):
         """Forward pass of the members on self.x (rows <= batch); logits in self.logits."""
-        f32 = 4
-        P, B, K = self.P, self.bufB, self.nout
-        E = N.DM_MLP_EPI_GELU_FWD
-        A, lda, ams = self.x.data_ptr(), 64, B * 64
-        for li in range(3):
-            inp = self.widths[li]
-            self._gemm(E, rows, 256, inp, A, lda, ams, self._w(li), inp, P, bias=self.params.data_ptr() + f32 * self.layers[li][1],
-                       out_f32=self.pre[li].data_ptr() if train else None, ld_f32=256, f32_ms=B * 256,
-                       out_bf16=self.h[li], out_t=self.ht[li] if train else None)
-            A, lda, ams = self.h[li].data_ptr(), 256, B * 256
-        self._gemm(N.DM_MLP_EPI_BIAS_F32, rows, K, 256, A, lda, ams, self._w(3), 256, P,
-                   bias=self.params.data_ptr() + f32 * self.layers[3][1], out_f32=self.logits.data_ptr(), ld_f32=K,
-                   f32_ms=B * K)
+        N.call('dm_mlp_forward', self._net(), rows, int(bool(train)), self._stream())
 
     def backward(self, rows):
         """Gradients of the mean KL loss (self.dz / self.dzt already hold dL/dz) into self.grads."""
-        vp = ctypes.c_void_p
-        f32 = 4
-        P, B, K = self.P, self.bufB, self.nout
-        g0 = self.grads.data_ptr()
-        # output layer
-        self._gemm(N.DM_MLP_EPI_F32, K, 256, rows, self.dzt.data_ptr(), B, K * B, self.ht[2].data_ptr(), B,
-                   256 * B, out_f32=g0 + f32 * self.layers[3][0], ld_f32=256, f32_ms=P)
-        N.call('dm_mlp_bias_grad', vp(self.dzt.data_ptr()), ctypes.c_int64(B), ctypes.c_int64(K * B), K, rows,
-               self.M, vp(g0 + f32 * self.layers[3][1]), ctypes.c_int64(P), self._stream())
-        dA, lda, ams, inw = self.dz.data_ptr(), K, B * K, K
-        for li in (2, 1, 0):
-            cur = (2 - li) % 2
-            # dU_li = (d_next @ W_{li+1}) * gelu'(pre_li)
-            self._gemm(N.DM_MLP_EPI_GELU_BWD, rows, 256, inw, dA, lda, ams, self._w(li + 1, True), inw, P,
-                       pre=self.pre[li], out_bf16=self.du[cur], out_t=self.dut[cur])
-            prev_t = self.ht[li - 1].data_ptr() if li > 0 else self.xt.data_ptr()
-            width_in = self.widths[li]
-            self._gemm(N.DM_MLP_EPI_F32, 256, width_in, rows, self.dut[cur].data_ptr(), B, 256 * B, prev_t, B,
-                       width_in * B, out_f32=g0 + f32 * self.layers[li][0], ld_f32=width_in, f32_ms=P)
-            N.call('dm_mlp_bias_grad', vp(self.dut[cur].data_ptr()), ctypes.c_int64(B), ctypes.c_int64(256 * B), 256,
-                   rows, self.M, vp(g0 + f32 * self.layers[li][1]), ctypes.c_int64(P), self._stream())
-            dA, lda, ams, inw = self.du[cur].data_ptr(), 256, B * 256, 256
+        N.call('dm_mlp_backward', self._net(), rows, self._stream())
 
     def gather(self, feats, targets, index, rows):
         vp = ctypes.c_void_p
@@ -269,18 +225,15 @@ class MLPEnsemble:
 
     def loss_and_grads(self, rows):
         """Forward + softmax/KL + backward on the gathered minibatch (self.x, self.t)."""
-        vp = ctypes.c_void_p
-        self.forward(rows, True)
-        N.call('dm_mlp_softmax_xent', vp(self.logits.data_ptr()), vp(self.t.data_ptr()), rows, self.M, self.nout,
-               ctypes.c_float(1.0 / rows), vp(self.probs.data_ptr()), vp(self.dz.data_ptr()),
-               vp(self.dzt.data_ptr()), vp(self.loss_rows.data_ptr()), self._stream())
-        self.backward(rows)
+        N.call('dm_mlp_loss_and_grads', self._net(), rows, self._stream())
 
     def train_step(self, feats, targets, index, lr):
-        self.gather(feats, targets, index, self.B)
-        self.loss_and_grads(self.B)
-        self.step_count += 1
-        self._adam(self.step_count, lr)
+        vp = ctypes.c_void_p
+        step = self.step_count + 1
+        N.call('dm_mlp_train_step', self._net(), vp(feats.data_ptr()), N_FEATURES, vp(targets.data_ptr()),
+               ctypes.c_int64(feats.shape[0]), vp(index.data_ptr()), ctypes.c_float(lr), ctypes.c_float(0.9),
+               ctypes.c_float(0.999), ctypes.c_float(1e-8), step, self._stream())
+        self.step_count = step
 
     def fit(self, feats, targets, epochs, lr=2e-3, lr_min=2e-5, seed=0, log_every=0):
         """Train every member on (feats [S, 6], targets [S, 1024]) device tensors; own shuffles per member."""
@@ -314,18 +267,8 @@ class MLPEnsemble:
         S = feats.shape[0]
         out = torch.empty((self.M, S, self.nout), dtype=torch.float32, device=self.device)
         vp = ctypes.c_void_p
-        for s0 in range(0, S, self.B):
-            rows = min(self.B, S - s0)
-            padded = ((rows + 127) // 128) * 128
-            idx = torch.arange(s0, s0 + padded, device=self.device, dtype=torch.int32).clamp_(max=S - 1)
-            idx = idx.unsqueeze(0).expand(self.M, padded).contiguous()
-            N.call('dm_mlp_gather', vp(feats.data_ptr()), N_FEATURES, None, self.nout, ctypes.c_int64(S),
-                   vp(idx.data_ptr()), padded, self.M, 64, vp(self.x.data_ptr()), vp(self.xt.data_ptr()), None,
-                   self._stream())
-            self.forward(padded, False)
-            N.call('dm_mlp_softmax_xent', vp(self.logits.data_ptr()), None, padded, self.M, self.nout, ctypes.c_float(1.0),
-                   vp(self.probs.data_ptr()), None, None, None, self._stream())
-            out[:, s0:s0 + rows] = self.probs[:, :rows]
+        N.call('dm_mlp_predict', self._net(), vp(feats.data_ptr()), N_FEATURES, ctypes.c_int64(S), vp(out.data_ptr()),
+               self._stream())
         return out
 
     def ensemble(self, member_probs, ref=None):

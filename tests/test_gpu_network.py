@@ -1,0 +1,158 @@
+"""The surrogate network's kernels at the edges of their tiles: chunk counts around the GEMM's stages,
+rows that do not fill a softmax CTA, weight shapes that do not fill an Adam tile, ragged predictions.
+
+Tolerances: BF16 products are exact in FP32, so a GEMM of K terms is held to K * 2**-24 times the sum
+of the terms' magnitudes; softmax and KL sums to (nout + 16) * 2**-24 times theirs."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from oracle import mlp_oracle as MO
+from qiskit_aakash_gb300 import _native as N
+from qiskit_aakash_gb300 import surrogate as S
+
+pytestmark = pytest.mark.gpu
+U = 2.0 ** -24
+
+
+def _torch():
+    import torch
+    return torch
+
+
+def _bf16(a):
+    r = MO.bf16(a).astype(np.float32).view(np.uint32) >> 16
+    return _torch().from_numpy(r.astype(np.uint16).view(np.int16)).cuda()
+
+
+def _f(t):
+    return (t.cpu().numpy().view(np.uint16).astype(np.uint32) << 16).view(np.float32)
+
+
+@pytest.mark.parametrize('K', [64, 128, 192, 256, 320, 448])
+@pytest.mark.parametrize('aligned', [True, False])
+def test_gemm_stages_and_transposed_copy(K, aligned):
+    """1 to 7 chunks through the stages; the transposed copy with and without 16-byte alignment."""
+    torch = _torch()
+    M, Nn, Z = 256, 128, 2
+    rng = np.random.default_rng(K)
+    A = MO.bf16(rng.normal(size=(Z, M, K)).astype(np.float32))
+    B = MO.bf16(rng.normal(size=(Z, Nn, K)).astype(np.float32))
+    pre = rng.normal(size=(Z, M, Nn)).astype(np.float32)
+    a, b, pt = _bf16(A), _bf16(B), torch.from_numpy(pre).cuda()
+    ld = M + (0 if aligned else 1)
+    f32 = torch.zeros((Z, M, Nn), dtype=torch.float32, device='cuda')
+    bf = torch.zeros((Z, M, Nn), dtype=torch.int16, device='cuda')
+    t = torch.zeros((Z, Nn, ld), dtype=torch.int16, device='cuda')
+    status = torch.zeros(1, dtype=torch.int32, device='cuda')
+    for epi in (N.DM_MLP_EPI_F32, N.DM_MLP_EPI_GELU_BWD):
+        g = N.DmMlpGemm()
+        g.epi, g.M, g.N, g.K, g.members = epi, M, Nn, K, Z
+        g.A, g.lda, g.a_ms, g.B, g.ldb, g.b_ms = a.data_ptr(), K, M * K, b.data_ptr(), K, Nn * K
+        if epi == N.DM_MLP_EPI_F32:
+            g.out_f32, g.ld_f32, g.f32_ms = f32.data_ptr(), Nn, M * Nn
+        else:
+            g.pre, g.ld_pre, g.pre_ms = pt.data_ptr(), Nn, M * Nn
+            g.out_bf16, g.ld_bf16, g.bf16_ms = bf.data_ptr(), Nn, M * Nn
+            g.out_t, g.ld_t, g.t_ms = t.data_ptr(), ld, Nn * ld
+        N.call('dm_mlp_gemm_run', ctypes.byref(g), ctypes.c_void_p(status.data_ptr()), None)
+    assert int(status.item()) == 0
+    A64, B64 = A.astype(np.float64), B.astype(np.float64)
+    want = np.einsum('zmk,znk->zmn', A64, B64)
+    terms = np.einsum('zmk,znk->zmn', np.abs(A64), np.abs(B64))
+    assert np.all(np.abs(f32.cpu().numpy() - want) <= K * U * terms)
+    d = want * MO.gelu_grad(pre.astype(np.float64))
+    # one BF16 rounding of the FP32 result (GELU' itself to a few FP32 units of 1)
+    assert np.all(np.abs(_f(bf) - d) <= 2.0 ** -8 * np.abs(d) + (K + 32) * U * terms)
+    assert np.array_equal(bf.cpu().numpy(), np.swapaxes(t.cpu().numpy()[:, :, :M], 1, 2))
+
+
+@pytest.mark.parametrize('rows', [1, 31, 32, 40, 100])
+@pytest.mark.parametrize('nout', [256, 1024, 4096])
+def test_softmax_rows(rows, nout):
+    torch = _torch()
+    Z = 2
+    rng = np.random.default_rng(rows + nout)
+    x = (3 * rng.normal(size=(Z, rows, nout))).astype(np.float32)
+    t = rng.dirichlet(np.ones(nout) * 0.3, size=(Z, rows)).astype(np.float32)
+    lx, lt = torch.from_numpy(x).cuda(), torch.from_numpy(t).cuda()
+    probs = torch.zeros_like(lx)
+    dz = torch.zeros((Z, rows, nout), dtype=torch.int16, device='cuda')
+    dzt = torch.zeros((Z, nout, rows), dtype=torch.int16, device='cuda')
+    loss = torch.zeros((Z, rows), dtype=torch.float32, device='cuda')
+    vp = ctypes.c_void_p
+    N.call('dm_mlp_softmax_xent', vp(lx.data_ptr()), vp(lt.data_ptr()), rows, Z, nout, ctypes.c_float(0.25),
+           vp(probs.data_ptr()), vp(dz.data_ptr()), vp(dzt.data_ptr()), vp(loss.data_ptr()), None)
+    x64 = x.astype(np.float64)
+    lq = x64 - x64.max(axis=2, keepdims=True)
+    lq -= np.log(np.exp(lq).sum(axis=2, keepdims=True))
+    q = np.exp(lq)
+    tol = (nout + 16) * U
+    got = probs.cpu().numpy()
+    # the exponent's own FP32 rounding (|x| < 40) beside the sum's
+    assert np.all(np.abs(got - q) <= (tol + 64 * U) * q)
+    t64 = t.astype(np.float64)
+    terms = np.where(t64 > 0, t64 * (np.log(np.where(t64 > 0, t64, 1.0)) - lq), 0.0)
+    assert np.all(np.abs(loss.cpu().numpy() - terms.sum(axis=2)) <= (tol + 64 * U) * (np.abs(terms).sum(axis=2) + 1))
+    d = (q - t64) * 0.25
+    assert np.all(np.abs(_f(dz) - d) <= 2.0 ** -8 * np.abs(d) + (tol + 64 * U) * q)
+    assert np.array_equal(dz.cpu().numpy(), np.swapaxes(dzt.cpu().numpy(), 1, 2))
+
+
+def test_adam_of_ragged_shapes():
+    torch = _torch()
+    shapes = [(5, 7), (33, 64), (64, 33), (300, 32), (1, 1)]
+    P = sum(o * i + o for o, i in shapes)
+    Z = 3
+    rng = np.random.default_rng(1)
+    p0 = rng.normal(size=(Z, P)).astype(np.float32)
+    g = rng.normal(size=(Z, P)).astype(np.float32)
+    p, gd = torch.from_numpy(p0).cuda(), torch.from_numpy(g).cuda()
+    m, v = torch.zeros_like(p), torch.zeros_like(p)
+    wb = torch.full((Z, P), 7, dtype=torch.int16, device='cuda')
+    wtb = torch.full((Z, P), 7, dtype=torch.int16, device='cuda')
+    flat = (ctypes.c_int32 * (2 * len(shapes)))(*[x for s in shapes for x in s])
+    vp = ctypes.c_void_p
+    N.call('dm_mlp_adam', vp(p.data_ptr()), vp(gd.data_ptr()), vp(m.data_ptr()), vp(v.data_ptr()), ctypes.c_int64(P),
+           Z, flat, len(shapes), ctypes.c_float(1e-2), ctypes.c_float(0.9), ctypes.c_float(0.999), ctypes.c_float(1e-8),
+           1, vp(wb.data_ptr()), vp(wtb.data_ptr()), None)
+    want = p0 - 1e-2 * np.sign(g) * (np.abs(g) / (np.abs(g) + 1e-8))
+    got = p.cpu().numpy()
+    assert np.max(np.abs(got - want)) < 1e-6
+    off = 0
+    bits = (MO.bf16(got).view(np.uint32) >> 16).astype(np.uint16).view(np.int16)
+    for o, i in shapes:
+        for z in range(Z):
+            w = bits[z, off:off + o * i]
+            assert np.array_equal(wb[z, off:off + o * i].cpu().numpy(), w)
+            assert np.array_equal(wtb[z, off:off + o * i].cpu().numpy().reshape(i, o), w.reshape(o, i).T)
+        assert int((wb[:, off + o * i:off + o * i + o] != 7).sum()) == 0      # biases have no copies
+        off += o * i + o
+
+
+@pytest.mark.parametrize('points', [1, 127, 128, 129, 300, 513])
+def test_predictions_do_not_depend_on_the_last_chunk(points):
+    """A last chunk of any length gives each member the rows it has in whole chunks."""
+    torch = _torch()
+    ens = S.MLPEnsemble(members=3, batch=256, nout=256, seed=2)
+    f = torch.rand(1024, 6, device='cuda', generator=torch.Generator('cuda').manual_seed(points)) * 2 - 1
+    whole = ens.predict(f)
+    assert torch.equal(ens.predict(f[:points].contiguous()), whole[:, :points])
+    assert float((whole.sum(dim=2) - 1).abs().max()) < 1e-5
+    assert not torch.equal(whole[0], whole[1])
+
+
+def test_network_calls_reject_bad_arguments():
+    """Checked before any launch."""
+    ens = S.MLPEnsemble(members=2, batch=128, nout=256)
+    for rows in (0, 129, 32):
+        with pytest.raises(N.NativeError) as e:
+            ens.loss_and_grads(rows)
+        assert e.value.code == N.DM_ERR_ARG
+    net = ens._net()
+    net._obj.count -= 1
+    assert N.lib().dm_mlp_forward(net, 128, 0, None) == N.DM_ERR_ARG
+    net = ens._net()
+    net._obj.h[1] = None
+    assert N.lib().dm_mlp_forward(net, 128, 0, None) == N.DM_ERR_ARG
