@@ -257,6 +257,35 @@ int dm_levelize(int n, int count, const int32_t *kind, const int32_t *qoff, cons
                 int32_t *placed_inst, int32_t *placed_pos, int32_t *placed_count, int32_t *table_len,
                 int32_t *levels);
 
+/* ------------------------------------------------------------------- planning */
+
+/* An operation to plan: DM_OP_* on qubit a, or on the pair (a, b). */
+typedef struct dm_plan_op {
+    int16_t kind, a, b;
+    int16_t ideal;      /* DM_OP_CX: its coefficients are those of the ideal gate */
+} dm_plan_op;
+
+/* Group count ops (program order) into passes of up to kmax resident qubits,
+ * the `low` last ones always among them; host code.  pass_of[i] is op i's pass
+ * and slot_of[i] its slot in the pass (one-axis maps that share a slot are to
+ * be multiplied, in order); resident[p] (count entries) is the mask of pass
+ * p's resident qubits.  With `partial` the ops are a prefix of a longer
+ * stream: passes that later ops could still join are left out, and their ops'
+ * pass_of and slot_of are -1.  DM_ERR_PROGRAM when an op fits no pass. */
+int dm_plan_passes(int n, int kmax, int low, const dm_plan_op *ops, int count, int partial, int32_t *pass_of,
+                   int32_t *slot_of, uint32_t *resident, int32_t *npasses);
+
+/* Descriptors and coefficients of planned passes for dm_apply_pass; host code.
+ * coefs holds the ops' coefficients one after another (DM_OP_MAP1 and
+ * DM_OP_DIAG2 16, DM_OP_CX 5, DM_OP_MAP2 256).  With width > 0 a pass's ops are
+ * grouped into register rounds of width axes when it has width..max_axes
+ * resident axes, qubit n-1 among them, no DM_OP_MAP2 and at most DM_MAX_ROUNDS
+ * rounds.  mats (host memory of the state's type, mats_capacity values) gets
+ * the coefficients, *mats_used of them; their offsets count from mats_off. */
+int dm_encode_passes(int n, int dtype, int width, int max_axes, const dm_plan_op *ops, int count, const double *coefs,
+                     const int32_t *pass_of, const int32_t *slot_of, const uint32_t *resident, int npasses,
+                     size_t mats_off, dm_pass *passes, void *mats, size_t mats_capacity, size_t *mats_used);
+
 /* ------------------------------------------------------------- batched sweeps */
 
 /* One pass of a batched program (the n-independent part of dm_pass). */

@@ -19,7 +19,7 @@ INCLUDE = os.path.join(REPO_DIR, 'include')
 BUILD_DIR = os.path.join(PKG_DIR, '_build')
 LIB_PATH = os.path.join(PKG_DIR, 'libdmgb300.so')
 SOURCES = ['dm_misc.cu', 'dm_pass.cu', 'dm_noise.cu', 'dm_state.cu', 'dm_measure.cu', 'dm_tc.cu', 'dm_tma.cu', 'dm_mlp.cu',
-           'dm_sample.cu', 'dm_sched.cpp']
+           'dm_sample.cu', 'dm_sched.cpp', 'dm_plan.cpp']
 ARCH = ['-gencode', 'arch=compute_103a,code=sm_103a']
 NVCC_FLAGS = ['-O3', '-std=c++17', '-lineinfo', '-Xcompiler', '-fPIC', '-Xptxas', '-warn-spills',
               '--expt-relaxed-constexpr']
@@ -203,6 +203,8 @@ SIGNATURES = {
     'dm_fp64_fma_probe_threads': (_i, []),
     'dm_fp64_fma_probe': (_i, [_vp, ctypes.c_int64, _vp]),
     'dm_levelize': (_i, [_i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
+    'dm_plan_passes': (_i, [_i, _i, _i, _vp, _i, _i, _vp, _vp, _vp, _vp]),
+    'dm_encode_passes': (_i, [_i, _i, _i, _i, _vp, _i, _vp, _vp, _vp, _vp, _i, _sz, _vp, _vp, _sz, _vp]),
     'dm_host_alloc': (_vp, [_sz]),
     'dm_host_device_pointer': (_vp, [_vp]),
     'dm_host_free': (_i, [_vp]),

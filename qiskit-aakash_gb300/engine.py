@@ -14,9 +14,8 @@ import numpy as np
 
 from . import _native as N
 from .exceptions import BasicAerError
-from .program import (TC_AXES, Op, OpTableError, TcPlanError, cx_coefficients, encode_pass, encode_pass_tc,
-                      encode_pass_tc_ops, encode_pass_tma,
-                      plan_passes)
+from .program import (TC_AXES, Op, OpTableError, Plan, TcPlanError, cx_coefficients, encode_pass, encode_pass_tc,
+                      encode_pass_tc_ops, encode_pass_tma, encode_plan, plan_passes)
 
 # Tile sizes of the fused pass: 4**6 FP64 = 32 KB and 4**7 FP32 = 64 KB of
 # shared memory per tile; the two lowest qubit axes (16 contiguous
@@ -279,9 +278,7 @@ class DeviceState:
         The device starts on the first passes while the host is still
         producing the rest of the circuit's operations.
         """
-        passes, self.pending = plan_passes(self.pending, self.n, self.kmax, self.low, partial=True)
-        if passes:
-            self._launch(passes)
+        self.pending = self._run_ops(self.pending, partial=True)
         self._stream_at = len(self.pending) + STREAM_OPS
 
     def flush(self):
@@ -293,15 +290,28 @@ class DeviceState:
         if not self.fusion:
             self._run_unfused(ops)
             return
-        self._launch(plan_passes(ops, self.n, self.kmax, self.low))
+        self._run_ops(ops)
         if self.tensor_cores and int(self.status.item()) != 0:
             raise BasicAerError('a tensor-core pass abandoned a bounded wait (status %d)' % int(self.status.item()))
 
-    def _launch(self, passes):
+    def _run_ops(self, ops, partial=False):
+        """Plan and launch ``ops``; with ``partial`` only the closed passes.  Returns the ops left."""
         if self.tensor_cores:
-            self._run_passes_tc(passes)
-        else:
-            self._run_passes(passes)
+            passes, rest = plan_passes(ops, self.n, self.kmax, self.low, partial=True) if partial \
+                else (plan_passes(ops, self.n, self.kmax, self.low), [])
+            if passes:
+                self._run_passes_tc(passes)
+            return rest
+        plan = Plan(ops, self.n, self.kmax, self.low, partial)
+        if len(plan.resident):
+            size = plan.coefficients()
+            h = _torch().empty(size, dtype=self.torch_dtype, pin_memory=self.device.type == 'cuda')
+            descs, used = encode_plan(plan, self.n, self.np_dtype, self._round_width(), h.data_ptr(), size)
+            self._apply_passes(descs, h[:used])
+        return plan.rest() if partial else []
+
+    def _round_width(self):
+        return N.DM_ROUND_AXES[self.dtype] if self.rounds else None
 
     def _encode_tc(self, p):
         """(entry point, descriptor, ops table or None, coefficients or FP16 images) of a tensor-core pass, or None.
@@ -424,20 +434,20 @@ class DeviceState:
         keep.append((h, dev, img, group))
 
     def _run_passes(self, passes):
-        torch = _torch()
         mats = []
-        width = N.DM_ROUND_AXES[self.dtype] if self.rounds else None
-        descs = [encode_pass(p, mats, self.np_dtype, width, self.n) for p in passes]
-        host = np.concatenate(mats) if mats else np.zeros(1, dtype=self.np_dtype)
-        h = torch.from_numpy(host)
+        descs = [encode_pass(p, mats, self.np_dtype, self._round_width(), self.n) for p in passes]
+        h = _torch().from_numpy(np.concatenate(mats) if mats else np.zeros(1, dtype=self.np_dtype))
         if self.device.type == 'cuda':
             h = h.pin_memory()
+        self._apply_passes(descs, h)
+
+    def _apply_passes(self, descs, h):
+        """Upload the coefficients (a host tensor) and launch the passes."""
         dev = h.to(self.device, non_blocking=True)
-        self.h2d_bytes += host.nbytes
-        mp = ctypes.c_void_p(dev.data_ptr())
+        self.h2d_bytes += h.numel() * h.element_size()
+        sp, mp, size, stream = self.ptr, ctypes.c_void_p(dev.data_ptr()), ctypes.c_size_t(h.numel()), self.stream
         for d in descs:
-            self._call('dm_apply_pass', self.ptr, self.n, self.dtype, ctypes.byref(d), mp,
-                       ctypes.c_size_t(host.size), self.stream, keep=(d, dev))
+            self._call('dm_apply_pass', sp, self.n, self.dtype, ctypes.byref(d), mp, size, stream, keep=(d, dev))
         self.passes_run += len(descs)
         self._keep = (h, dev)    # keep both alive until the next flush
 

@@ -25,8 +25,10 @@ program order, provided every earlier operation sharing one of its axes
 has run: the planner scans the pending operations in order and takes every
 operation whose axes fit in the pass and none of whose axes is held back by
 an earlier operation it could not take.  Consecutive 4x4 maps on one axis
-inside a pass are multiplied together (in FP64) into one map.
+inside a pass are multiplied together (in FP64) into one map.  The scan and
+the encoding of CUDA-core passes are compiled (csrc/dm_plan.cpp).
 """
+import ctypes
 import functools
 import math
 
@@ -192,6 +194,68 @@ class Pass:
         return self.axes.index(q)
 
 
+_OP_KINDS = {'map1': N.DM_OP_MAP1, 'map2': N.DM_OP_MAP2, 'diag2': N.DM_OP_DIAG2, 'cx': N.DM_OP_CX}
+_OP_COEFFICIENTS = np.array([0, 16, 256, 16, 5])      # by DM_OP_*
+
+
+def _vp(a):
+    return ctypes.c_void_p(a.ctypes.data)
+
+
+class Plan:
+    """Passes of ``ops``, planned by dm_plan_passes (csrc/dm_plan.cpp).
+
+    ``pass_of`` and ``slot_of`` name each op's pass and its slot there (one-axis
+    maps sharing a slot are multiplied in order), -1 for the ops that partial
+    planning left; ``resident`` holds the passes' qubit masks.
+    """
+    __slots__ = ('ops', 'table', 'pass_of', 'slot_of', 'resident')
+
+    def __init__(self, ops, n, kmax, low, partial=False):
+        self.ops = ops
+        self.table = _op_table(ops)
+        count = len(ops)
+        self.pass_of, self.slot_of = np.empty(count, np.int32), np.empty(count, np.int32)
+        resident, npasses = np.empty(count, np.uint32), ctypes.c_int32()
+        rc = N.lib().dm_plan_passes(n, kmax, low, _vp(self.table), count, int(partial), _vp(self.pass_of),
+                                    _vp(self.slot_of), _vp(resident), ctypes.byref(npasses))
+        if rc == N.DM_ERR_PROGRAM:
+            raise RuntimeError('planner made no progress')
+        if rc != N.DM_OK:
+            raise N.NativeError('dm_plan_passes', rc, N.lib().dm_error_string(rc).decode())
+        self.resident = resident[:npasses.value]
+
+    @classmethod
+    def of_pass(cls, p):
+        """The plan of one planned pass: every op in a slot of its own."""
+        plan = cls.__new__(cls)
+        plan.ops = p.ops
+        plan.table = _op_table(p.ops)
+        plan.pass_of = np.zeros(len(p.ops), np.int32)
+        plan.slot_of = np.arange(len(p.ops), dtype=np.int32)
+        plan.resident = np.array([sum(1 << q for q in p.axes)], np.uint32)
+        return plan
+
+    def coefficients(self):
+        """Values that the ops' coefficients take."""
+        return int(_OP_COEFFICIENTS[self.table[::4]].sum())
+
+    def rest(self):
+        """The ops that no pass took, in order."""
+        return [op for op, p in zip(self.ops, self.pass_of.tolist()) if p < 0]
+
+
+def _op_table(ops):
+    """dm_plan_op entries of ``ops`` (kind, axes, ideal)."""
+    flat = []
+    for op in ops:
+        kind = _OP_KINDS.get(op.kind)
+        if kind is None:
+            raise ValueError(op.kind)
+        flat += (kind, op.axes[0], op.axes[-1], op.ideal)
+    return np.array(flat, dtype=np.int16)
+
+
 def plan_passes(ops, n, kmax, low, partial=False):
     """Group ``ops`` (program order) into fused passes.
 
@@ -205,58 +269,24 @@ def plan_passes(ops, n, kmax, low, partial=False):
     are exactly the passes the whole stream would give), together with the
     ops they left, in order: ``(passes, rest)``.
     """
-    kmax = min(kmax, n)
-    low = min(low, kmax)
-    base = tuple(range(n - 1, n - 1 - low, -1))
-    pending = list(ops)
-    index_of = {id(op): i for i, op in enumerate(pending)}
-    passes = []
-    while pending:
-        resident = set(base)
-        full = len(resident) >= kmax
-        blocked = set()
-        closed = False
-        taken_idx = []
-        body = []          # list of Op (possibly composed)
-        last_on_axis = {}  # axis -> index into body of the last op touching it
-        for i, op in enumerate(pending):
-            axes = op.axes
-            if blocked.intersection(axes) or \
-                    len(resident) + sum(a not in resident for a in axes) > kmax or \
-                    len(body) >= N.DM_MAX_PASS_OPS:
-                blocked.update(axes)
-                # Once the pass is full and every resident axis is held back,
-                # no later operation can be taken.
-                if (full and blocked.issuperset(resident)) or len(blocked) >= n:
-                    closed = True
-                    break
-                continue
-            grow = [a for a in axes if a not in resident]
-            resident.update(grow)
-            taken_idx.append(i)
-            src = op.src if op.src is not None else [index_of[id(op)]]
-            if op.kind == 'map1':
-                a = axes[0]
-                j = last_on_axis.get(a)
-                if j is not None and body[j].kind == 'map1':
-                    body[j] = Op('map1', (a,), op.data @ body[j].data, src=body[j].src + src)
-                    continue
-                body.append(Op('map1', axes, op.data, src=src))
-            else:
-                body.append(Op(op.kind, axes, op.data, op.ideal, src=src))
-            for a in axes:
-                last_on_axis[a] = len(body) - 1
-            if len(resident) >= kmax:
-                full = True
-        if not taken_idx:
-            raise RuntimeError('planner made no progress')
-        if partial and not closed:
-            return passes, pending     # later ops could still join this pass
-        keep = set(taken_idx)
-        pending = [op for i, op in enumerate(pending) if i not in keep]
-        axes = sorted(resident, reverse=True)
-        passes.append(Pass(axes, body))
-    return (passes, []) if partial else passes
+    ops = list(ops)
+    plan = Plan(ops, n, kmax, low, partial)
+    bodies = [[] for _ in plan.resident]
+    rest = []
+    for i, (op, p, slot) in enumerate(zip(ops, plan.pass_of.tolist(), plan.slot_of.tolist())):
+        if p < 0:
+            rest.append(op)
+            continue
+        body = bodies[p]
+        src = op.src if op.src is not None else [i]
+        if slot < len(body):
+            before = body[slot]
+            body[slot] = Op('map1', before.axes, op.data @ before.data, src=before.src + src)
+        else:
+            body.append(Op(op.kind, op.axes, op.data, op.ideal, src=src))
+    passes = [Pass([q for q in range(n - 1, -1, -1) if mask >> q & 1], body)
+              for mask, body in zip(plan.resident.tolist(), bodies)]
+    return (passes, rest) if partial else passes
 
 
 def plan_rounds(p, width, pad='low'):
@@ -295,8 +325,29 @@ def plan_rounds(p, width, pad='low'):
 ROUND_MAX_AXES = {np.dtype(np.float32): 7, np.dtype(np.float64): 6}
 
 
+def _encode(plan, n, dtype_np, round_width, mats_off, mats_ptr, capacity):
+    """(dm_pass descriptors, coefficients written) of a plan: dm_encode_passes."""
+    coefs = np.concatenate([op.data for op in plan.ops], axis=None).astype(np.float64, copy=False) \
+        if plan.ops else np.zeros(0)
+    if coefs.size != plan.coefficients():
+        raise ValueError('an operation holds %d coefficients more than its kind has' % (coefs.size - plan.coefficients()))
+    descs = (N.DmPass * len(plan.resident))()
+    used = ctypes.c_size_t()
+    dtype_np = np.dtype(dtype_np)
+    N.call('dm_encode_passes', n, N.DM_F64 if dtype_np == np.float64 else N.DM_F32, round_width or 0,
+           ROUND_MAX_AXES[dtype_np], _vp(plan.table), len(plan.ops), _vp(coefs), _vp(plan.pass_of), _vp(plan.slot_of),
+           _vp(plan.resident), len(plan.resident), mats_off, ctypes.cast(descs, ctypes.c_void_p), mats_ptr, capacity,
+           ctypes.byref(used))
+    return descs, used.value
+
+
+def encode_plan(plan, n, dtype_np, round_width, mats_ptr, capacity):
+    """Descriptors of every pass of ``plan``, coefficients at host address ``mats_ptr``; see encode_pass."""
+    return _encode(plan, n, dtype_np, round_width, 0, ctypes.c_void_p(mats_ptr), capacity)
+
+
 def encode_pass(p, mats, dtype_np, round_width=None, n=None):
-    """Fill a ctypes DmPass for ``p``; append its coefficients to ``mats`` (list of arrays).
+    """Fill a ctypes DmPass for ``p``; append its coefficients to ``mats`` (list of arrays, one per op).
 
     With ``round_width`` (and the register count ``n``) the ops are grouped
     into register rounds when the pipelined round kernel can run the pass:
@@ -304,66 +355,17 @@ def encode_pass(p, mats, dtype_np, round_width=None, n=None):
     lowest qubit axis resident (16-byte chunks are contiguous), no 16x16
     general maps, and the rounds fit the descriptor.
     """
-    dp = N.DmPass()
-    dp.k = len(p.axes)
-    for r, q in enumerate(p.axes):
-        dp.axes[r] = q
-    rounds = None
-    if round_width and n is not None and round_width <= dp.k <= ROUND_MAX_AXES[np.dtype(dtype_np)] \
-            and p.axes[0] == n - 1 and all(op.kind != 'map2' for op in p.ops):
-        rounds = plan_rounds(p, round_width)
-        if len(rounds) > N.DM_MAX_ROUNDS or sum(len(ops) for _, ops in rounds) > N.DM_MAX_PASS_OPS:
-            rounds = None
-    if rounds is not None:
-        ops_local = []
-        dp.nrounds = len(rounds)
-        for ri, (axes, rops) in enumerate(rounds):
-            for i, a in enumerate(axes):
-                dp.round_axes[ri][i] = a
-            for i in range(len(axes), 4):
-                dp.round_axes[ri][i] = -1
-            for op in rops:
-                ops_local.append((op, [axes.index(a) for a in op.axes]))
-            dp.round_end[ri] = len(ops_local)
-    else:
-        dp.nrounds = 0
-        ops_local = [(Op(op.kind, tuple(p.local(a) for a in op.axes), op.data, op.ideal), None) for op in p.ops]
-    dp.nops = len(ops_local)
+    plan = Plan.of_pass(p)
+    out = np.empty(max(plan.coefficients(), 1), dtype=dtype_np)
     off = sum(m.size for m in mats)
-    for i, (op, digits) in enumerate(ops_local):
-        o = dp.ops[i]
-        o.a = op.axes[0]
-        o.moff = off
-        if op.kind == 'map1':
-            o.kind = N.DM_OP_MAP1
-            m = np.ascontiguousarray(op.data, dtype=np.float64).reshape(16)
-            flags = N.DM_MAP1_ROW0_IDENTITY if (m[0] == 1.0 and not m[1:4].any()) else 0
-            flags |= N.DM_MAP1_XY_UNITAL if (m[4] == 0.0 and m[8] == 0.0) else 0
-            o.b = 0
-        elif op.kind == 'cx':
-            o.kind = N.DM_OP_CX
-            o.b = op.axes[1]
-            flags = N.DM_CX_IDEAL if op.ideal else 0
-            m = np.asarray(op.data, dtype=np.float64)
-        elif op.kind == 'diag2':
-            o.kind = N.DM_OP_DIAG2
-            o.b = op.axes[1]
-            flags = 0
-            m = np.asarray(op.data, dtype=np.float64).reshape(16)
-        elif op.kind == 'map2':
-            o.kind = N.DM_OP_MAP2
-            o.b = op.axes[1]
-            flags = 0
-            m = np.asarray(op.data, dtype=np.float64).reshape(256)
-        else:
-            raise ValueError(op.kind)
-        if digits is not None:              # round digit positions of the op's axes
-            flags |= digits[0] << 8
-            if len(digits) > 1:
-                flags |= digits[1] << 12
-        o.flags = flags
-        mats.append(m.astype(dtype_np))
-        off += m.size
+    descs, used = _encode(plan, n if n is not None else p.axes[0] + 1, dtype_np, round_width if n is not None else 0,
+                          off, _vp(out), out.size)
+    dp = descs[0]
+    ends = [dp.ops[i].moff - off for i in range(1, dp.nops)] + [used]
+    at = 0
+    for end in ends if dp.nops else []:
+        mats.append(out[at:end])
+        at = end
     return dp
 
 

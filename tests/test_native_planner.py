@@ -1,0 +1,133 @@
+"""The compiled planner against the same scan written over sets of axes, and its descriptors against program order."""
+import ctypes
+import importlib
+
+import numpy as np
+import pytest
+
+from test_planner import apply_op, random_ops
+
+P = importlib.import_module('qiskit-aakash_gb300.program')
+N = importlib.import_module('qiskit-aakash_gb300._native')
+
+
+def scan(ops, n, kmax, low, partial):
+    """(pass, slot) of each op, and the passes' resident sets."""
+    kmax = min(kmax, n)
+    base = set(range(n - 1, n - 1 - min(low, kmax), -1))
+    where, residents, pending = [(-1, -1)] * len(ops), [], list(range(len(ops)))
+    while pending:
+        resident, blocked, taken, last, slots, closed = set(base), set(), [], {}, 0, False
+        for i in pending:
+            axes = set(ops[i].axes)
+            if blocked & axes or len(resident | axes) > kmax or slots >= N.DM_MAX_PASS_OPS:
+                blocked |= axes
+                if (len(resident) >= kmax and blocked >= resident) or len(blocked) >= n:
+                    closed = True
+                    break
+                continue
+            resident |= axes
+            if ops[i].kind == 'map1' and last.get(ops[i].axes[0]) is not None:
+                slot = last[ops[i].axes[0]]
+            else:
+                slot, slots = slots, slots + 1
+                for a in axes:
+                    last[a] = slot if ops[i].kind == 'map1' else None
+            taken.append((i, slot))
+        assert taken
+        if partial and not closed:
+            break
+        for i, slot in taken:
+            where[i] = (len(residents), slot)
+        residents.append(resident)
+        gone = {i for i, _ in taken}
+        pending = [i for i in pending if i not in gone]
+    return where, residents
+
+
+CASES = [(1, 6, 2), (2, 6, 2), (5, 4, 2), (8, 6, 2), (8, 7, 3), (9, 4, 0), (6, 2, 0), (17, 7, 2), (16, 3, 0)]
+
+
+@pytest.mark.parametrize('partial', [False, True])
+@pytest.mark.parametrize('n,kmax,low', CASES)
+def test_same_passes_as_the_scan_over_sets(n, kmax, low, partial):
+    rng = np.random.default_rng(n * 100 + kmax * 10 + low + partial)
+    for count in (0, 1, 2, 40, 300, 900):
+        ops = random_ops(rng, n, count)
+        plan = P.Plan(ops, n, kmax, low, partial)
+        where, residents = scan(ops, n, kmax, low, partial)
+        assert list(zip(plan.pass_of.tolist(), plan.slot_of.tolist())) == where
+        assert [{q for q in range(n) if m >> q & 1} for m in plan.resident.tolist()] == residents
+        assert plan.rest() == [op for op, (p, _) in zip(ops, where) if p < 0]
+
+
+@pytest.mark.parametrize('width', [2, 3, None])
+@pytest.mark.parametrize('n,kmax,low', [(1, 6, 2), (3, 6, 2), (5, 4, 2), (8, 6, 2), (8, 7, 2), (7, 5, 0)])
+def test_descriptors_equal_program_order(n, kmax, low, width):
+    rng = np.random.default_rng(7 * n + kmax + low)
+    for count in (1, 30, 250):
+        ops = random_ops(rng, n, count)
+        for op in ops:                  # bounded growth, so that a relative bound means something
+            if op.kind in ('map1', 'map2'):
+                op.data = op.data / np.abs(op.data).sum(axis=1, keepdims=True)
+            elif op.kind == 'diag2':
+                op.data = np.clip(op.data, -1, 1)
+        want = got = rng.normal(size=4 ** n)
+        for op in ops:
+            want = apply_op(want, n, op)
+        plan = P.Plan(ops, n, kmax, low)
+        mats = np.empty(plan.coefficients())
+        descs, used = P.encode_plan(plan, n, np.float64, width, mats.ctypes.data, mats.size)
+        if kmax <= 6:      # the FP32 form: the same descriptors, the coefficients rounded once
+            mats32 = np.empty(plan.coefficients(), np.float32)
+            descs32, used32 = P.encode_plan(plan, n, np.float32, width, mats32.ctypes.data, mats32.size)
+            assert used32 == used and bytes(descs32) == bytes(descs)
+            assert np.array_equal(mats32[:used], mats[:used].astype(np.float32))
+        at = 0
+        for d in descs:
+            axes = list(d.axes[:d.k])
+            assert axes == sorted(axes, reverse=True)
+            for i in range(d.nops):
+                o = d.ops[i]
+                assert o.moff == at
+                kind = {v: k for k, v in P._OP_KINDS.items()}[o.kind]
+                size = {'map1': 16, 'cx': 5, 'diag2': 16, 'map2': 256}[kind]
+                data = mats[at:at + size]
+                at += size
+                local = (o.a,) if kind == 'map1' else (o.a, o.b)
+                if d.nrounds:
+                    r = next(r for r in range(d.nrounds) if i < d.round_end[r])
+                    digits = list(d.round_axes[r])
+                    assert digits[width:] == [-1] * (4 - width) and digits[:width] == sorted(set(digits[:width]))
+                    assert tuple(digits[(o.flags >> (8 + 4 * j)) & 15] for j in range(len(local))) == local
+                shape = {'map1': (4, 4), 'map2': (16, 16)}.get(kind, (size,))
+                if kind == 'map1':
+                    assert bool(o.flags & N.DM_MAP1_ROW0_IDENTITY) == bool(data[0] == 1 and not data[1:4].any())
+                    assert bool(o.flags & N.DM_MAP1_XY_UNITAL) == bool(data[4] == 0 and data[8] == 0)
+                got = apply_op(got, n, P.Op(kind, tuple(axes[a] for a in local), data.reshape(shape),
+                                            bool(kind == 'cx' and o.flags & N.DM_CX_IDEAL)))
+        assert at == used
+        # every op rounds each value once per term: 250 ops x 16 terms x half an ulp, doubled
+        eps = np.finfo(np.float64).eps
+        np.testing.assert_allclose(got, want, rtol=0, atol=250 * 16 * eps * np.abs(want).max() + 1e-300)
+
+
+def test_full_pass_of_128_ops_and_what_is_refused():
+    coef, ideal = P.cx_coefficients([0.99, 0.01])
+    ops = [P.Op('cx', (i % 2, 1 - i % 2), np.array(coef), ideal) for i in range(300)]
+    passes = P.plan_passes(ops, 2, 2, 2)
+    assert [len(p.ops) for p in passes] == [128, 128, 44]
+    with pytest.raises(RuntimeError, match='no progress'):
+        P.plan_passes([P.Op('cx', (0, 1), np.array(coef), ideal)], 4, 1, 0)
+    with pytest.raises(N.NativeError):
+        P.plan_passes([P.Op('map1', (4,), np.eye(4))], 4, 4, 2)
+    with pytest.raises(ValueError):
+        P.plan_passes([P.Op('swap', (0, 1), np.eye(16))], 4, 4, 2)
+    # a buffer that is too small is an error, not an overrun
+    plan = P.Plan([P.Op('map1', (0,), np.eye(4))], 1, 1, 0)
+    mats = np.full(32, 7.0)
+    with pytest.raises(N.NativeError):
+        P.encode_plan(plan, 1, np.float64, None, mats.ctypes.data, 15)
+    assert (mats == 7.0).all()
+    with pytest.raises(ValueError):
+        P.encode_plan(P.Plan([P.Op('map1', (0,), np.eye(3))], 1, 1, 0), 1, np.float64, None, mats.ctypes.data, 16)
