@@ -136,12 +136,13 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_kernel(const __grid_constant
                      "n"(kTmemCols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
-    if constexpr (EPI == DM_MLP_EPI_GELU_FWD || EPI == DM_MLP_EPI_BIAS_F32)
-        if (tid >= 64 && tid < 64 + kBN) bias_s[tid - 64] = g.bias[z * g.bias_ms + n0 + tid - 64];
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_base_s;
+    grid_wait();
+    if constexpr (EPI == DM_MLP_EPI_GELU_FWD || EPI == DM_MLP_EPI_BIAS_F32)
+        if (tid >= 64 && tid < 64 + kBN) bias_s[tid - 64] = waited(g.bias)[z * g.bias_ms + n0 + tid - 64];
 
     // A thread whose wait gives up flags the abort and stops; the others' waits then run out in turn.
     auto wait_for = [&](uint64_t &bar, uint32_t parity) {
@@ -314,7 +315,9 @@ __global__ void __launch_bounds__(32 * kSoftRows, 2)
     const bool live = r < rows;
     const int per = Per ? Per : nout / kRowThreads;
     const int64_t base = (z * row_ms + (live ? r : r0)) * nout;
-    const float *row = logits + base;
+    grid_wait();
+    const float *row = waited(logits) + base;
+    targets = waited(targets);
     float held[Per ? Per * kSoftSlices : 1] = {};
     if constexpr (Per > 0) {
 #pragma unroll
@@ -386,10 +389,8 @@ static int launch_softmax(const float *logits, const float *targets, int rows, i
                 : nout == 512 ? softmax_kernel<2>
                 : nout == 768 ? softmax_kernel<3>
                 : nout == 1024 ? softmax_kernel<4> : softmax_kernel<0>;
-    kernel<<<grid, block, 0, s>>>(logits, targets, rows, nout, row_ms, out_ms, ld_t, grad_scale, probs, dz, dzt,
-                                  loss_rows);
-    count_launch();
-    return launch_status();
+    return launch_early(kernel, grid, block, 0, s, logits, targets, rows, nout, row_ms, out_ms, ld_t, grad_scale, probs,
+                        dz, dzt, loss_rows);
 }
 
 // db[n] = sum_b d_t[n][b] for up to four layers: one warp per (layer, n, member)
@@ -405,6 +406,7 @@ struct BiasGrads {
 __global__ void bias_grad_kernel(const __grid_constant__ BiasGrads B) {
     const int lane = threadIdx.x & 31;
     int n = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    grid_wait();
     if (n >= B.first[B.count]) return;
     int i = 0;
     while (n >= B.first[i + 1]) ++i;
@@ -419,9 +421,7 @@ __global__ void bias_grad_kernel(const __grid_constant__ BiasGrads B) {
 
 static int launch_bias_grads(const BiasGrads &B, int members, cudaStream_t s) {
     const int warps = 8;
-    bias_grad_kernel<<<dim3((B.first[B.count] + warps - 1) / warps, members), 32 * warps, 0, s>>>(B);
-    count_launch();
-    return launch_status();
+    return launch_early(bias_grad_kernel, dim3((B.first[B.count] + warps - 1) / warps, members), dim3(32 * warps), 0, s, B);
 }
 
 struct Layers {
@@ -440,6 +440,8 @@ __global__ void __launch_bounds__(256) adam_kernel(float *__restrict__ params, c
                                                    float eps, float c1, float c2, int step, int members,
                                                    uint16_t *__restrict__ wb, uint16_t *__restrict__ wtb) {
     __shared__ uint16_t tr[32][33];
+    grid_wait();
+    grads = waited(grads);
     auto update = [&](int64_t i) {
         float p = params[i];
         if (step > 0) {
@@ -495,6 +497,10 @@ __global__ void gather_kernel(const float *__restrict__ features, int nfeat, con
                               int64_t row_ms, int width, uint16_t *__restrict__ x, uint16_t *__restrict__ xt,
                               float *__restrict__ t) {
     const int64_t r = blockIdx.x, z = blockIdx.y;
+    grid_wait();
+    features = waited(features);
+    targets = waited(targets);
+    index = waited(index);
     int64_t s;
     if (index) {
         s = index[z * rows + r];
@@ -524,6 +530,9 @@ __global__ void __launch_bounds__(kRowThreads) ensemble_kernel(const float *__re
     __shared__ float red[kRowThreads / 32][Members + 1];
     const int64_t r = blockIdx.x;
     float dev[Members + 1] = {};                          // the members', then the reference's
+    grid_wait();
+    probs = waited(probs);
+    ref = waited(ref);
 #pragma unroll 4
     for (int j = threadIdx.x; j < nout; j += kRowThreads) {
         float q[Members];
@@ -567,9 +576,8 @@ static int launch_ensemble(const float *probs, int rows, int members, int nout, 
     using Kernel = void (*)(const float *, int, int, const float *, float *, float *, float *);
     static constexpr Kernel kernels[8] = {ensemble_kernel<1>, ensemble_kernel<2>, ensemble_kernel<3>, ensemble_kernel<4>,
                                           ensemble_kernel<5>, ensemble_kernel<6>, ensemble_kernel<7>, ensemble_kernel<8>};
-    kernels[members - 1]<<<rows, kRowThreads, 0, s>>>(probs, rows, nout, ref, mean, spread, tv_ref);
-    count_launch();
-    return launch_status();
+    return launch_early(kernels[members - 1], dim3(rows), dim3(kRowThreads), 0, s, probs, rows, nout, ref, mean, spread,
+                        tv_ref);
 }
 
 using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
@@ -618,9 +626,7 @@ static int launch_gemms(const dm_mlp_gemm *g, int count, int *status, cudaStream
             !operand_map(&G.b[i], g[i].B, g[i].K, g[i].N, g[i].members, g[i].ldb, g[i].b_ms, kBN))
             return DM_ERR_CUDA;
     }
-    gemm_kernel<EPI><<<dim3(G.first[count], g[0].members), kThreads, kSmemBytes, s>>>(G, status);
-    count_launch();
-    return launch_status();
+    return launch_early(gemm_kernel<EPI>, dim3(G.first[count], g[0].members), dim3(kThreads), kSmemBytes, s, G, status);
 }
 
 static bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -717,10 +723,8 @@ extern "C" int dm_mlp_adam(float *params, const float *grads, float *m, float *v
     const double c1 = step > 0 ? 1.0 - pow(double(beta1), step) : 1.0;
     const double c2 = step > 0 ? 1.0 - pow(double(beta2), step) : 1.0;
     const dim3 grid(L.tiles[nlayers] + L.bias_blocks[nlayers], members < 65535 ? members : 65535);
-    mlp::adam_kernel<<<grid, 256, 0, as_stream(stream)>>>(params, grads, m, v, count_per_member, L, lr, beta1, beta2, eps,
-                                                          float(c1), float(c2), step, members, w_bf16, wt_bf16);
-    count_launch();
-    return launch_status();
+    return launch_early(mlp::adam_kernel, grid, dim3(256), 0, as_stream(stream), params, grads, m, v, count_per_member, L, lr,
+                        beta1, beta2, eps, float(c1), float(c2), step, members, w_bf16, wt_bf16);
 }
 
 extern "C" int dm_mlp_gather(const float *features, int nfeat, const float *targets, int nout, int64_t samples,
@@ -729,10 +733,8 @@ extern "C" int dm_mlp_gather(const float *features, int nfeat, const float *targ
     DM_CHECK_ARG(features && index && x && xt && nfeat > 0 && nfeat <= width && samples > 0);
     DM_CHECK_ARG(rows > 0 && members >= 1 && members <= 65535 && width % 8 == 0 && nout > 0 && nout % 4 == 0);
     DM_CHECK_ARG(!targets || (t && mlp::aligned16(targets) && mlp::aligned16(t)));
-    mlp::gather_kernel<<<dim3(rows, members), 256, 0, as_stream(stream)>>>(features, nfeat, targets, nout, samples, index,
-                                                                          0, rows, rows, width, x, xt, t);
-    count_launch();
-    return launch_status();
+    return launch_early(mlp::gather_kernel, dim3(rows, members), dim3(256), 0, as_stream(stream), features, nfeat, targets,
+                        nout, samples, index, int64_t(0), rows, int64_t(rows), width, x, xt, t);
 }
 
 extern "C" int dm_mlp_ensemble(const float *probs, int rows, int members, int nout, const float *ref, float *mean,
@@ -946,10 +948,11 @@ extern "C" int dm_mlp_predict(const dm_mlp_net *net, const float *features, int 
     for (int64_t s0 = 0; s0 < samples; s0 += n.batch) {
         const int rows = int(samples - s0 < n.batch ? samples - s0 : n.batch);
         const int padded = (rows + mlp::kBM - 1) / mlp::kBM * mlp::kBM;
-        mlp::gather_kernel<<<dim3(padded, n.members), 64, 0, s>>>(features, nfeat, nullptr, n.nout, samples, nullptr, s0,
-                                                                  padded, n.batch, mlp::kInput, n.x, nullptr, nullptr);
-        count_launch();
-        if ((rc = launch_status())) return rc;
+        rc = launch_early(mlp::gather_kernel, dim3(padded, n.members), dim3(64), 0, s, features, nfeat,
+                          static_cast<const float *>(nullptr), n.nout, samples, static_cast<const int32_t *>(nullptr), s0,
+                          padded, int64_t(n.batch), mlp::kInput, n.x, static_cast<uint16_t *>(nullptr),
+                          static_cast<float *>(nullptr));
+        if (rc) return rc;
         if ((rc = mlp::forward(n, rows, false, s))) return rc;
         if ((rc = mlp::launch_softmax(n.logits, nullptr, rows, n.members, n.nout, n.batch, samples, 0, 1.f,
                                       out + s0 * n.nout, nullptr, nullptr, nullptr, s)))

@@ -378,7 +378,8 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
     __shared__ int abort_s;
     TcCta c{smem, smem + kABytes, smem + 2 * kABytes, &mbar, hi_off, &abort_s, 0, 0, false};
     tc_setup(c, &tmem_base_s);
-    tc_pass_tiles(st, p, umats, blockIdx.x, gridDim.x, c, status);
+    grid_wait();
+    tc_pass_tiles(st, p, waited(umats), blockIdx.x, gridDim.x, c, status);
     tc_teardown(c);
 }
 
@@ -1101,10 +1102,8 @@ extern "C" int dm_apply_pass_tc(void *state_dev, int n, const dm_tc_pass *pass, 
     // 88 KB of shared memory, <= 128 registers per thread and 256 TMEM columns per CTA: two CTAs per SM
     int64_t grid = int64_t(sm_count()) * tc::kCtasPerSm;
     if (grid > ntiles) grid = ntiles;
-    tc::pass_tc_kernel<<<int(grid), tc::kThreads, tc::kSmemBytes, as_stream(stream)>>>(
-        static_cast<float *>(state_dev), p, umats_dev, status_dev);
-    count_launch();
-    return launch_status();
+    return launch_early(tc::pass_tc_kernel, dim3(unsigned(grid)), dim3(tc::kThreads), tc::kSmemBytes, as_stream(stream),
+                        static_cast<float *>(state_dev), p, umats_dev, status_dev);
 }
 
 extern "C" size_t dm_batch_tc_scratch_bytes(void) {

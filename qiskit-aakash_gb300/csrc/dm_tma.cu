@@ -201,9 +201,13 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_base_s + uint32_t(team * 256);
+    if (tid == 0) asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap)) : "memory");
+    grid_wait();
 
+    // team 1 takes a grid's width further, so that a pass of fewer tiles than SMs has one per SM: at 64
+    // tiles two teams on 32 SMs share their shared memory and tensor pipe (16.7 us a pass; 13.1 us on 64)
     const int64_t stride = int64_t(gridDim.x) * kTeams;
-    int64_t t = int64_t(blockIdx.x) * kTeams + team;
+    int64_t t = int64_t(blockIdx.x) + int64_t(gridDim.x) * team;
     if (tid == 0) {   // the pass's round images, once per CTA
         tcg::mbar_expect_tx(ubar, uint32_t(p.nres) * kUBytes);
         for (int r = 0; r < p.nres; ++r)
@@ -558,14 +562,12 @@ extern "C" int dm_apply_pass_tma(void *state_dev, int n, const dm_tc_pass *pass,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return DM_ERR_CUDA;
-    const int64_t grid = std::min<int64_t>(sm_count(), (p.ntiles + tma::kTeams - 1) / tma::kTeams);
+    const int64_t grid = std::min<int64_t>(sm_count(), p.ntiles);
     if (ensure_max_dynamic_smem(reinterpret_cast<const void *>(tma::pass_tma_kernel), int(tma::kSmemBytes)) !=
         cudaSuccess)
         return DM_ERR_CUDA;
-    tma::pass_tma_kernel<<<int(grid), tma::kThreads, tma::kSmemBytes, as_stream(stream)>>>(
-        map, p, static_cast<float *>(state_dev), umats_dev, status_dev);
-    count_launch();
-    return launch_status();
+    return launch_early(tma::pass_tma_kernel, dim3(unsigned(grid)), dim3(tma::kThreads), tma::kSmemBytes, as_stream(stream),
+                        map, p, static_cast<float *>(state_dev), umats_dev, status_dev);
 }
 
 // ---------------------------------------------------------------------------

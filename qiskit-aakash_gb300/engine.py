@@ -348,7 +348,8 @@ class DeviceState:
         copy, one dm_compose_passes launch writes its round images and the
         passes read them.  A composition alone is a few dozen warps for
         several microseconds, so groups double from one pass (the device
-        starts at once) up to COMPOSE_PASSES; the stream orders a group's
+        starts at once) up to COMPOSE_PASSES, which a recording uses from the
+        first pass on (its replays wait for no host); the stream orders a group's
         composition after the previous group's reads of the image buffer."""
         keep = []
         ran = 0
@@ -366,7 +367,7 @@ class DeviceState:
                 self._run_host_composed(enc, keep)
             else:
                 group.append(enc)
-                if len(group) >= self._group:
+                if len(group) >= (self._group if self.tape is None else COMPOSE_PASSES):
                     self._group = min(2 * self._group, COMPOSE_PASSES)
                     self._run_group(group, keep)
                     group = []
