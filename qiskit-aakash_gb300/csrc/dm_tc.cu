@@ -431,66 +431,49 @@ __device__ void batch_tc_setup(Pass &ps, const dm_batch_tc_pass &bp, int n) {
         out[i] = i % kWords == 1 ? uint32_t(i / kWords * kUHalves) : in[i];   // word 1: umoff
 }
 
-// Round r's matrix U (64 x 64 in its K-digit order) is the round's operations
-// applied to the 64 unit vectors: column k of U = ops(e_k), composed in FP64
-// in shared memory and written as the FP16 images that the MMAs read, K-major
+// Round r's matrix U (64 x 64 in its K-digit order), composed in FP64 from the
+// round's operations and written as the FP16 images that the MMAs read, K-major
 // (value (n%8)*8 + k%8 + (k/8)*64 + (n/8)*512 for output n, input k), with
 // Uh = fp16(U) and Ul = fp16(2**11 (U - Uh)): three images 2**11 Uh | Ul | Uh
 // for the cp.async-fed kernels, two images Uh | Ul for the TMA-fed one.
 //
 // What bounds it is the FP64 pipe: two FMAs per clock and SM, one warp
-// instruction per 64 cycles on each of its four quarters.  So one warp owns C
-// columns (index j = d0 + 4 d1 + 16 d2 of column c at c * kColStride + j; no
-// block barrier between operations), its lanes sharing each operation's
-// independent groups: 8 columns in the batched sweeps, where a CTA composes a
-// whole pass and the pair operations then fill the lanes, and 2 in the
-// single-state launches, whose rounds have the chip to themselves and spread
-// over 32 warps each.  The 4x4 maps that come before the round's first pair
-// operation form a Kronecker product and are written as such (two products
-// per entry instead of 16 FMAs per four entries and map); and a map whose I
-// row is (1,0,0,0), whose X and Y rows take no I, costs 10 FMAs per four
-// entries instead of 16.
+// instruction per 64 cycles on each of its four quarters.  So the operations are
+// not applied to the 64 columns of U one by one (40-70 FP64 instructions per
+// entry of a two-CX round with noise and rotations).  They act on pairs of the
+// round's three digits: those up to the first operation that needs the third
+// pair form two 16 x 16 blocks, T1 on the digits (y, x) and T2 on (c, x), and
+//     U[(y',x',c'), (y,x,c)] = sum_m T2[(c',x'), (c,m)] T1[(y',m), (y,x)],
+// four FMAs per entry (a single pair with maps on the third digit: one product).
+// A one-axis map counts to the block that its neighbours on its digit belong to.
+// The few operations beyond (a third CX) are applied to the columns.  The split
+// into FP16 parts works on the bits of the doubles, without FP64 instructions
+// (its conversions and subtractions were five of them per entry).
+// 1,024 points of a 10-qubit template: XX.
 constexpr int kColStride = 65;   // doubles per column: a warp's lanes spread over the banks
-constexpr int kColBytes = 64 * kColStride * 8;   // one round's columns
-static_assert(kColBytes <= int(kSmemBytes), "one round of FP64 columns fits the pass's shared memory");
+constexpr int kBlkStride = 17;   // doubles per column of a block
+constexpr int kBlkDoubles = 16 * kBlkStride;
 
-// One operation on the warp's C columns (digit positions from the op flags).
-// Map2: 16x16 general maps too (the single-state passes; the batched plans hold none).
-template <bool Map2, int C>
-__device__ __forceinline__ void cols_apply(double *w, const dm_op &op, const double *__restrict__ mg, int lane) {
-    const int da = (op.flags >> 8) & 3, db = (op.flags >> 12) & 3;
-    if (op.kind == DM_OP_MAP1) {
-        double m[16];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) m[i] = mg[i];
-        const bool row0 = m[0] == 1.0 && m[1] == 0.0 && m[2] == 0.0 && m[3] == 0.0;
-        const bool xy = row0 && m[4] == 0.0 && m[8] == 0.0;
-        const int S = 1 << (2 * da);
-        const int g = lane & 15;
-        const int j0 = ((g >> (2 * da)) << (2 * da + 2)) | (g & (S - 1));
-        double *col = w + (lane >> 4) * kColStride + j0;
-#pragma unroll
-        for (int it = 0; it < C / 2; ++it) {
-            double *x = col + 2 * it * kColStride;
-            double x0 = x[0], x1 = x[S], x2 = x[2 * S], x3 = x[3 * S];
-            if (xy) {
-                map4_tp_xy(m, x0, x1, x2, x3);
-            } else if (row0) {
-                map4<true>(m, x0, x1, x2, x3);
-            } else {
-                map4<false>(m, x0, x1, x2, x3);
-                x[0] = x0;
-            }
-            x[S] = x1;
-            x[2 * S] = x2;
-            x[3 * S] = x3;
-        }
-        return;
+// A 4x4 map on four values S apart.
+__device__ __forceinline__ void map1_at(double *x, int S, const double (&m)[16], bool row0, bool xy) {
+    double x0 = x[0], x1 = x[S], x2 = x[2 * S], x3 = x[3 * S];
+    if (xy) {
+        map4_tp_xy(m, x0, x1, x2, x3);
+    } else if (row0) {
+        map4<true>(m, x0, x1, x2, x3);
+    } else {
+        map4<false>(m, x0, x1, x2, x3);
+        x[0] = x0;
     }
-    // pair operations: lane = (column, value of the third digit)
-    if (lane >= 4 * C) return;
-    const int SA = 1 << (2 * da), SB = 1 << (2 * db), SC = 1 << (2 * (3 - da - db));
-    double *col = w + (lane >> 2) * kColStride + (lane & 3) * SC;
+    x[S] = x1;
+    x[2 * S] = x2;
+    x[3 * S] = x3;
+}
+
+// A pair operation on the 16 values at col, the operation's axes SA and SB apart.
+// Map2: 16x16 general maps too (the single-state passes; the batched plans hold none).
+template <bool Map2>
+__device__ __forceinline__ void pair_at(double *col, int SA, int SB, const dm_op &op, const double *__restrict__ mg) {
     double x[16];
 #pragma unroll
     for (int i = 0; i < 16; ++i) x[i] = col[(i >> 2) * SA + (i & 3) * SB];
@@ -517,108 +500,274 @@ __device__ __forceinline__ void cols_apply(double *w, const dm_op &op, const dou
     for (int i = 0; i < 16; ++i) col[(i >> 2) * SA + (i & 3) * SB] = x[i];
 }
 
-// Columns k0 .. k0 + C - 1 (k0 a multiple of C) of the round of operations ops[o] .. ops[oe - 1] by
-// one warp, w its C columns of scratch; the round's images at img (three or two of them).  Packed: op
-// o's coefficients are at mats + kCoefStride * o instead of mats + moff.
-template <bool Map2, bool Packed, int C>
-__device__ void compose_warp(const dm_op *ops, int o, int oe, int k0, const double *__restrict__ mats, double *w,
-                             uint16_t *__restrict__ img, bool three, int lane) {
-    auto coef = [&](int i) { return mats + (Packed ? kCoefStride * i : ops[i].moff); };
-    // the leading 4x4 maps, at most one per digit: their Kronecker product
-    const double *lead[3] = {nullptr, nullptr, nullptr};
-    for (; o < oe && ops[o].kind == DM_OP_MAP1; ++o) {
-        const int d = (ops[o].flags >> 8) & 3;
-        if (d == 0 ? lead[0] != nullptr : d == 1 ? lead[1] != nullptr : lead[2] != nullptr) break;
-        const double *m = coef(o);
-        if (d == 0) lead[0] = m;
-        else if (d == 1) lead[1] = m;
-        else lead[2] = m;
-    }
+__device__ __forceinline__ void load_map(double (&m)[16], const double *__restrict__ mg, bool &row0, bool &xy) {
 #pragma unroll
-    for (int it = 0; it < 2 * C; ++it) {   // lane's rows j of column c
-        const int c = it >> 1, j = lane + 32 * (it & 1), k = k0 + c;
-        const double f0 = lead[0] ? lead[0][4 * (j & 3) + (k & 3)] : ((j ^ k) & 3 ? 0.0 : 1.0);
-        const double f1 = lead[1] ? lead[1][4 * ((j >> 2) & 3) + ((k >> 2) & 3)] : ((j ^ k) & 12 ? 0.0 : 1.0);
-        const double f2 = lead[2] ? lead[2][4 * (j >> 4) + (k >> 4)] : ((j ^ k) & 48 ? 0.0 : 1.0);
-        w[c * kColStride + j] = f2 * f1 * f0;
+    for (int i = 0; i < 16; ++i) m[i] = mg[i];
+    row0 = m[0] == 1.0 && m[1] == 0.0 && m[2] == 0.0 && m[3] == 0.0;
+    xy = row0 && m[4] == 0.0 && m[8] == 0.0;
+}
+
+// u (a map's entry) -> FP16 parts h = fp16(u), l = fp16(2**11 (u - h)), both rounded to nearest as from
+// the FP64 values.  |u| = f + g, f its leading 24 bits, g the 29 below; f and f - h + g are rounded to odd
+// where bits are dropped, which a later rounding to 11 bits does not notice.
+__device__ __forceinline__ void split_bits(double u, uint16_t &h16, uint16_t &l16) {
+    const uint32_t hi = uint32_t(__double2hiint(u)), lo = uint32_t(__double2loint(u));
+    const int e = int((hi >> 20) & 0x7FF) - 1023;
+    const uint32_t sign = (hi >> 16) & 0x8000u;
+    if (e > 14) {                          // beyond FP16 (or not a number): the conversions' own results
+        const __half h = __double2half(u);
+        h16 = __half_as_ushort(h);
+        l16 = __half_as_ushort(__double2half((u - double(__half2float(h))) * double(kLoScale)));
+        return;
     }
+    if (e < -60) {                         // both parts round to zero
+        h16 = l16 = uint16_t(sign);
+        return;
+    }
+    const uint32_t tail = lo & 0x1FFFFFFFu;
+    const uint32_t fb = uint32_t(e + 127) << 23 | (hi & 0xFFFFFu) << 3 | lo >> 29;
+    const __half h = __float2half_rn(__uint_as_float(fb | (tail != 0 ? 1u : 0u)));
+    const float a = __uint_as_float(fb) - __half2float(h);        // exact
+    const float t = __uint2float_rz(tail);
+    const float g = __uint_as_float(__float_as_uint(t) | (uint32_t(t) != tail ? 1u : 0u)) *
+                    __uint_as_float(uint32_t(e - 52 + 127) << 23);
+    const float s = __fadd_rz(a, g);
+    const uint32_t odd = g - (s - a) != 0.0f ? 1u : 0u;
+    const __half l = __float2half_rn(__uint_as_float(__float_as_uint(s) | odd) * kLoScale);
+    h16 = uint16_t(__half_as_ushort(h) | sign);
+    l16 = uint16_t(__half_as_ushort(l) ^ sign);
+}
+
+// How a round's operations [begin, end) are composed: up to `stop` as the two blocks, T2's pair
+// operations from p2 on.  Without a second pair T2 holds maps on c alone (single).
+struct RoundPlan {
+    int16_t begin, p2, stop, end;
+    int8_t y, x, c, single;
+};
+
+__device__ __forceinline__ RoundPlan plan_round(const dm_op *ops, int begin, int end) {
+    RoundPlan P;
+    int m1 = 0, m2 = 0, p2 = end, stop = end;
+    for (int i = begin; i < end; ++i) {
+        const dm_op &op = ops[i];
+        if (op.kind == DM_OP_MAP1) continue;
+        const int m = (1 << ((op.flags >> 8) & 3)) | (1 << ((op.flags >> 12) & 3));
+        if (m1 == 0) {
+            m1 = m;
+        } else if (m2 == 0) {
+            if (m != m1) {
+                m2 = m;
+                p2 = i;
+            }
+        } else if (m != m2) {
+            stop = i;
+            break;
+        }
+    }
+    if (m1 == 0) m1 = 3;
+    const int c = 31 - __clz(7 ^ m1), x = __ffs(m2 ? m1 & m2 : m1) - 1;
+    P.begin = int16_t(begin);
+    P.p2 = int16_t(p2);
+    P.stop = int16_t(stop);
+    P.end = int16_t(end);
+    P.c = int8_t(c);
+    P.x = int8_t(x);
+    P.y = int8_t(3 - c - x);
+    P.single = m2 == 0;
+    return P;
+}
+
+// A pass's operations in shared memory (an operation's own read from global memory would cost every warp
+// a round trip per operation), 16 coefficients each; 16x16 maps keep theirs at mats + moff.
+struct ComposeShared {
+    double coefs[DM_MAX_PASS_OPS * kCoefStride];
+    dm_op ops[DM_MAX_PASS_OPS];
+    RoundPlan plan[DM_MAX_ROUNDS];
+};
+static_assert(sizeof(dm_op) == 16, "operations are copied as words");
+
+// The operations of rounds [r0, r1) of a pass and their plans (all threads of the block).
+__device__ __forceinline__ void compose_load(ComposeShared &cs, const dm_batch_pass &bp, const double *__restrict__ mats,
+                                             int r0, int r1) {
+    const int o0 = r0 > 0 ? bp.round_end[r0 - 1] : 0, o1 = bp.round_end[r1 - 1];
+    for (int i = o0 * kCoefStride + int(threadIdx.x); i < o1 * kCoefStride; i += blockDim.x) {
+        const dm_op &op = bp.ops[i / kCoefStride];
+        if (op.kind != DM_OP_MAP2 && (op.kind != DM_OP_CX || i % kCoefStride < 5))
+            cs.coefs[i] = mats[op.moff + i % kCoefStride];
+    }
+    for (int i = o0 * 4 + int(threadIdx.x); i < o1 * 4; i += blockDim.x)
+        reinterpret_cast<uint32_t *>(cs.ops)[i] = reinterpret_cast<const uint32_t *>(bp.ops)[i];
+    __syncthreads();
+    for (int r = r0 + int(threadIdx.x); r < r1; r += blockDim.x)
+        cs.plan[r] = plan_round(cs.ops, r > 0 ? bp.round_end[r - 1] : 0, bp.round_end[r]);
+    __syncthreads();
+}
+
+template <bool Map2>
+__device__ __forceinline__ const double *op_coefs(const ComposeShared &cs, const double *mats, int i) {
+    return Map2 && cs.ops[i].kind == DM_OP_MAP2 ? mats + cs.ops[i].moff : cs.coefs + kCoefStride * i;
+}
+
+// Columns c0 .. c0 + nc - 1 of block T1 (second = false) or T2 of a round by one warp.
+template <bool Map2>
+__device__ void compose_block(const ComposeShared &cs, const RoundPlan &P, const double *mats, bool second, int c0, int nc,
+                              double *blk, int lane) {
+    const int high = second ? P.c : P.y;
+    double *w = blk + c0 * kBlkStride;
+    for (int i = lane; i < nc * 16; i += 32) w[(i >> 4) * kBlkStride + (i & 15)] = (i & 15) == c0 + (i >> 4) ? 1.0 : 0.0;
     __syncwarp();
-    for (; o < oe; ++o) {
-        cols_apply<Map2, C>(w, ops[o], coef(o), lane);
+    for (int i = P.begin; i < P.stop; ++i) {
+        const dm_op &op = cs.ops[i];
+        const int da = (op.flags >> 8) & 3;
+        if (op.kind == DM_OP_MAP1) {
+            if ((da == P.x ? i >= P.p2 : da == P.c) != second) continue;
+            double m[16];
+            bool row0, xy;
+            load_map(m, op_coefs<Map2>(cs, mats, i), row0, xy);
+            const int S = da == high ? 4 : 1;
+            for (int g = lane; g < nc * 4; g += 32)
+                map1_at(w + (g >> 2) * kBlkStride + (g & 3) * (5 - S), S, m, row0, xy);
+        } else {
+            if ((i >= P.p2) != second) continue;
+            const int SA = da == high ? 4 : 1;
+            if (lane < nc) pair_at<Map2>(w + lane * kBlkStride, SA, 5 - SA, op, op_coefs<Map2>(cs, mats, i));
+        }
         __syncwarp();
     }
-    // row j of the C columns: one chunk of C halves per image (16 bytes of 8 columns)
+}
+
+// Columns k0 .. k0 + C - 1 (k0 a multiple of C) of a round from its blocks by one warp, into the images at
+// img (three or two of them); w: the warp's scratch of C columns.
+template <bool Map2, int C>
+__device__ void compose_cols(const ComposeShared &cs, const RoundPlan &P, const double *mats, const double *t1,
+                             const double *t2, int k0, double *w, uint16_t *__restrict__ img, bool three, int lane) {
+    const bool more = P.stop < P.end;
     const int uh = three ? 8192 : 0;   // three: 2**11 Uh at 0, Ul at 4096, Uh at 8192; two: Uh at 0, Ul at 4096
-    struct alignas(2 * C) Chunk {
+    struct alignas(2 * C) Chunk {      // row j of the C columns: one chunk of C halves per image
         uint32_t v[C / 2];
     };
+    double u[C];
+    auto entries = [&](int j) {
+        const int jy = (j >> (2 * P.y)) & 3, jx = (j >> (2 * P.x)) & 3, jc = (j >> (2 * P.c)) & 3;
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-        const int j = lane + 32 * half;
+        for (int c = 0; c < C; ++c) {
+            const int k = k0 + c, ky = (k >> (2 * P.y)) & 3, kx = (k >> (2 * P.x)) & 3, kc = (k >> (2 * P.c)) & 3;
+            const double *a = t1 + (4 * ky + kx) * kBlkStride + 4 * jy;
+            const double *b = t2 + 4 * kc * kBlkStride + 4 * jc;
+            if (P.single) {
+                u[c] = b[0] * a[jx];
+            } else {
+                u[c] = b[jx] * a[0];
+#pragma unroll
+                for (int m = 1; m < 4; ++m) u[c] = fma(b[m * kBlkStride + jx], a[m], u[c]);
+            }
+        }
+    };
+    auto images = [&](int j) {
         const uint32_t pos = uint32_t(k0 >> 3) * 64 + uint32_t(k0 & 7) + uint32_t(j & 7) * 8 + uint32_t(j >> 3) * 512;
         Chunk h2, l2, s2;
 #pragma unroll
         for (int c = 0; c < C; c += 2) {
-            const double u0 = w[c * kColStride + j], u1 = w[(c + 1) * kColStride + j];
-            const __half h0 = __double2half(u0), h1 = __double2half(u1);
-            const float f0 = __half2float(h0), f1 = __half2float(h1);
-            const __half l0 = __double2half((u0 - double(f0)) * double(kLoScale));
-            const __half l1 = __double2half((u1 - double(f1)) * double(kLoScale));
-            h2.v[c >> 1] = uint32_t(__half_as_ushort(h0)) | (uint32_t(__half_as_ushort(h1)) << 16);
-            l2.v[c >> 1] = uint32_t(__half_as_ushort(l0)) | (uint32_t(__half_as_ushort(l1)) << 16);
-            s2.v[c >> 1] = uint32_t(__half_as_ushort(__float2half_rn(f0 * kLoScale))) |
-                           (uint32_t(__half_as_ushort(__float2half_rn(f1 * kLoScale))) << 16);
+            uint16_t h0, h1, l0, l1;
+            split_bits(u[c], h0, l0);
+            split_bits(u[c + 1], h1, l1);
+            h2.v[c >> 1] = uint32_t(h0) | (uint32_t(h1) << 16);
+            l2.v[c >> 1] = uint32_t(l0) | (uint32_t(l1) << 16);
+            const __half2 s = __floats2half2_rn(__half2float(__ushort_as_half(h0)) * kLoScale,
+                                                __half2float(__ushort_as_half(h1)) * kLoScale);
+            s2.v[c >> 1] = *reinterpret_cast<const uint32_t *>(&s);
         }
         if (three) *reinterpret_cast<Chunk *>(img + pos) = s2;
         *reinterpret_cast<Chunk *>(img + 4096 + pos) = l2;
         *reinterpret_cast<Chunk *>(img + uh + pos) = h2;
+    };
+    if (!more) {
+#pragma unroll 1
+        for (int half = 0; half < 2; ++half) {
+            entries(lane + 32 * half);
+            images(lane + 32 * half);
+        }
+        return;
     }
-    __syncwarp();   // the columns are read before the next round's are written
+#pragma unroll 1
+    for (int half = 0; half < 2; ++half) {
+        entries(lane + 32 * half);
+#pragma unroll
+        for (int c = 0; c < C; ++c) w[c * kColStride + lane + 32 * half] = u[c];
+    }
+    __syncwarp();
+    for (int i = P.stop; i < P.end; ++i) {
+        const dm_op &op = cs.ops[i];
+        const int da = (op.flags >> 8) & 3, db = (op.flags >> 12) & 3;
+        if (op.kind == DM_OP_MAP1) {
+            double m[16];
+            bool row0, xy;
+            load_map(m, op_coefs<Map2>(cs, mats, i), row0, xy);
+            const int S = 1 << (2 * da), g = lane & 15;
+            double *col = w + (lane >> 4) * kColStride + (((g >> (2 * da)) << (2 * da + 2)) | (g & (S - 1)));
+#pragma unroll
+            for (int it = 0; it < C / 2; ++it) map1_at(col + 2 * it * kColStride, S, m, row0, xy);
+        } else if (lane < 4 * C) {     // lane = (column, value of the third digit)
+            pair_at<Map2>(w + (lane >> 2) * kColStride + (lane & 3) * (1 << (2 * (3 - da - db))), 1 << (2 * da),
+                          1 << (2 * db), op, op_coefs<Map2>(cs, mats, i));
+        }
+        __syncwarp();
+    }
+#pragma unroll 1
+    for (int half = 0; half < 2; ++half) {
+#pragma unroll
+        for (int c = 0; c < C; ++c) u[c] = w[c * kColStride + lane + 32 * half];
+        images(lane + 32 * half);
+    }
+    __syncwarp();   // the columns are read before the next item's are written
 }
 
-// This CTA's share of a batched pass's round images (three per round): the group's ranks take the
-// (round, columns) items in turn, warp by warp; the operand region is free between passes.  Alone a
-// CTA takes 8 columns per warp, which fills the lanes in pair operations; in a group 2, which spreads
-// a round over all SM quarters (one FP64 warp instruction per 64 cycles each).
-struct ComposeShared {                // behind the columns in the operand region
-    double coefs[DM_MAX_PASS_OPS * kCoefStride];
-    dm_op ops[DM_MAX_PASS_OPS];
-    int16_t round_end[DM_MAX_ROUNDS];
+// A batched pass's composition works in the operand region, which is free between passes: the blocks of
+// up to kBlockRounds rounds, the warps' columns, the operations.
+constexpr int kBlockRounds = 8;
+struct ComposeWork {
+    double blocks[kBlockRounds * 2 * kBlkDoubles];
+    double cols[kThreads / 32 * 8 * kColStride];
+    ComposeShared cs;
 };
-static_assert(kColBytes + sizeof(ComposeShared) <= kSmemBytes, "columns and operations fit the pass's shared memory");
+static_assert(sizeof(ComposeWork) <= kSmemBytes, "blocks, columns and operations fit the pass's shared memory");
 
+// This CTA's share of a batched pass's round images (three per round): the group's ranks take equal runs
+// of (round, columns) items and compose the blocks of their own rounds; alone a CTA takes 8 columns per
+// warp and whole blocks, in a group 2 and half blocks, for the work is then spread thinner than the warps.
 template <int C>
-__device__ void compose_items(const ComposeShared &cs, int nrounds, uint16_t *__restrict__ umats, double *work,
-                              int rank, int G) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int i = rank + G * warp; i < nrounds * (64 / C); i += G * (kThreads / 32)) {
-        const int r = i / (64 / C), k0 = i % (64 / C) * C;
-        compose_warp<false, true, C>(cs.ops, r > 0 ? cs.round_end[r - 1] : 0, cs.round_end[r], k0, cs.coefs,
-                                     work + warp * C * kColStride, umats + int64_t(r) * kUHalves, true, lane);
+__device__ void compose_items(ComposeWork &cw, int nrounds, uint16_t *__restrict__ umats, int rank, int G) {
+    constexpr int kPer = 64 / C, nc = C == 8 ? 16 : 8;       // items of a round, columns of a block unit
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = kThreads / 32;
+    const int total = nrounds * kPer, first = total * rank / G, last = total * (rank + 1) / G;
+    for (int rb = first / kPer; rb * kPer < last; rb += kBlockRounds) {
+        const int re = min(rb + kBlockRounds, (last + kPer - 1) / kPer);
+        for (int i = warp; i < (re - rb) * 2 * (16 / nc); i += warps) {
+            const int b = i / (16 / nc);
+            compose_block<false>(cw.cs, cw.cs.plan[rb + (b >> 1)], nullptr, b & 1, i % (16 / nc) * nc, nc,
+                                 cw.blocks + b * kBlkDoubles, lane);
+        }
+        __syncthreads();
+        for (int i = max(first, rb * kPer) + warp; i < min(last, re * kPer); i += warps) {
+            const int r = i / kPer, b = 2 * (r - rb);
+            compose_cols<false, C>(cw.cs, cw.cs.plan[r], nullptr, cw.blocks + b * kBlkDoubles,
+                                   cw.blocks + (b + 1) * kBlkDoubles, i % kPer * C, cw.cols + warp * C * kColStride,
+                                   umats + int64_t(r) * kUHalves, true, lane);
+        }
+        __syncthreads();
     }
 }
 
-// The pass's operations and coefficients are copied to shared memory first: an operation's own read
-// from global memory would cost every warp a round trip per operation.
 __device__ __noinline__ void compose_share(const dm_batch_pass &bp, const double *mats, uint16_t *umats,
                                            unsigned char *smem, int rank, int G) {
-    ComposeShared &cs = *reinterpret_cast<ComposeShared *>(smem + kColBytes);
-    const int nops = bp.nops, nr = bp.nrounds;
-    for (int i = threadIdx.x; i < nops * kCoefStride; i += kThreads) {
-        const dm_op &op = bp.ops[i / kCoefStride];
-        if (op.kind != DM_OP_CX || i % kCoefStride < 5) cs.coefs[i] = mats[op.moff + i % kCoefStride];
-    }
-    for (int i = threadIdx.x; i < nops * 4; i += kThreads)
-        reinterpret_cast<uint32_t *>(cs.ops)[i] = reinterpret_cast<const uint32_t *>(bp.ops)[i];
-    for (int i = threadIdx.x; i < nr; i += kThreads) cs.round_end[i] = bp.round_end[i];
-    __syncthreads();
-    double *work = reinterpret_cast<double *>(smem);
+    ComposeWork &cw = *reinterpret_cast<ComposeWork *>(smem);
+    const int nr = bp.nrounds;
+    compose_load(cw.cs, bp, mats, 0, nr);
     if (G < 8)
-        compose_items<8>(cs, nr, umats, work, rank, G);
+        compose_items<8>(cw, nr, umats, rank, G);
     else
-        compose_items<2>(cs, nr, umats, work, rank, G);
+        compose_items<2>(cw, nr, umats, rank, G);
 }
-static_assert(sizeof(dm_op) == 16, "operations are copied as words");
 
 // ---------------------------------------------------------------------------
 // groups of CTAs
@@ -778,19 +927,28 @@ __device__ __forceinline__ void group_init_zero(float *st, int n, int rank, int 
     }
 }
 
-// The single-state launches: CTA (r, c) takes the columns 8c .. 8c + 7 of a round, 2 per warp.
+// The single-state launches: CTA (r, c) takes the columns 8c .. 8c + 7 of a round, 2 per warp, after a
+// quarter of its blocks per warp.
 constexpr int kComposeWarps = 4, kComposeCols = 2, kComposeGrid = 64 / (kComposeWarps * kComposeCols);
+
+__device__ __forceinline__ void compose_round(const dm_batch_pass &bp, int r, const double *__restrict__ mats,
+                                              uint16_t *__restrict__ img, bool three) {
+    __shared__ ComposeShared cs;
+    __shared__ double blocks[2 * kBlkDoubles], cols[kComposeWarps * kComposeCols * kColStride];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    compose_load(cs, bp, mats, r, r + 1);
+    compose_block<true>(cs, cs.plan[r], mats, warp >> 1, (warp & 1) * 8, 8, blocks + (warp >> 1) * kBlkDoubles, lane);
+    __syncthreads();
+    compose_cols<true, kComposeCols>(cs, cs.plan[r], mats, blocks, blocks + kBlkDoubles,
+                                     (int(blockIdx.y) * kComposeWarps + warp) * kComposeCols,
+                                     cols + warp * kComposeCols * kColStride, img, three, lane);
+}
 
 // One pass's round images (CTA x = round of the pass).
 __global__ void __launch_bounds__(32 * kComposeWarps)
     compose_pass_kernel(const __grid_constant__ dm_batch_pass bp, const double *__restrict__ mats,
                         uint16_t *__restrict__ images, int image_halves) {
-    __shared__ double cols[kComposeWarps * kComposeCols * kColStride];
-    const int r = blockIdx.x, warp = threadIdx.x >> 5;
-    compose_warp<true, false, kComposeCols>(bp.ops, r > 0 ? bp.round_end[r - 1] : 0, bp.round_end[r],
-                                            (int(blockIdx.y) * kComposeWarps + warp) * kComposeCols, mats,
-                                            cols + warp * kComposeCols * kColStride, images + int64_t(r) * image_halves,
-                                            image_halves == kUHalves, threadIdx.x & 31);
+    compose_round(bp, blockIdx.x, mats, images + int64_t(blockIdx.x) * image_halves, image_halves == kUHalves);
 }
 
 // The round images of several passes (CTA x = entry of the round table).  A pass's composition alone
@@ -800,14 +958,8 @@ __global__ void __launch_bounds__(32 * kComposeWarps)
 __global__ void __launch_bounds__(32 * kComposeWarps)
     compose_passes_kernel(const dm_batch_pass *__restrict__ passes, const dm_compose_round *__restrict__ rounds,
                           const double *__restrict__ mats, uint16_t *__restrict__ images) {
-    __shared__ double cols[kComposeWarps * kComposeCols * kColStride];
     const dm_compose_round e = rounds[blockIdx.x];
-    const int warp = threadIdx.x >> 5;
-    const dm_batch_pass &bp = passes[e.pass];
-    compose_warp<true, false, kComposeCols>(bp.ops, e.round > 0 ? bp.round_end[e.round - 1] : 0, bp.round_end[e.round],
-                                            (int(blockIdx.y) * kComposeWarps + warp) * kComposeCols, mats + e.mats_off,
-                                            cols + warp * kComposeCols * kColStride, images + e.image_off,
-                                            e.format == DM_IMAGE_TC, threadIdx.x & 31);
+    compose_round(passes[e.pass], e.round, mats + e.mats_off, images + e.image_off, e.format == DM_IMAGE_TC);
 }
 
 // Shared memory of the batched kernels beside the operand and matrix regions.  In a group the tile

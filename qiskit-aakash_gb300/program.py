@@ -777,23 +777,35 @@ def _choose_layouts_tma_cached(rounds_axes):
 def _tma_last_candidates(axes, prev):
     """(digits, rowbits) candidates of the last round of a TMA-fed pass, which stores its rows to
     global memory: with local axis 0 among its axes, axis 0 is K digit 0 (four contiguous
-    coefficients per thread, 16-byte stores); otherwise tile bits 0-3 (axes 0 and 1, or axis 0
-    and the lowest free bits) are rows 0-3, so 16 lanes cover contiguous coefficients."""
+    coefficients per thread, 16-byte stores) and axis 1 among the lanes; otherwise tile bits 0-3
+    (axes 0 and 1, or axis 0 and the lowest free bits) are rows 0-3, so 16 lanes cover contiguous
+    coefficients.
+
+    What the epilogue into this round costs depends on which bits are rows 0-2 (the banks of an
+    operand row), not on their order: one candidate per choice.  (With the rows in one fixed order
+    where axis 0 is a K digit, the incoming epilogue met 4- to 16-way bank conflicts: a 16-way
+    transition takes as many shared-memory cycles as seven rounds without.)"""
     import itertools
     nonround = [tb for tb in range(2 * TC_AXES) if tb // 2 not in axes]
     out = []
     if 0 in axes:
         others = [a for a in axes if a != 0]
-        rows = nonround
-        for perm in itertools.permutations(others):
-            out.append(([0] + list(perm), rows))
+        near = [tb for tb in (2, 3) if tb in nonround]
+        for tri in itertools.combinations(nonround, 3):
+            rows = _fill_rows(list(tri), near, [], nonround)
+            for perm in itertools.permutations(others):
+                out.append(([0] + list(perm), rows))
         return out
     head = [tb for tb in TMA_FIXED_ROWS if tb in nonround]
     head += [tb for tb in nonround if tb not in head][:4 - len(head)]
     rest = [tb for tb in nonround if tb not in head]
+    if 1 in axes:                                     # rows 0-1 hold axis 0, row 2 any other bit
+        heads = [head[:2] + [tb] + [x for x in head[2:] if x != tb] for tb in nonround if tb not in head[:2]]
+    else:
+        heads = [head[i + 1:] + head[:i + 1] for i in range(4)]      # each of the four as row 3
     for digits in itertools.permutations(axes):
-        for h in itertools.permutations(head):      # rows 0-3 in any order: lanes 0-15 stay contiguous
-            out.append((list(digits), list(h) + rest))
+        for h in heads:
+            out.append((list(digits), h + [tb for tb in rest if tb not in h]))
     return out
 
 
