@@ -36,14 +36,19 @@
 namespace dmg {
 namespace mlp {
 
-constexpr int kThreads = 512;
 constexpr int kBM = 128, kBN = 64, kBK = 64;
 constexpr uint32_t kABytes = kBM * kBK * 2;        // 16 KB
 constexpr uint32_t kBBytes = kBN * kBK * 2;        // 8 KB
 constexpr uint32_t kStage = kABytes + kBBytes;     // 24 KB
-constexpr int kStages = 4;
-constexpr uint32_t kSmemBytes = kStages * kStage + 1024;   // 97 KB with alignment slack: two CTAs per SM
-constexpr int kCols = kBN / 4;                     // columns of a thread in the epilogue
+// Threads, stages and CTAs per SM of a launch: few tiles get deep pipelines and wide epilogues, many
+// tiles more CTAs at once, one's loads and MMAs beside the others' epilogues.
+template <int T, int S, int P>
+struct Shape {
+    static constexpr int kThreads = T, kStages = S, kPerSm = P;
+    static constexpr uint32_t kSmemBytes = S * kStage + 1024;        // with alignment slack
+};
+using Deep = Shape<512, 4, 2>;       // 97 KB
+using Wide = Shape<256, 2, 4>;       // 49 KB
 constexpr int kF32Row = kBN + 4;                   // epilogue rows in shared memory: FP32 values,
 constexpr int kBf16Row = kBN + 8;                  // BF16 values (16-byte accesses of 8 rows hit all banks)
 constexpr int kMaxGroup = 4;                       // products per launch
@@ -103,8 +108,10 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
     for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
 }
 
-template <int EPI>
-__global__ void __launch_bounds__(kThreads, 2) gemm_kernel(const __grid_constant__ GemmGroup G, int *status) {
+template <int EPI, typename Sh>
+__global__ void __launch_bounds__(Sh::kThreads, Sh::kPerSm) gemm_kernel(const __grid_constant__ GemmGroup G, int *status) {
+    constexpr int kThreads = Sh::kThreads, kStages = Sh::kStages;
+    constexpr int kCols = kBM * kBN / kThreads;       // columns of a thread in the epilogue
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t full[kStages], empty[kStages], done;
     __shared__ uint32_t tmem_base_s;
@@ -194,10 +201,16 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_kernel(const __grid_constant
     __syncthreads();
 
     if (!*static_cast<volatile int *>(&abort_s)) {
-        // the thread's row and its 16 columns
+        // the thread's row and columns
         const int row = 32 * (warp & 3) + lane, c0 = kCols * (warp >> 2);
         float v[kCols];
-        tmem_ld16(tmem + (uint32_t(32 * (warp & 3)) << 16) + uint32_t(c0), v);
+#pragma unroll
+        for (int j = 0; j < kCols; j += 16) {
+            float part[16];
+            tmem_ld16(tmem + (uint32_t(32 * (warp & 3)) << 16) + uint32_t(c0 + j), part);
+#pragma unroll
+            for (int e = 0; e < 16; ++e) v[j + e] = part[e];
+        }
         float *st = reinterpret_cast<float *>(smem);             // the tile in FP32 rows, then in BF16 rows
         if constexpr (EPI == DM_MLP_EPI_GELU_FWD || EPI == DM_MLP_EPI_BIAS_F32) {
 #pragma unroll
@@ -238,8 +251,10 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_kernel(const __grid_constant
             }
         }
         if constexpr (EPI == DM_MLP_EPI_GELU_FWD || EPI == DM_MLP_EPI_GELU_BWD) {
-            // behind the FP32 rows
-            uint16_t *sb = reinterpret_cast<uint16_t *>(smem + kBM * kF32Row * 4);
+            // behind the FP32 rows, or in their place
+            constexpr bool apart = kStages * kStage >= kBM * (kF32Row * 4 + kBf16Row * 2);
+            uint16_t *sb = reinterpret_cast<uint16_t *>(smem + (apart ? kBM * kF32Row * 4 : 0));
+            if (!apart && (EPI == DM_MLP_EPI_GELU_BWD || g.out_f32)) __syncthreads();
 #pragma unroll
             for (int j = 0; j < kCols; j += 8)
                 *reinterpret_cast<uint4 *>(sb + row * kBf16Row + c0 + j) =
@@ -490,63 +505,91 @@ __global__ void __launch_bounds__(256) adam_kernel(float *__restrict__ params, c
     }
 }
 
-// Row r of member z from sample index[z * rows + r], or sample first + r without an index (the last one
-// beyond the data set); the members' rows lie row_ms apart.
+// Row r of member z from sample index[z * rows + r].
 __global__ void gather_kernel(const float *__restrict__ features, int nfeat, const float *__restrict__ targets,
-                              int nout, int64_t samples, const int32_t *__restrict__ index, int64_t first, int rows,
-                              int64_t row_ms, int width, uint16_t *__restrict__ x, uint16_t *__restrict__ xt,
-                              float *__restrict__ t) {
+                              int nout, int64_t samples, const int32_t *__restrict__ index, int rows, int width,
+                              uint16_t *__restrict__ x, uint16_t *__restrict__ xt, float *__restrict__ t) {
     const int64_t r = blockIdx.x, z = blockIdx.y;
     grid_wait();
     features = waited(features);
     targets = waited(targets);
-    index = waited(index);
-    int64_t s;
-    if (index) {
-        s = index[z * rows + r];
-        if (s < 0 || s >= samples) s = 0;   // an index outside the data set reads sample 0
-    } else {
-        s = first + r < samples ? first + r : samples - 1;
-    }
+    int64_t s = waited(index)[z * rows + r];
+    if (s < 0 || s >= samples) s = 0;       // an index outside the data set reads sample 0
     if (targets) {
         const float4 *src = reinterpret_cast<const float4 *>(targets + s * nout);
-        float4 *dst = reinterpret_cast<float4 *>(t + (z * row_ms + r) * nout);
+        float4 *dst = reinterpret_cast<float4 *>(t + (z * rows + r) * nout);
         for (int j = threadIdx.x; j < nout / 4; j += blockDim.x) dst[j] = src[j];
     }
     for (int f = threadIdx.x; f < width; f += blockDim.x) {
         const uint16_t b = to_bf16(f < nfeat ? features[s * nfeat + f] : 0.f);
-        x[(z * row_ms + r) * width + f] = b;
-        if (xt) xt[(z * width + f) * row_ms + r] = b;
+        x[(z * rows + r) * width + f] = b;
+        xt[(z * width + f) * rows + r] = b;
     }
+}
+
+// Rows of samples first, first + 1, ... (the last one beyond the data set) for every member alike, kPackCols
+// BF16 values per thread.
+constexpr int kPackCols = 8, kPackWidth = 64;
+__global__ void pack_kernel(const float *__restrict__ features, int nfeat, int64_t samples, int64_t first, int rows,
+                            uint16_t *__restrict__ x) {
+    grid_wait();
+    features = waited(features);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, r = i / (kPackWidth / kPackCols);
+    if (r >= rows) return;
+    const int f0 = i % (kPackWidth / kPackCols) * kPackCols;
+    const int64_t s = first + r < samples ? first + r : samples - 1;
+    float v[kPackCols];
+#pragma unroll
+    for (int e = 0; e < kPackCols; ++e) v[e] = f0 + e < nfeat ? features[s * nfeat + f0 + e] : 0.f;
+    *reinterpret_cast<uint4 *>(x + int64_t(i) * kPackCols) =
+        make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
 }
 
 // One CTA per row: every member's deviation is reduced within the warps, the CTA meets once, and one lane
 // per member adds its warps' sums (thread 0 alone over all of them was a chain of 48 shared-memory reads).
 // 5 members x 10,233 rows x 1,024 columns, 252 MB: 139 -> 75 us.
-template <int Members>
+static bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+// Four columns per load where the rows are 16-byte aligned.
+template <int Members, bool Vec>
 __global__ void __launch_bounds__(kRowThreads) ensemble_kernel(const float *__restrict__ probs, int rows, int nout,
                                                                const float *__restrict__ ref, float *__restrict__ mean,
                                                                float *__restrict__ spread, float *__restrict__ tv_ref) {
+    constexpr int V = Vec ? 4 : 1;
     __shared__ float red[kRowThreads / 32][Members + 1];
     const int64_t r = blockIdx.x;
     float dev[Members + 1] = {};                          // the members', then the reference's
     grid_wait();
     probs = waited(probs);
     ref = waited(ref);
-#pragma unroll 4
-    for (int j = threadIdx.x; j < nout; j += kRowThreads) {
-        float q[Members];
-        float mu = 0.f;
-#pragma unroll
-        for (int zz = 0; zz < Members; ++zz) {
-            q[zz] = probs[(int64_t(zz) * rows + r) * nout + j];
-            mu += q[zz];
+    auto load = [](const float *p, float (&v)[V]) {
+        if constexpr (Vec) {
+            const float4 f = *reinterpret_cast<const float4 *>(p);
+            v[0] = f.x, v[1] = f.y, v[2] = f.z, v[3] = f.w;
+        } else {
+            v[0] = *p;
         }
-        mu /= float(Members);
-        mean[r * nout + j] = mu;
+    };
+#pragma unroll 2
+    for (int j = V * threadIdx.x; j < nout; j += V * kRowThreads) {
+        float q[Members][V], mu[V], rv[V];
 #pragma unroll
-        for (int zz = 0; zz < Members; ++zz) dev[zz] += fabsf(q[zz] - mu);
-        if (ref) dev[Members] += fabsf(mu - ref[r * nout + j]);
+        for (int zz = 0; zz < Members; ++zz) load(probs + (int64_t(zz) * rows + r) * nout + j, q[zz]);
+        if (ref) load(ref + r * nout + j, rv);
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+            mu[e] = q[0][e];
+#pragma unroll
+            for (int zz = 1; zz < Members; ++zz) mu[e] += q[zz][e];
+            mu[e] /= float(Members);
+#pragma unroll
+            for (int zz = 0; zz < Members; ++zz) dev[zz] += fabsf(q[zz][e] - mu[e]);
+            if (ref) dev[Members] += fabsf(mu[e] - rv[e]);
+        }
+        if constexpr (Vec)
+            *reinterpret_cast<float4 *>(mean + r * nout + j) = make_float4(mu[0], mu[1], mu[2], mu[3]);
+        else
+            mean[r * nout + j] = mu[0];
     }
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
@@ -574,10 +617,14 @@ __global__ void __launch_bounds__(kRowThreads) ensemble_kernel(const float *__re
 static int launch_ensemble(const float *probs, int rows, int members, int nout, const float *ref, float *mean,
                            float *spread, float *tv_ref, cudaStream_t s) {
     using Kernel = void (*)(const float *, int, int, const float *, float *, float *, float *);
-    static constexpr Kernel kernels[8] = {ensemble_kernel<1>, ensemble_kernel<2>, ensemble_kernel<3>, ensemble_kernel<4>,
-                                          ensemble_kernel<5>, ensemble_kernel<6>, ensemble_kernel<7>, ensemble_kernel<8>};
-    return launch_early(kernels[members - 1], dim3(rows), dim3(kRowThreads), 0, s, probs, rows, nout, ref, mean, spread,
-                        tv_ref);
+    static constexpr Kernel kernels[2][8] = {
+        {ensemble_kernel<1, false>, ensemble_kernel<2, false>, ensemble_kernel<3, false>, ensemble_kernel<4, false>,
+         ensemble_kernel<5, false>, ensemble_kernel<6, false>, ensemble_kernel<7, false>, ensemble_kernel<8, false>},
+        {ensemble_kernel<1, true>, ensemble_kernel<2, true>, ensemble_kernel<3, true>, ensemble_kernel<4, true>,
+         ensemble_kernel<5, true>, ensemble_kernel<6, true>, ensemble_kernel<7, true>, ensemble_kernel<8, true>}};
+    const bool vec = nout % 4 == 0 && aligned16(probs) && aligned16(mean) && (!ref || aligned16(ref));
+    return launch_early(kernels[vec][members - 1], dim3(rows), dim3(kRowThreads), 0, s, probs, rows, nout, ref, mean,
+                        spread, tv_ref);
 }
 
 using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
@@ -612,10 +659,16 @@ static bool operand_map(CUtensorMap *map, const uint16_t *base, int K, int rows,
 }
 
 // count products of one epilogue and member count in one launch
+template <int EPI, typename Sh>
+static int launch_shape(const GemmGroup &G, int members, int *status, cudaStream_t s) {
+    auto kernel = gemm_kernel<EPI, Sh>;
+    if (ensure_max_dynamic_smem(reinterpret_cast<const void *>(kernel), int(Sh::kSmemBytes)) != cudaSuccess)
+        return DM_ERR_CUDA;
+    return launch_early(kernel, dim3(G.first[G.count], members), dim3(Sh::kThreads), Sh::kSmemBytes, s, G, status);
+}
+
 template <int EPI>
 static int launch_gemms(const dm_mlp_gemm *g, int count, int *status, cudaStream_t s) {
-    if (ensure_max_dynamic_smem(reinterpret_cast<const void *>(gemm_kernel<EPI>), int(kSmemBytes)) != cudaSuccess)
-        return DM_ERR_CUDA;
     GemmGroup G;
     G.count = count;
     G.first[0] = 0;
@@ -626,10 +679,11 @@ static int launch_gemms(const dm_mlp_gemm *g, int count, int *status, cudaStream
             !operand_map(&G.b[i], g[i].B, g[i].K, g[i].N, g[i].members, g[i].ldb, g[i].b_ms, kBN))
             return DM_ERR_CUDA;
     }
-    return launch_early(gemm_kernel<EPI>, dim3(G.first[count], g[0].members), dim3(kThreads), kSmemBytes, s, G, status);
+    if (int64_t(G.first[count]) * g[0].members > int64_t(Deep::kPerSm) * sm_count())
+        return launch_shape<EPI, Wide>(G, g[0].members, status, s);
+    return launch_shape<EPI, Deep>(G, g[0].members, status, s);
 }
 
-static bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 static bool mult8(int64_t x) { return x >= 0 && (x & 7) == 0; }
 
 }  // namespace mlp
@@ -734,7 +788,7 @@ extern "C" int dm_mlp_gather(const float *features, int nfeat, const float *targ
     DM_CHECK_ARG(rows > 0 && members >= 1 && members <= 65535 && width % 8 == 0 && nout > 0 && nout % 4 == 0);
     DM_CHECK_ARG(!targets || (t && mlp::aligned16(targets) && mlp::aligned16(t)));
     return launch_early(mlp::gather_kernel, dim3(rows, members), dim3(256), 0, as_stream(stream), features, nfeat, targets,
-                        nout, samples, index, int64_t(0), rows, int64_t(rows), width, x, xt, t);
+                        nout, samples, index, rows, width, x, xt, t);
 }
 
 extern "C" int dm_mlp_ensemble(const float *probs, int rows, int members, int nout, const float *ref, float *mean,
@@ -809,7 +863,8 @@ static dm_mlp_gemm product(const dm_mlp_net &n, int epi, int M, int N, int K, co
     return g;
 }
 
-static int forward(const dm_mlp_net &n, int rows, bool train, cudaStream_t s) {
+// x_ms: the members' stride in x (0: the same rows for all)
+static int forward(const dm_mlp_net &n, int rows, bool train, int64_t x_ms, cudaStream_t s) {
     NetLayer L[kLayers];
     int rc = net_layers(n, L);
     const int64_t B = n.batch;
@@ -818,7 +873,7 @@ static int forward(const dm_mlp_net &n, int rows, bool train, cudaStream_t s) {
     for (int i = 0; !rc && i < kLayers; ++i) {
         const bool out = i == kLayers - 1;
         dm_mlp_gemm g = product(n, out ? DM_MLP_EPI_BIAS_F32 : DM_MLP_EPI_GELU_FWD, padded, L[i].out, L[i].in, A, L[i].in,
-                                B * L[i].in, n.wb + L[i].w, L[i].in, n.count);
+                                i == 0 ? x_ms : B * L[i].in, n.wb + L[i].w, L[i].in, n.count);
         g.bias = n.params + L[i].b;
         g.bias_ms = n.count;
         g.ld_f32 = L[i].out;
@@ -895,7 +950,7 @@ static int backward(const dm_mlp_net &n, int rows, cudaStream_t s) {
 }
 
 static int loss_and_grads(const dm_mlp_net &n, int rows, cudaStream_t s) {
-    int rc = forward(n, rows, true, s);
+    int rc = forward(n, rows, true, int64_t(n.batch) * kInput, s);
     if (rc) return rc;
     if ((rc = launch_softmax(n.logits, n.t, rows, n.members, n.nout, n.batch, n.batch, n.batch, float(1.0 / rows), n.probs,
                              n.dz, n.dzt, n.loss_rows, s)))
@@ -908,7 +963,7 @@ static int loss_and_grads(const dm_mlp_net &n, int rows, cudaStream_t s) {
 
 extern "C" int dm_mlp_forward(const dm_mlp_net *net, int rows, int train, void *stream) {
     const int rc = mlp::check_net(net, rows, train != 0);
-    return rc ? rc : mlp::forward(*net, rows, train != 0, as_stream(stream));
+    return rc ? rc : mlp::forward(*net, rows, train != 0, int64_t(net->batch) * mlp::kInput, as_stream(stream));
 }
 
 extern "C" int dm_mlp_backward(const dm_mlp_net *net, int rows, void *stream) {
@@ -948,12 +1003,10 @@ extern "C" int dm_mlp_predict(const dm_mlp_net *net, const float *features, int 
     for (int64_t s0 = 0; s0 < samples; s0 += n.batch) {
         const int rows = int(samples - s0 < n.batch ? samples - s0 : n.batch);
         const int padded = (rows + mlp::kBM - 1) / mlp::kBM * mlp::kBM;
-        rc = launch_early(mlp::gather_kernel, dim3(padded, n.members), dim3(64), 0, s, features, nfeat,
-                          static_cast<const float *>(nullptr), n.nout, samples, static_cast<const int32_t *>(nullptr), s0,
-                          padded, int64_t(n.batch), mlp::kInput, n.x, static_cast<uint16_t *>(nullptr),
-                          static_cast<float *>(nullptr));
+        rc = launch_early(mlp::pack_kernel, dim3((padded * mlp::kPackWidth / mlp::kPackCols + 255) / 256), dim3(256), 0, s,
+                          features, nfeat, samples, s0, padded, n.x);
         if (rc) return rc;
-        if ((rc = mlp::forward(n, rows, false, s))) return rc;
+        if ((rc = mlp::forward(n, rows, false, 0, s))) return rc;
         if ((rc = mlp::launch_softmax(n.logits, nullptr, rows, n.members, n.nout, n.batch, samples, 0, 1.f,
                                       out + s0 * n.nout, nullptr, nullptr, nullptr, s)))
             return rc;

@@ -156,3 +156,38 @@ def test_network_calls_reject_bad_arguments():
     net = ens._net()
     net._obj.h[1] = None
     assert N.lib().dm_mlp_forward(net, 128, 0, None) == N.DM_ERR_ARG
+
+
+@pytest.mark.parametrize('workspace', [1, 3 << 20, 64 << 20])
+@pytest.mark.parametrize('points', [1, 700, 1301])
+def test_predictions_do_not_depend_on_the_workspace(points, workspace, monkeypatch):
+    """Passes of one batch, of several tiles and of all points; member strides and ragged ends."""
+    torch = _torch()
+    ens = S.MLPEnsemble(members=3, batch=128, nout=512, seed=4)
+    f = torch.rand(points, 6, device='cuda', generator=torch.Generator('cuda').manual_seed(points)) * 2 - 1
+    want = torch.cat([ens.predict(f[i:i + 128].contiguous()) for i in range(0, points, 128)], dim=1)
+    monkeypatch.setattr(S, 'PREDICT_WORKSPACE', workspace)
+    assert ens._predict_rows(points) % 128 == 0
+    assert torch.equal(ens.predict(f), want)
+
+
+@pytest.mark.parametrize('nout', [1024, 1023, 4, 1, 258])
+@pytest.mark.parametrize('members', [1, 5, 8])
+def test_ensemble_statistics(nout, members):
+    """Rows that are and are not multiples of four columns, against FP64 sums."""
+    torch = _torch()
+    rows = 5
+    rng = np.random.default_rng(nout + members)
+    p = rng.random((members, rows, nout)).astype(np.float32)
+    ref = rng.random((rows, nout)).astype(np.float32)
+    pd, rd = torch.from_numpy(p).cuda(), torch.from_numpy(ref).cuda()
+    mean = torch.empty((rows, nout), dtype=torch.float32, device='cuda')
+    spread, tv = (torch.empty(rows, dtype=torch.float32, device='cuda') for _ in range(2))
+    vp = ctypes.c_void_p
+    N.call('dm_mlp_ensemble', vp(pd.data_ptr()), rows, members, nout, vp(rd.data_ptr()), vp(mean.data_ptr()),
+           vp(spread.data_ptr()), vp(tv.data_ptr()), None)
+    mu = p.astype(np.float64).mean(axis=0)
+    tol = (nout + 16) * U * max(nout, 1)
+    assert np.abs(mean.cpu().numpy() - mu).max() <= 16 * U
+    assert np.abs(spread.cpu().numpy() - 0.5 * np.abs(p - mu).sum(axis=2).mean(axis=0)).max() <= tol
+    assert np.abs(tv.cpu().numpy() - 0.5 * np.abs(mu - ref).sum(axis=1)).max() <= tol
