@@ -2,12 +2,12 @@
 //
 // The network maps noise parameters to a fixed circuit's outcome
 // distribution.  Its matrix products run on the tensor cores: a CTA computes a
-// 128 x 64 tile of C = A B^T with BF16 operands (kind::f16, FP32 accumulation
-// in 64 TMEM columns).  K is streamed in 64-wide chunks by TMA into kStages
+// 128 x 32 or 128 x 64 tile of C = A B^T with BF16 operands (kind::f16, FP32
+// accumulation in TMEM).  K is streamed in 64-wide chunks by TMA into 2 to 4
 // shared-memory stages (128-byte rows, 128-byte swizzle, K-major): one thread
 // keeps the loads going, another issues the four K = 16 MMAs of a chunk as it
 // lands and commits them to the barrier that frees the stage.  The epilogue
-// runs on 16 warps (32 rows x 16 columns each, tcgen05.ld), applies bias and
+// runs on 8 or 16 warps (32 rows of a quadrant each, tcgen05.ld), applies bias and
 // GELU, or the GELU derivative of the backward pass, and goes through shared
 // memory so that global accesses are whole rows; it writes the row-major result
 // plus, where the next product needs it, its transpose, so that every later
@@ -16,10 +16,11 @@
 // GFLOP at most, and bound by latencies: of a chunk's load, multiply and wait,
 // and of the epilogue's chains.  With 4 warps per CTA (64 columns and 64 tanhf a
 // thread), 16-byte cp.async loads and a wait per chunk the ten products of a
-// training step of 5 x 1,024 rows, 1,024 outcomes took 260 us; with TMA, 4
-// stages and 16 warps the eight launches take 111 us (13 us for 1,024 x 256 x
-// 256, 15 us for 1,024 x 1,024 x 256).  The whole step went from 402 to 192 us,
-// the prediction of 10,233 points from 1,764 to 654 us.
+// training step of 5 x 1,024 rows, 1,024 outcomes took 260 us; with TMA, stages
+// and the work spread over more warps the eight launches take 95 us (11 us for
+// 1,024 x 256 x 256, 13 us for 1,024 x 1,024 x 256).  The whole step went from
+// 402 to 150 us, the prediction of 10,233 points with the ensemble's spread from
+// 1,670 to 283 us.
 // Waits on an mbarrier are bounded and record an error in *status.
 //
 // The other kernels are memory-light helpers: softmax with the KL loss and
@@ -36,26 +37,27 @@
 namespace dmg {
 namespace mlp {
 
-constexpr int kBM = 128, kBN = 64, kBK = 64;
+constexpr int kBM = 128, kBK = 64;
 constexpr uint32_t kABytes = kBM * kBK * 2;        // 16 KB
-constexpr uint32_t kBBytes = kBN * kBK * 2;        // 8 KB
-constexpr uint32_t kStage = kABytes + kBBytes;     // 24 KB
-// Threads, stages and CTAs per SM of a launch: few tiles get deep pipelines and wide epilogues, many
-// tiles more CTAs at once, one's loads and MMAs beside the others' epilogues.
-template <int T, int S, int P>
+// Tile width, threads, stages and CTAs per SM of a launch.  Tiles beyond two per SM: four CTAs per SM, one's
+// loads and MMAs beside the others' epilogues (3,456 x 1,024 x 256 for 5 members: 35 us with two of 512
+// threads per SM, 27 us).  Fewer: half the tile's columns, twice the CTAs (1,024 x 256 x 256: 13.3 us with 64
+// columns, 11.0 us; the GELU derivative's 1,024 x 256 x 1,024: 17.1 and 15.7 us), unless K is long and the
+// epilogue only stores (the weight gradients, K = 1,024: 17.7 us with 32 columns, 11.0 us with 64).
+template <int BN, int T, int S, int P>
 struct Shape {
-    static constexpr int kThreads = T, kStages = S, kPerSm = P;
+    static constexpr int kBN = BN, kThreads = T, kStages = S, kPerSm = P;
+    static constexpr uint32_t kStage = kABytes + BN * kBK * 2;
     static constexpr uint32_t kSmemBytes = S * kStage + 1024;        // with alignment slack
+    // kind::f16: D = F32 (bits 4-5 = 1), A = B = BF16 (bits 7-9 and 10-12 = 1), K-major, N = BN, M = 128.
+    static constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t(BN) >> 3) << 17) |
+                                       ((uint32_t(kBM) >> 4) << 24);
 };
-using Deep = Shape<512, 4, 2>;       // 97 KB
-using Wide = Shape<256, 2, 4>;       // 49 KB
-constexpr int kF32Row = kBN + 4;                   // epilogue rows in shared memory: FP32 values,
-constexpr int kBf16Row = kBN + 8;                  // BF16 values (16-byte accesses of 8 rows hit all banks)
+using Small = Shape<32, 256, 3, 3>;      // 61 KB
+using Wide = Shape<64, 256, 2, 4>;       // 49 KB
+using Deep = Shape<64, 512, 4, 2>;       // 97 KB
+constexpr int kLongK = 512;
 constexpr int kMaxGroup = 4;                       // products per launch
-constexpr uint32_t kTmemCols = 64;
-// kind::f16: D = F32 (bits 4-5 = 1), A = B = BF16 (bits 7-9 and 10-12 = 1), K-major, N = 64, M = 128.
-constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t(kBN) >> 3) << 17) |
-                            ((uint32_t(kBM) >> 4) << 24);
 
 constexpr float kGeluC = 0.7978845608028654f;   // sqrt(2 / pi)
 constexpr float kGeluA = 0.044715f;
@@ -110,8 +112,12 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
 
 template <int EPI, typename Sh>
 __global__ void __launch_bounds__(Sh::kThreads, Sh::kPerSm) gemm_kernel(const __grid_constant__ GemmGroup G, int *status) {
-    constexpr int kThreads = Sh::kThreads, kStages = Sh::kStages;
+    constexpr int kThreads = Sh::kThreads, kStages = Sh::kStages, kBN = Sh::kBN;
+    constexpr uint32_t kStage = Sh::kStage, kTmemCols = kBN;
     constexpr int kCols = kBM * kBN / kThreads;       // columns of a thread in the epilogue
+    constexpr int kF32Row = kBN + 4;                  // epilogue rows in shared memory: FP32 values,
+    constexpr int kBf16Row = kBN + 8;                 // BF16 values (16-byte accesses of 8 rows hit all banks)
+    constexpr int kF4 = kBN / 4, kH8 = kBN / 8;       // 16-byte pieces of such a row
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t full[kStages], empty[kStages], done;
     __shared__ uint32_t tmem_base_s;
@@ -184,7 +190,7 @@ __global__ void __launch_bounds__(Sh::kThreads, Sh::kPerSm) gemm_kernel(const __
                 asm volatile(
                     "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
                     "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
-                    "l"(da + uint64_t(2 * ks)), "l"(db + uint64_t(2 * ks)), "r"(kIdesc), "r"(acc));
+                    "l"(da + uint64_t(2 * ks)), "l"(db + uint64_t(2 * ks)), "r"(Sh::kIdesc), "r"(acc));
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                 tcg::smem_u32(&empty[st])));
@@ -193,6 +199,19 @@ __global__ void __launch_bounds__(Sh::kThreads, Sh::kPerSm) gemm_kernel(const __
             tcg::smem_u32(&done)));
     }
     __syncwarp();
+    // the backward pass's pre-activations arrive while the products run (where registers hold them)
+    constexpr int kPre = kBM * kF4 / kThreads;
+    constexpr bool early = EPI == DM_MLP_EPI_GELU_BWD && kPre <= 4;
+    auto load_pre = [&](int q) {
+        const int i = tid + q * kThreads;
+        return *reinterpret_cast<const float4 *>(g.pre + z * g.pre_ms + int64_t(m0 + i / kF4) * g.ld_pre + n0 +
+                                                 4 * (i % kF4));
+    };
+    float4 pre[early ? kPre : 1];
+    if constexpr (early) {
+#pragma unroll
+        for (int q = 0; q < kPre; ++q) pre[q] = load_pre(q);
+    }
     wait_for(done, 0);
     if (tid == 0 && *static_cast<volatile int *>(&abort_s))   // loads in flight are drained before the CTA ends
         for (int i = issued > kStages ? issued - kStages : 0; i < issued; ++i)
@@ -225,9 +244,9 @@ __global__ void __launch_bounds__(Sh::kThreads, Sh::kPerSm) gemm_kernel(const __
                 __syncthreads();
                 float *o = g.out_f32 + z * g.f32_ms + int64_t(m0) * g.ld_f32 + n0;
 #pragma unroll
-                for (int i = tid; i < kBM * 16; i += kThreads)
-                    *reinterpret_cast<float4 *>(o + int64_t(i >> 4) * g.ld_f32 + 4 * (i & 15)) =
-                        *reinterpret_cast<const float4 *>(st + (i >> 4) * kF32Row + 4 * (i & 15));
+                for (int i = tid; i < kBM * kF4; i += kThreads)
+                    *reinterpret_cast<float4 *>(o + int64_t(i / kF4) * g.ld_f32 + 4 * (i % kF4)) =
+                        *reinterpret_cast<const float4 *>(st + (i / kF4) * kF32Row + 4 * (i % kF4));
             }
         }
         if constexpr (EPI == DM_MLP_EPI_GELU_FWD) {
@@ -235,11 +254,11 @@ __global__ void __launch_bounds__(Sh::kThreads, Sh::kPerSm) gemm_kernel(const __
             for (int j = 0; j < kCols; ++j) v[j] = gelu(v[j]);
         }
         if constexpr (EPI == DM_MLP_EPI_GELU_BWD) {
-            const float *pre = g.pre + z * g.pre_ms + int64_t(m0) * g.ld_pre + n0;
 #pragma unroll
-            for (int i = tid; i < kBM * 16; i += kThreads)
-                *reinterpret_cast<float4 *>(st + (i >> 4) * kF32Row + 4 * (i & 15)) =
-                    *reinterpret_cast<const float4 *>(pre + int64_t(i >> 4) * g.ld_pre + 4 * (i & 15));
+            for (int q = 0; q < kPre; ++q) {
+                const int i = tid + q * kThreads;
+                *reinterpret_cast<float4 *>(st + (i / kF4) * kF32Row + 4 * (i % kF4)) = early ? pre[early ? q : 0] : load_pre(q);
+            }
             __syncthreads();
 #pragma unroll
             for (int j = 0; j < kCols; j += 4) {
@@ -264,9 +283,9 @@ __global__ void __launch_bounds__(Sh::kThreads, Sh::kPerSm) gemm_kernel(const __
             if (g.out_bf16) {
                 uint16_t *o = g.out_bf16 + z * g.bf16_ms + int64_t(m0) * g.ld_bf16 + n0;
 #pragma unroll
-                for (int i = tid; i < kBM * 8; i += kThreads)
-                    *reinterpret_cast<uint4 *>(o + int64_t(i >> 3) * g.ld_bf16 + 8 * (i & 7)) =
-                        *reinterpret_cast<const uint4 *>(sb + (i >> 3) * kBf16Row + 8 * (i & 7));
+                for (int i = tid; i < kBM * kH8; i += kThreads)
+                    *reinterpret_cast<uint4 *>(o + int64_t(i / kH8) * g.ld_bf16 + 8 * (i % kH8)) =
+                        *reinterpret_cast<const uint4 *>(sb + (i / kH8) * kBf16Row + 8 * (i % kH8));
             }
             if (g.out_t) {       // column j of the tile: 256 contiguous bytes of 128 rows
                 uint16_t *o = g.out_t + z * g.t_ms + int64_t(n0) * g.ld_t + m0;
@@ -547,7 +566,7 @@ __global__ void pack_kernel(const float *__restrict__ features, int nfeat, int64
 
 // One CTA per row: every member's deviation is reduced within the warps, the CTA meets once, and one lane
 // per member adds its warps' sums (thread 0 alone over all of them was a chain of 48 shared-memory reads).
-// 5 members x 10,233 rows x 1,024 columns, 252 MB: 139 -> 75 us.
+// 5 members x 10,233 rows x 1,024 columns, 252 MB: 139 -> 75 us, with four columns per load 49 us.
 static bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 // Four columns per load where the rows are 16-byte aligned.
@@ -660,28 +679,35 @@ static bool operand_map(CUtensorMap *map, const uint16_t *base, int K, int rows,
 
 // count products of one epilogue and member count in one launch
 template <int EPI, typename Sh>
-static int launch_shape(const GemmGroup &G, int members, int *status, cudaStream_t s) {
-    auto kernel = gemm_kernel<EPI, Sh>;
-    if (ensure_max_dynamic_smem(reinterpret_cast<const void *>(kernel), int(Sh::kSmemBytes)) != cudaSuccess)
-        return DM_ERR_CUDA;
-    return launch_early(kernel, dim3(G.first[G.count], members), dim3(Sh::kThreads), Sh::kSmemBytes, s, G, status);
-}
-
-template <int EPI>
-static int launch_gemms(const dm_mlp_gemm *g, int count, int *status, cudaStream_t s) {
+static int launch_shape(const dm_mlp_gemm *g, int count, int *status, cudaStream_t s) {
     GemmGroup G;
     G.count = count;
     G.first[0] = 0;
     for (int i = 0; i < count; ++i) {
         G.g[i] = g[i];
-        G.first[i + 1] = G.first[i] + (g[i].M / kBM) * (g[i].N / kBN);
+        G.first[i + 1] = G.first[i] + (g[i].M / kBM) * (g[i].N / Sh::kBN);
         if (!operand_map(&G.a[i], g[i].A, g[i].K, g[i].M, g[i].members, g[i].lda, g[i].a_ms, kBM) ||
-            !operand_map(&G.b[i], g[i].B, g[i].K, g[i].N, g[i].members, g[i].ldb, g[i].b_ms, kBN))
+            !operand_map(&G.b[i], g[i].B, g[i].K, g[i].N, g[i].members, g[i].ldb, g[i].b_ms, Sh::kBN))
             return DM_ERR_CUDA;
     }
-    if (int64_t(G.first[count]) * g[0].members > int64_t(Deep::kPerSm) * sm_count())
-        return launch_shape<EPI, Wide>(G, g[0].members, status, s);
-    return launch_shape<EPI, Deep>(G, g[0].members, status, s);
+    auto kernel = gemm_kernel<EPI, Sh>;
+    if (ensure_max_dynamic_smem(reinterpret_cast<const void *>(kernel), int(Sh::kSmemBytes)) != cudaSuccess)
+        return DM_ERR_CUDA;
+    return launch_early(kernel, dim3(G.first[count], g[0].members), dim3(Sh::kThreads), Sh::kSmemBytes, s, G, status);
+}
+
+template <int EPI>
+static int launch_gemms(const dm_mlp_gemm *g, int count, int *status, cudaStream_t s) {
+    int64_t tiles = 0;
+    int longest = 0;
+    for (int i = 0; i < count; ++i) {
+        tiles += int64_t(g[i].M / kBM) * (g[i].N / Wide::kBN) * g[i].members;
+        longest = g[i].K > longest ? g[i].K : longest;
+    }
+    if (tiles > 2 * sm_count()) return launch_shape<EPI, Wide>(g, count, status, s);
+    if constexpr (EPI == DM_MLP_EPI_F32 || EPI == DM_MLP_EPI_BIAS_F32)
+        if (longest > kLongK) return launch_shape<EPI, Deep>(g, count, status, s);
+    return launch_shape<EPI, Small>(g, count, status, s);
 }
 
 static bool mult8(int64_t x) { return x >= 0 && (x & 7) == 0; }
@@ -695,7 +721,7 @@ extern "C" int dm_mlp_gemm_run(const dm_mlp_gemm *g, int *status_dev, void *stre
     using namespace mlp;
     DM_CHECK_ARG(g && status_dev);
     DM_CHECK_ARG(g->M > 0 && g->N > 0 && g->K > 0 && g->members >= 1 && g->members <= 65535);
-    DM_CHECK_ARG(g->M % kBM == 0 && g->N % kBN == 0 && g->K % kBK == 0 && g->M / kBM <= 65535);
+    DM_CHECK_ARG(g->M % kBM == 0 && g->N % Wide::kBN == 0 && g->K % kBK == 0 && g->M / kBM <= 65535);
     DM_CHECK_ARG(g->A && g->B && aligned16(g->A) && aligned16(g->B));
     DM_CHECK_ARG(mult8(g->lda) && mult8(g->ldb) && g->lda >= g->K && g->ldb >= g->K && mult8(g->a_ms) &&
                  mult8(g->b_ms));

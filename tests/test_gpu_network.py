@@ -191,3 +191,52 @@ def test_ensemble_statistics(nout, members):
     assert np.abs(mean.cpu().numpy() - mu).max() <= 16 * U
     assert np.abs(spread.cpu().numpy() - 0.5 * np.abs(p - mu).sum(axis=2).mean(axis=0)).max() <= tol
     assert np.abs(tv.cpu().numpy() - 0.5 * np.abs(mu - ref).sum(axis=1)).max() <= tol
+
+
+@pytest.mark.parametrize('M,N_,K,members', [(128, 64, 64, 1), (128, 64, 576, 1), (256, 192, 512, 3), (256, 192, 640, 3),
+                                            (2560, 1024, 64, 1), (640, 1024, 192, 4)])
+@pytest.mark.parametrize('epi', ['f32', 'fwd', 'bwd'])
+def test_gemm_launch_shapes(M, N_, K, members, epi):
+    """The narrow, the deep and the wide tiles: few and many of them, short and long K, each epilogue."""
+    torch = _torch()
+    rng = np.random.default_rng(M + K)
+    A = MO.bf16(rng.normal(size=(members, M, K)).astype(np.float32))
+    B = MO.bf16((rng.normal(size=(members, N_, K)) / np.sqrt(K)).astype(np.float32))
+    pre = rng.normal(size=(members, M, N_)).astype(np.float32)
+    bias = rng.normal(size=(members, N_)).astype(np.float32)
+    a, b, pt, bt = _bf16(A), _bf16(B), torch.from_numpy(pre).cuda(), torch.from_numpy(bias).cuda()
+    f32 = torch.full((members, M, N_), 7.0, device='cuda')
+    bf = torch.zeros((members, M, N_), dtype=torch.int16, device='cuda')
+    t = torch.zeros((members, N_, M), dtype=torch.int16, device='cuda')
+    status = torch.zeros(1, dtype=torch.int32, device='cuda')
+    g = N.DmMlpGemm()
+    g.epi = {'f32': N.DM_MLP_EPI_F32, 'fwd': N.DM_MLP_EPI_GELU_FWD, 'bwd': N.DM_MLP_EPI_GELU_BWD}[epi]
+    g.M, g.N, g.K, g.members = M, N_, K, members
+    g.A, g.lda, g.a_ms, g.B, g.ldb, g.b_ms = a.data_ptr(), K, M * K, b.data_ptr(), K, N_ * K
+    if epi != 'bwd':
+        g.out_f32, g.ld_f32, g.f32_ms = f32.data_ptr(), N_, M * N_
+    if epi != 'f32':
+        g.bias, g.bias_ms = bt.data_ptr(), N_
+        g.pre, g.ld_pre, g.pre_ms = pt.data_ptr(), N_, M * N_
+        g.out_bf16, g.ld_bf16, g.bf16_ms = bf.data_ptr(), N_, M * N_
+        g.out_t, g.ld_t, g.t_ms = t.data_ptr(), M, M * N_
+    N.call('dm_mlp_gemm_run', ctypes.byref(g), ctypes.c_void_p(status.data_ptr()), None)
+    assert int(status.item()) == 0
+    A64, Bt = A.astype(np.float64), np.swapaxes(B.astype(np.float64), 1, 2)
+    want = A64 @ Bt
+    tol = (K + 2) * U * (np.abs(A64) @ np.abs(Bt) + 4)
+    if epi == 'fwd':
+        want = want + bias[:, None, :]
+    if epi != 'bwd':
+        assert np.all(np.abs(f32.cpu().numpy() - want) <= tol)
+    if epi != 'f32':
+        # GELU (slope below 1.13) and its derivative (below 1.13) in FP32, rounded to BF16
+        x = want if epi == 'fwd' else pre.astype(np.float64)
+        c, k = 0.7978845608028654, 0.044715
+        y = c * (x + k * x ** 3)
+        gate = 0.5 * (1 + np.tanh(y))
+        d = gate + 0.5 * x * (1 - np.tanh(y) ** 2) * c * (1 + 3 * k * x * x)
+        want = x * gate if epi == 'fwd' else want * d
+        err = np.abs(_f(bf) - want)
+        assert np.all(err <= 2.0 ** -8 * np.abs(want) + 1.13 * tol + 64 * U)
+        assert np.array_equal(bf.cpu().numpy(), np.swapaxes(t.cpu().numpy(), 1, 2))
