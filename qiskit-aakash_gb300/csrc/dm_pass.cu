@@ -489,7 +489,8 @@ __global__ void __launch_bounds__(kPipeThreads, 1) pass_pipe_kernel(T *__restric
                                                                     const T *__restrict__ mats) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int64_t hi_off[64];
-    pipe_tiles<T, R>(st, p, mats, blockIdx.x, gridDim.x, reinterpret_cast<T *>(smem_raw), hi_off);
+    grid_wait();
+    pipe_tiles<T, R>(st, p, waited(mats), blockIdx.x, gridDim.x, reinterpret_cast<T *>(smem_raw), hi_off);
 }
 
 // ---------------------------------------------------------------------------
@@ -589,9 +590,7 @@ static int launch_rounds(T *st, const PassRounds &p, const T *mats, cudaStream_t
     const int64_t ntiles = int64_t(1) << (2 * p.m);
     int64_t grid = sm_count();
     if (grid > ntiles) grid = ntiles;
-    pass_pipe_kernel<T, R><<<int(grid), kPipeThreads, smem, s>>>(st, p, mats);
-    count_launch();
-    return launch_status();
+    return launch_early(pass_pipe_kernel<T, R>, dim3(unsigned(grid)), dim3(kPipeThreads), smem, s, st, p, mats);
 }
 
 template <typename T>

@@ -190,7 +190,7 @@ class DeviceState:
         self._images = None       # device round images of the group of passes in flight
         self._group = 1           # passes of the next group composed in one launch
         self.status = torch.zeros(1, dtype=torch.int32, device=self.device) if self.tensor_cores else None
-        self.kmax = min(tile_axes or DEFAULT_TILE_AXES[precision], N.DM_MAX_TILE_AXES)
+        self.kmax = min(tile_axes or self._default_tile_axes(), N.DM_MAX_TILE_AXES)
         self.low = low_axes
         self.pending = []
         self._stream_at = STREAM_OPS
@@ -200,6 +200,17 @@ class DeviceState:
         self.tape = None          # list of recorded C-ABI calls (see record())
         self.copy_stats = {}      # the last large copy-out: seconds, whether it went into a result block
         self._keep_alive = []
+
+    def _default_tile_axes(self):
+        """Resident axes of a tile: DEFAULT_TILE_AXES, one less for an FP64 state whose smaller tiles
+        still fit on the SMs at once.
+
+        FP64 passes are bound by the FP64 pipe of the SMs that have a tile, so a few qubits' work is
+        better spread than fused (20 layers, device time with 6 and 5 axes: 7 qubits 518 and 325 us,
+        8 qubits, 16 or 64 tiles, 612 and 384 us; 9 qubits, 64 or 256 tiles on 152 SMs, 718 and 856 us)."""
+        k = DEFAULT_TILE_AXES[self.precision]
+        sms = _torch().cuda.get_device_properties(self.device).multi_processor_count
+        return k - 1 if self.precision == 'double' and 4 ** (self.n - k + 1) <= sms else k
 
     # -- recording -----------------------------------------------------------
     def record(self):

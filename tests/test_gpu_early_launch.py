@@ -88,3 +88,31 @@ def test_training_back_to_back():
         ens, p, q = _train(False)
         assert torch.equal(p, params) and torch.equal(q, probs)
         assert int(ens.status.item()) == 0
+
+
+@pytest.mark.parametrize('n', [4, 6, 8, 9])
+def test_small_fp64_states_take_smaller_tiles(n):
+    """The default tile of a small FP64 state against six resident axes: the same maps, grouped otherwise.
+
+    4**n values of at most 2**-n; 12 layers of maps that do not grow them, 3 n roundings of each value
+    per layer at 16 terms: 12 * 3 * n * 16 * 2**-53 * 2**-n, doubled for the other grouping."""
+    torch = _torch()
+    rng = np.random.default_rng(n)
+    angles = rng.uniform(0, 6, (12, n, 3))
+    pairs = [rng.permutation(n) for _ in range(12)]
+    err = {'rx': [1, 0], 'ry': [1, 0], 'rz': [1, 0]}
+    states = []
+    for axes in (None, 6):
+        dev = engine.DeviceState(n, precision='double', tile_axes=axes)
+        dev.init_product([[1.0, 0.0, 0.0, 1.0]] * n, 2.0 ** -n)
+        for layer, order in zip(angles, pairs):
+            for q in range(n):
+                dev.map1(q, P.u_gate_ptm('u3', layer[q], err))
+                dev.map1(q, P.noise_ptm(0.999, 0.99, 0.998))
+            for a, b in zip(order[::2], order[1::2]):
+                dev.cx(int(a), int(b), [0.995, 0.01])
+        dev.flush()
+        states.append(dev.state.clone())
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert engine.DeviceState(n, precision='double').kmax == (5 if 4 ** (n - 5) <= sms else 6)
+    assert float((states[0] - states[1]).abs().max()) <= 2 * 12 * 3 * n * 16 * 2.0 ** -53 * 2.0 ** -n
