@@ -71,8 +71,9 @@ struct Pass {
     float up, down;                  // 2**n, 2**-n
     int64_t res_stride[kAxes];
     int64_t nonres_stride[DM_MAX_QUBITS];
-    uint32_t natrow[8], natk[6];
-    int64_t lastg[14];               // direct: global element offsets of the last round's row bits 0-7, K bits 0-5
+    alignas(16) uint32_t natrow[8];
+    alignas(16) uint32_t natk[8];
+    alignas(16) int64_t lastg[14];               // direct: global element offsets of the last round's row bits 0-7, K bits 0-5
     Round rounds[DM_MAX_ROUNDS];
 };
 
@@ -195,24 +196,31 @@ __device__ __forceinline__ bool tc_pass_tiles(float *__restrict__ st, const Pass
             constexpr int kItems = kGroups * 8 / kThreads;   // 8
             const float *nat = reinterpret_cast<const float *>(AH);
             const float up = p.up;      // 2**n: the tile in units of 2**-n
+            struct alignas(16) { uint32_t row[8], k[8]; } nt;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint4 w = reinterpret_cast<const uint4 *>(i < 2 ? p.natrow : p.natk)[i & 1];
+                uint32_t *o = i < 2 ? nt.row + 4 * i : nt.k + 4 * (i - 2);
+                o[0] = w.x, o[1] = w.y, o[2] = w.z, o[3] = w.w;
+            }
             float x[kItems][8];
 #pragma unroll
             for (int q = 0; q < kItems; ++q) {
                 const int i = tid + kThreads * q;
                 const int crow = ((i >> 6) << 3) | (i & 7), c = (i >> 3) & 7;
                 // chunk c holds K = 8c .. 8c + 7: K bits 3-5 come from c, bits 0-2 from the element
-                const uint32_t nb = xor_bits<8>(uint32_t(crow), p.natrow) ^ ((c & 1) ? p.natk[3] : 0u) ^
-                                    ((c & 2) ? p.natk[4] : 0u) ^ ((c & 4) ? p.natk[5] : 0u);
+                const uint32_t nb = xor_bits<8>(uint32_t(crow), nt.row) ^ ((c & 1) ? nt.k[3] : 0u) ^
+                                    ((c & 2) ? nt.k[4] : 0u) ^ ((c & 4) ? nt.k[5] : 0u);
                 if (p.vec0 == 0) {   // digit 0 is local axis 0: four adjacent natural elements
                     const float4 a4 = *reinterpret_cast<const float4 *>(nat + nb);
-                    const float4 b4 = *reinterpret_cast<const float4 *>(nat + (nb ^ p.natk[2]));
+                    const float4 b4 = *reinterpret_cast<const float4 *>(nat + (nb ^ nt.k[2]));
                     x[q][0] = a4.x; x[q][1] = a4.y; x[q][2] = a4.z; x[q][3] = a4.w;
                     x[q][4] = b4.x; x[q][5] = b4.y; x[q][6] = b4.z; x[q][7] = b4.w;
                 } else {
 #pragma unroll
                     for (int e = 0; e < 8; ++e)
-                        x[q][e] = nat[nb ^ ((e & 1) ? p.natk[0] : 0u) ^ ((e & 2) ? p.natk[1] : 0u) ^
-                                      ((e & 4) ? p.natk[2] : 0u)];
+                        x[q][e] = nat[nb ^ ((e & 1) ? nt.k[0] : 0u) ^ ((e & 2) ? nt.k[1] : 0u) ^
+                                      ((e & 4) ? nt.k[2] : 0u)];
                 }
             }
             __syncthreads();
@@ -283,7 +291,7 @@ __device__ __forceinline__ bool tc_pass_tiles(float *__restrict__ st, const Pass
             load_u(r + 1 < p.nrounds ? r + 1 : 0);
             // ---- epilogue: D -> next operand (h / l), or the natural tile after the last round ----
             // the thread holds row tid % 128 of M block tid / 128 (TMEM columns 0-127 / 128-255)
-            const Round &R = p.rounds[r];
+            const Round R = p.rounds[r];
             uint32_t tk[3][4];
             digit_tables(R.kc, tk);
             const bool last = r + 1 == p.nrounds;
@@ -392,6 +400,7 @@ constexpr int64_t kScratchHalves = int64_t(DM_MAX_ROUNDS) * kUHalves;   // a pas
 // Kernel parameters of one batched pass, each field by a thread of its own (the pass table is in
 // global memory: one thread reading it field by field takes microseconds).
 static_assert(sizeof(Round) == sizeof(dm_tc_round), "a round's table is copied as words");
+static_assert(offsetof(dm_tc_round, rowc) == 8 && offsetof(dm_tc_round, kc) == 40, "its order");
 __device__ void batch_tc_setup(Pass &ps, const dm_batch_tc_pass &bp, int n) {
     const int tid = threadIdx.x, lane = tid & 31;
     const int nr = bp.ops.nrounds;
@@ -428,7 +437,9 @@ __device__ void batch_tc_setup(Pass &ps, const dm_batch_tc_pass &bp, int n) {
     uint32_t *out = reinterpret_cast<uint32_t *>(ps.rounds);
     constexpr int kWords = sizeof(Round) / 4;
     for (int i = tid; i < nr * kWords; i += kThreads)
-        out[i] = i % kWords == 1 ? uint32_t(i / kWords * kUHalves) : in[i];   // word 1: umoff
+        out[i] = i % kWords == kWords - 1 ? uint32_t(i / kWords * kUHalves)               // umoff
+               : i % kWords == kWords - 2 ? uint32_t(int32_t(in[i - kWords + 2]) >> 24)   // vec, the fourth byte
+                                          : in[i + 2];
 }
 
 // Round r's matrix U (64 x 64 in its K-digit order), composed in FP64 from the
@@ -967,7 +978,7 @@ __global__ void __launch_bounds__(32 * kComposeWarps)
 // and spills in the tile loop (10 % of a sweep); with the constants of a lone CTA it has enough.
 struct BatchShared {
     Pass ps;
-    int64_t hi_off[kTile / 4 / kThreads];
+    alignas(16) int64_t hi_off[kTile / 4 / kThreads];
     uint64_t mbar;
     uint32_t tmem, phase;
     int pending, abort_s;
@@ -1235,7 +1246,6 @@ extern "C" int dm_apply_pass_tc(void *state_dev, int n, const dm_tc_pass *pass, 
         tc::Round &o = p.rounds[r];
         for (int i = 0; i < 3; ++i) {
             if (in.digits[i] < 0 || in.digits[i] >= tc::kAxes) return DM_ERR_PROGRAM;
-            o.digits[i] = in.digits[i];
         }
         o.vec = in.vec;
         const bool direct_round = p.direct && r + 1 == nr;

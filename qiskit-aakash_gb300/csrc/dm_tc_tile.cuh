@@ -44,12 +44,13 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) { return tcg::smem
 constexpr uint32_t kIdesc128 = (1u << 4) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
 constexpr uint32_t kIdesc64 = (1u << 4) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
 
-struct Round {
-    int8_t digits[3];
-    int8_t vec;
-    int32_t umoff;
+// A round's tables as the kernels read them, in 16-byte words: the batched kernels have them in shared
+// memory, where each word that a warp reads takes a cycle of its bandwidth.
+struct alignas(16) Round {
     uint32_t rowc[8];
     uint32_t kc[6];
+    int32_t vec;
+    int32_t umoff;
 };
 
 // XOR-combination of the offsets of the set bits of x (nbits of them).

@@ -530,7 +530,6 @@ extern "C" int dm_apply_pass_tma(void *state_dev, int n, const dm_tc_pass *pass,
         tc::Round &o = p.rounds[r];
         for (int i = 0; i < 3; ++i) {
             if (in.digits[i] < 0 || in.digits[i] >= tc::kAxes) return DM_ERR_PROGRAM;
-            o.digits[i] = in.digits[i];
         }
         o.vec = in.vec;
         const bool ok = r + 1 == nr ? linear_tables(in.rowc, in.kc, -1) : operand_tables(in.rowc, in.kc, in.vec);
