@@ -31,7 +31,7 @@
 //
 // Two CTAs of 256 threads share an SM, so one CTA's tile load, barriers
 // and MMA waits overlap the other's work.  Shared memory per CTA (dynamic,
-// 88 KB): AH / AL 32 KB each (round operand h / l, K-major core-matrix FP16
+// 88 KB): AH / AL 32 KB each (round operand h / l, swizzled K-major FP16
 // layout, 256 rows x 64; together they also hold the natural FP32 tile that
 // cp.async streams in and the last round writes out), B 24 KB (2**11 Uh and
 // Ul stacked as one 128-row operand, then Uh).  The h operand is read once
@@ -93,6 +93,13 @@ __device__ __forceinline__ int64_t tile_offset(const Pass &p, int e) {
     for (int r = p.low; r < kAxes; ++r) off += int64_t((e >> (2 * r)) & 3) * p.res_stride[r];
     return off;
 }
+
+// The dynamic shared memory from its first 1024-byte boundary (the swizzle's).
+__device__ __forceinline__ unsigned char *aligned_smem() {
+    extern __shared__ __align__(1024) unsigned char raw[];
+    return raw + ((1024 - (smem_u32(raw) & 1023)) & 1023);
+}
+constexpr uint32_t kAlignSlack = 1024;
 
 // Per-CTA tensor-core state shared by the single-state and the batched kernels.
 struct TcCta {
@@ -231,7 +238,7 @@ __device__ __forceinline__ bool tc_pass_tiles(float *__restrict__ st, const Pass
                 uint32_t hw[4], lw[4];
 #pragma unroll
                 for (int e = 0; e < 8; e += 2) split2(x[q][e] * up, x[q][e + 1] * up, hw[e >> 1], lw[e >> 1]);
-                const uint32_t o = row_off(crow) + uint32_t(c) * kLBO;
+                const uint32_t o = operand_chunk(crow, c);
                 *reinterpret_cast<uint4 *>(AH + o) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
                 *reinterpret_cast<uint4 *>(AL + o) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
             }
@@ -259,7 +266,7 @@ __device__ __forceinline__ bool tc_pass_tiles(float *__restrict__ st, const Pass
                         const uint32_t idesc = term == 0 ? kIdesc128 : kIdesc64;
 #pragma unroll
                         for (int ks = 0; ks < 4; ++ks) {      // K = 16 per MMA: two core matrices
-                            const uint64_t da = smem_desc(a + ks * 2 * kLBO);
+                            const uint64_t da = operand_desc(a + ks * kOperandStep);
                             const uint64_t db = smem_desc(b + ks * 2 * kLBO);
                             const uint32_t acc = (term | ks) ? 1u : 0u;
                             asm volatile(
@@ -379,7 +386,7 @@ __device__ __forceinline__ bool tc_pass_tiles(float *__restrict__ st, const Pass
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
     pass_tc_kernel(float *__restrict__ st, const __grid_constant__ Pass p, const uint16_t *__restrict__ umats,
                    int *status) {
-    extern __shared__ __align__(1024) unsigned char smem[];
+    unsigned char *smem = aligned_smem();
     __shared__ __align__(8) uint64_t mbar;
     __shared__ uint32_t tmem_base_s;
     __shared__ int64_t hi_off[kTile / 4 / kThreads];
@@ -439,7 +446,7 @@ __device__ void batch_tc_setup(Pass &ps, const dm_batch_tc_pass &bp, int n) {
     for (int i = tid; i < nr * kWords; i += kThreads)
         out[i] = i % kWords == kWords - 1 ? uint32_t(i / kWords * kUHalves)               // umoff
                : i % kWords == kWords - 2 ? uint32_t(int32_t(in[i - kWords + 2]) >> 24)   // vec, the fourth byte
-                                          : in[i + 2];
+               : i / kWords < nr - 1      ? operand_offset(in[i + 2]) : in[i + 2];
 }
 
 // Round r's matrix U (64 x 64 in its K-digit order), composed in FP64 from the
@@ -983,10 +990,10 @@ struct BatchShared {
     uint32_t tmem, phase;
     int pending, abort_s;
 };
-constexpr uint32_t kBatchSmemBytes = kSmemBytes + (sizeof(BatchShared) + 15) / 16 * 16;
+constexpr uint32_t kBatchSmemBytes = kSmemBytes + (sizeof(BatchShared) + 15) / 16 * 16 + kAlignSlack;
 
 __device__ __forceinline__ bool batch_tiles_inline(float *st, const uint16_t *umats, int t0, int dt, int *status) {
-    extern __shared__ __align__(1024) unsigned char smem[];
+    unsigned char *smem = aligned_smem();
     BatchShared &b = *reinterpret_cast<BatchShared *>(smem + kSmemBytes);
     TcCta c{smem, smem + kABytes, smem + 2 * kABytes, &b.mbar, b.hi_off, &b.abort_s, b.tmem, b.phase, b.pending != 0};
     const bool ok = tc_pass_tiles(st, b.ps, umats, t0, dt, c, status);
@@ -1033,7 +1040,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
     batch_tc_kernel(float *__restrict__ states, double *__restrict__ probs, const double *__restrict__ mats,
                     const dm_batch_instance *__restrict__ insts, int ninst, const dm_batch_tc_pass *__restrict__ passes,
                     int *counter, unsigned char *__restrict__ scratch, int ctas, int G, int *status) {
-    extern __shared__ __align__(1024) unsigned char smem[];
+    unsigned char *smem = aligned_smem();
     __shared__ int inst_s, ok_s;
     __shared__ Group g;
     __shared__ dm_batch_instance I;
@@ -1087,7 +1094,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm)
                           const dm_batch_tc_pass *__restrict__ passes, const double *__restrict__ params,
                           int params_stride, int ninst, int *counter, unsigned char *__restrict__ scratch, int ctas,
                           int G, int *status) {
-    extern __shared__ __align__(1024) unsigned char smem[];
+    unsigned char *smem = aligned_smem();
     __shared__ int inst_s, ok_s;
     __shared__ double prm[DM_PARAMS_MIN_STRIDE];
     __shared__ Group g;
@@ -1251,20 +1258,21 @@ extern "C" int dm_apply_pass_tc(void *state_dev, int n, const dm_tc_pass *pass, 
         const bool direct_round = p.direct && r + 1 == nr;
         if (!(direct_round ? direct_tables(in.rowc, in.kc) : valid_tables(in.rowc, in.kc, in.vec, r + 1 == nr)))
             return DM_ERR_PROGRAM;
-        for (int i = 0; i < 8; ++i) o.rowc[i] = in.rowc[i];
-        for (int i = 0; i < 6; ++i) o.kc[i] = in.kc[i];
+        const bool operand = r + 1 < nr;
+        for (int i = 0; i < 8; ++i) o.rowc[i] = operand ? tc::operand_offset(in.rowc[i]) : in.rowc[i];
+        for (int i = 0; i < 6; ++i) o.kc[i] = operand ? tc::operand_offset(in.kc[i]) : in.kc[i];
         if (direct_round) tc::direct_offsets(p, in.rowc, in.kc);
         if (in.umoff < 0 || (in.umoff & 7) || size_t(in.umoff) + tc::kUHalves > umats_count) return DM_ERR_PROGRAM;
         o.umoff = in.umoff;
     }
-    if (ensure_max_dynamic_smem(reinterpret_cast<const void *>(tc::pass_tc_kernel), int(tc::kSmemBytes)) !=
-        cudaSuccess)
+    constexpr uint32_t smem = tc::kSmemBytes + tc::kAlignSlack;
+    if (ensure_max_dynamic_smem(reinterpret_cast<const void *>(tc::pass_tc_kernel), int(smem)) != cudaSuccess)
         return DM_ERR_CUDA;
     const int64_t ntiles = int64_t(1) << (2 * p.m);
     // 88 KB of shared memory, <= 128 registers per thread and 256 TMEM columns per CTA: two CTAs per SM
     int64_t grid = int64_t(sm_count()) * tc::kCtasPerSm;
     if (grid > ntiles) grid = ntiles;
-    return launch_early(tc::pass_tc_kernel, dim3(unsigned(grid)), dim3(tc::kThreads), tc::kSmemBytes, as_stream(stream),
+    return launch_early(tc::pass_tc_kernel, dim3(unsigned(grid)), dim3(tc::kThreads), smem, as_stream(stream),
                         static_cast<float *>(state_dev), p, umats_dev, status_dev);
 }
 

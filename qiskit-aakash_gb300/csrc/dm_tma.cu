@@ -236,8 +236,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     uint64_t adesc_h[2], adesc_l[2];
 #pragma unroll
     for (int mb = 0; mb < 2; ++mb) {
-        adesc_h[mb] = smem_desc(smem_u32(AH) + mb * (kABytes / 2));
-        adesc_l[mb] = smem_desc(smem_u32(AL) + mb * (kABytes / 2));
+        adesc_h[mb] = operand_desc(smem_u32(AH) + mb * (kABytes / 2));
+        adesc_l[mb] = operand_desc(smem_u32(AL) + mb * (kABytes / 2));
     }
 
     // epilogue geometry: the thread holds row ttid of the 256-row operand, i.e. row ttid % 128 of
@@ -267,15 +267,14 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
             for (int j = 0; j < 64; ++j) x[j] = nat[nb ^ tn0[0][j & 3] ^ tn0[1][(j >> 2) & 3] ^ tn0[2][j >> 4]];
             team_sync(team);
-            const uint32_t o = row_off(ttid);
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
                 uint32_t hw[4], lw[4];
 #pragma unroll
                 for (int e = 0; e < 8; e += 2)
                     split2(x[8 * c + e] * up, x[8 * c + e + 1] * up, hw[e >> 1], lw[e >> 1]);
-                *reinterpret_cast<uint4 *>(AH + o + uint32_t(c) * kLBO) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
-                *reinterpret_cast<uint4 *>(AL + o + uint32_t(c) * kLBO) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+                *reinterpret_cast<uint4 *>(AH + operand_chunk(ttid, c)) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+                *reinterpret_cast<uint4 *>(AL + operand_chunk(ttid, c)) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
             }
         }
         bool alive = true;
@@ -315,9 +314,9 @@ __global__ void __launch_bounds__(kThreads, 1)
                         const uint32_t idesc = term == 0 ? kIdesc128 : kIdesc64;
 #pragma unroll
                         for (int ks = 0; ks < 4; ++ks) {
-                            // a K step of 16 values is two core matrices (256 bytes): +16 in the
-                            // descriptor's start-address field (address >> 4, bits 0-13)
-                            const uint64_t da = a + uint64_t(ks * (2 * kLBO >> 4));
+                            // a K step of 16 values: 32 bytes of the operand's rows, two core matrices
+                            // (256 bytes) of U, in the descriptors' start-address field (address >> 4, bits 0-13)
+                            const uint64_t da = a + uint64_t(ks * (kOperandStep >> 4));
                             const uint64_t db = ub + uint64_t(ks * (2 * kLBO >> 4));
                             const uint32_t acc = (term | ks) ? 1u : 0u;
                             asm volatile(
@@ -547,8 +546,8 @@ extern "C" int dm_apply_pass_tma(void *state_dev, int n, const dm_tc_pass *pass,
             // 4 elements, so each group of four lands 16-byte aligned
             p.last_vec = p.lastg[8] == 1 && p.lastg[9] == 2;
         }
-        for (int i = 0; i < 8; ++i) o.rowc[i] = in.rowc[i];
-        for (int i = 0; i < 6; ++i) o.kc[i] = in.kc[i];
+        for (int i = 0; i < 8; ++i) o.rowc[i] = tc::operand_offset(in.rowc[i]);   // the last round reads lastg
+        for (int i = 0; i < 6; ++i) o.kc[i] = tc::operand_offset(in.kc[i]);
         if (in.umoff < 0 || (in.umoff & 7) || size_t(in.umoff) + tma::kUHalves > umats_count) return DM_ERR_PROGRAM;
         o.umoff = in.umoff;
         p.uoff[r] = in.umoff;

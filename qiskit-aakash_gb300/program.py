@@ -536,6 +536,13 @@ class TcLayout:
     def byte_of_bit(self, tb):
         return self._byte[tb]
 
+    def bank_of_bit(self, tb):
+        """The byte's place in the kernels' operand, whose 128-byte rows are swizzled (operand_offset in
+        csrc/dm_tc_tile.cuh): what a store's bank conflicts depend on."""
+        o = self._byte[tb]
+        row, chunk = (o >> 4) & 7, (o >> 7) & 7
+        return (o & ~0x3F0) | (row << 7) | ((chunk ^ row) << 4)
+
 
 @functools.lru_cache(maxsize=None)
 def _store_wavefronts(lane_offs, vec_bytes):
@@ -616,7 +623,7 @@ def _best_next_cost_cached(rowbits, digit_set, next_axes):
     for digits in itertools.permutations(next_axes):
         nxt = TcLayout(list(digits), rows)
         vec = 8 if nxt.digits[0] in digit_set else None
-        lane_offs = tuple(nxt.byte_of_bit(tb) for tb in lane_bits)
+        lane_offs = tuple(nxt.bank_of_bit(tb) for tb in lane_bits)
         if vec:
             c = 16 * _store_wavefronts(lane_offs, vec) + 4
         else:
@@ -642,7 +649,7 @@ def _choose_layouts_cached(rounds_axes, nat='xor', direct=False):
             for d, rows in _tma_last_candidates(axes, prev):
                 cand = TcLayout(list(d), rows)
                 vec = 8 if _vec_digit(prev, cand.digits[0]) >= 0 else None
-                cost = _transition_cost(prev, cand.byte_of_bit, vec)
+                cost = _transition_cost(prev, cand.bank_of_bit, vec)
                 if best is None or cost < best[0]:
                     best = (cost, cand)
             layouts.append(best[1])
@@ -677,7 +684,7 @@ def _choose_layouts_cached(rounds_axes, nat='xor', direct=False):
                     cand = TcLayout(list(digits), _fill_rows(list(tri) + ([f] if f is not None else []),
                                                              lanes, keep, nonround))
                     vec = 8 if _vec_digit(prev, cand.digits[0]) >= 0 else None
-                    cost = _transition_cost(prev, cand.byte_of_bit, vec)
+                    cost = _transition_cost(prev, cand.bank_of_bit, vec)
                     cost += _natural_cost(cand, nat) if ri == nlast else _best_next_cost(cand, nxt_axes)
                     if best is None or cost < best[0]:
                         best = (cost, cand)
@@ -755,14 +762,14 @@ def _choose_layouts_tma_cached(rounds_axes):
             cost = _tma_conversion_cost(cand) if ri == 0 else 0
             if prev is not None:
                 vec = 8 if _vec_digit(prev, cand.digits[0]) >= 0 else None
-                cost += _transition_cost(prev, cand.byte_of_bit, vec)
+                cost += _transition_cost(prev, cand.bank_of_bit, vec)
             if ri < nlast:
                 if ri + 1 == nlast:      # the last round's rows are fixed: its exact incoming cost
                     # (it depends only on the candidate's lane bits and its set of axes)
                     key = (tuple(cand.rowbits[:5]), frozenset(cand.digits), tuple(sorted(nxt_axes)))
                     if key not in into_last:
                         into_last[key] = min(
-                            _transition_cost(cand, nxt.byte_of_bit, 8 if _vec_digit(cand, nxt.digits[0]) >= 0
+                            _transition_cost(cand, nxt.bank_of_bit, 8 if _vec_digit(cand, nxt.digits[0]) >= 0
                                              else None) for nxt in fixed_next(nxt_axes))
                     cost += into_last[key]
                 else:
@@ -835,47 +842,6 @@ def _choose_layouts(rounds_axes, nat='xor', direct=False):
 def _vec_digit(src, dst_first_axis):
     """Digit of ``src`` holding the destination's 4-vector axis, or -1."""
     return src.digits.index(dst_first_axis) if dst_first_axis in src.digits else -1
-
-
-def epilogue_wavefronts(src, dst, natural=False):
-    """Shared-memory store wavefronts of one warp writing src's rows 0..31 into dst's layout."""
-    lanes = np.arange(32)
-
-    def addr_bytes(row, k):
-        e = 0
-        for i, tb in enumerate(src.rowbits):
-            if (row >> i) & 1:
-                e |= 1 << tb
-        for i, tb in enumerate(src.kbits):
-            if (k >> i) & 1:
-                e |= 1 << tb
-        if natural:
-            return 4 * nat_swz(e)
-        return sum(dst.byte_of_bit(tb) for tb in range(2 * TC_AXES) if (e >> tb) & 1)
-
-    vec_axis = 0 if natural else dst.digits[0]
-    d = _vec_digit(src, vec_axis)
-    vec_bytes = 16 if natural else 8     # four FP32 natural values / four FP16 operand values
-    phase = 8 if natural else 16          # threads per shared-memory wavefront of that width
-    total = 0
-    if d >= 0:
-        others = [j for j in range(64) if (j >> (2 * d)) & 3 == 0]
-        for j in others:
-            addrs = [addr_bytes(int(r), j) for r in lanes]
-            for ph in range(32 // phase):
-                cnt = {}
-                for a in addrs[phase * ph:phase * ph + phase]:
-                    for w in range(a // 4, (a + vec_bytes) // 4):
-                        cnt.setdefault(w % 32, set()).add(w)
-                total += max(len(v) for v in cnt.values())
-    else:
-        for j in range(64):
-            words = [addr_bytes(int(r), j) // 4 for r in lanes]
-            cnt = {}
-            for w in words:
-                cnt.setdefault(w % 32, set()).add(w)
-            total += max(len(v) for v in cnt.values())
-    return total
 
 
 def plan_tc_rounds(p, n, nat='xor'):
