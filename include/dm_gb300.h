@@ -565,8 +565,9 @@ int dm_mlp_forward(const dm_mlp_net *net, int rows, int train, void *stream);
 int dm_mlp_backward(const dm_mlp_net *net, int rows, void *stream);
 /* Forward pass, softmax with the mean KL loss against t, backward pass. */
 int dm_mlp_loss_and_grads(const dm_mlp_net *net, int rows, void *stream);
-/* One training step on the minibatch index [members][batch]: dm_mlp_gather,
- * dm_mlp_loss_and_grads and dm_mlp_adam (step >= 1). */
+/* One training step on the minibatch index [members][batch]: the features of
+ * dm_mlp_gather, dm_mlp_loss_and_grads with the targets read from the data set
+ * (t is not written) and dm_mlp_adam (step >= 1). */
 int dm_mlp_train_step(const dm_mlp_net *net, const float *features, int nfeat, const float *targets,
                       int64_t samples, const int32_t *index, float lr, float beta1, float beta2, float eps,
                       int step, void *stream);

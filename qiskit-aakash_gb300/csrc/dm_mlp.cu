@@ -340,8 +340,8 @@ __device__ __forceinline__ float slice_sum(const float (&part)[kSoftSlices]) {
 // Per: nout / 256 where the row is held in registers, 0 otherwise.
 template <int Per>
 __global__ void __launch_bounds__(32 * kSoftRows, 2)
-    softmax_kernel(const float *__restrict__ logits, const float *__restrict__ targets, int rows, int nout,
-                   int64_t row_ms, int64_t out_ms, int64_t ld_t, float grad_scale, float *__restrict__ probs,
+    softmax_kernel(const float *__restrict__ logits, const float *__restrict__ targets,
+                   const int32_t *__restrict__ index, int64_t samples, int rows, int nout, int64_t row_ms, int64_t out_ms, int64_t ld_t, float grad_scale, float *__restrict__ probs,
                    uint16_t *__restrict__ dz, uint16_t *__restrict__ dzt, float *__restrict__ loss_rows) {
     __shared__ __align__(4) uint16_t tr[kRowThreads * kSoftStride];
     const int lane = threadIdx.x & 31, rl = threadIdx.x >> 5;
@@ -352,6 +352,12 @@ __global__ void __launch_bounds__(32 * kSoftRows, 2)
     grid_wait();
     const float *row = waited(logits) + base;
     targets = waited(targets);
+    // the row's targets: its own, or sample index[z * row_ms + r] of a data set (0 outside it)
+    int64_t tbase = base;
+    if (index) {
+        const int64_t smp = waited(index)[z * row_ms + (live ? r : r0)];
+        tbase = (smp < 0 || smp >= samples ? 0 : smp) * nout;
+    }
     float held[Per ? Per * kSoftSlices : 1] = {};
     if constexpr (Per > 0) {
 #pragma unroll
@@ -380,7 +386,7 @@ __global__ void __launch_bounds__(32 * kSoftRows, 2)
     for (int i = 0; i < per; ++i) {
         float t[kSoftSlices];
 #pragma unroll
-        for (int w = 0; w < kSoftSlices; ++w) t[w] = targets ? targets[base + i * kRowThreads + 32 * w + lane] : 0.f;
+        for (int w = 0; w < kSoftSlices; ++w) t[w] = targets ? targets[tbase + i * kRowThreads + 32 * w + lane] : 0.f;
 #pragma unroll
         for (int w = 0; w < kSoftSlices; ++w) {
             const int c = 32 * w + lane, j = i * kRowThreads + c;
@@ -415,7 +421,7 @@ __global__ void __launch_bounds__(32 * kSoftRows, 2)
     }
 }
 
-static int launch_softmax(const float *logits, const float *targets, int rows, int members, int nout, int64_t row_ms,
+static int launch_softmax(const float *logits, const float *targets, const int32_t *index, int64_t samples, int rows, int members, int nout, int64_t row_ms,
                           int64_t out_ms, int64_t ld_t, float grad_scale, float *probs, uint16_t *dz, uint16_t *dzt,
                           float *loss_rows, cudaStream_t s) {
     const dim3 grid((rows + kSoftRows - 1) / kSoftRows, members), block(32 * kSoftRows);
@@ -423,7 +429,7 @@ static int launch_softmax(const float *logits, const float *targets, int rows, i
                 : nout == 512 ? softmax_kernel<2>
                 : nout == 768 ? softmax_kernel<3>
                 : nout == 1024 ? softmax_kernel<4> : softmax_kernel<0>;
-    return launch_early(kernel, grid, block, 0, s, logits, targets, rows, nout, row_ms, out_ms, ld_t, grad_scale, probs,
+    return launch_early(kernel, grid, block, 0, s, logits, targets, index, samples, rows, nout, row_ms, out_ms, ld_t, grad_scale, probs,
                         dz, dzt, loss_rows);
 }
 
@@ -448,6 +454,7 @@ __global__ void bias_grad_kernel(const __grid_constant__ BiasGrads B) {
     const int64_t z = blockIdx.y;
     const uint16_t *src = B.dt[i] + z * B.d_ms[i] + int64_t(n) * B.ld;
     float s = 0.f;
+#pragma unroll 8
     for (int b = lane; b < B.rows; b += 32) s += from_bf16(src[b]);
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (lane == 0) B.db[i][z * B.db_ms + n] = s;
@@ -524,26 +531,47 @@ __global__ void __launch_bounds__(256) adam_kernel(float *__restrict__ params, c
     }
 }
 
-// Row r of member z from sample index[z * rows + r].
-__global__ void gather_kernel(const float *__restrict__ features, int nfeat, const float *__restrict__ targets,
-                              int nout, int64_t samples, const int32_t *__restrict__ index, int rows, int width,
-                              uint16_t *__restrict__ x, uint16_t *__restrict__ xt, float *__restrict__ t) {
-    const int64_t r = blockIdx.x, z = blockIdx.y;
+// Row r of member z from sample index[z * rows + r] (sample 0 for an index outside the data set): 32 rows
+// per block, the features through shared memory so that the transpose leaves in rows of 32 too.
+constexpr int kGatherRows = 32;
+__global__ void __launch_bounds__(256) gather_kernel(const float *__restrict__ features, int nfeat,
+                                                     const float *__restrict__ targets, int nout, int64_t samples,
+                                                     const int32_t *__restrict__ index, int rows, int width,
+                                                     uint16_t *__restrict__ x, uint16_t *__restrict__ xt,
+                                                     float *__restrict__ t) {
+    __shared__ int64_t sample[kGatherRows];
+    __shared__ uint16_t tile[kGatherRows][33];
+    const int64_t z = blockIdx.y;
+    const int r0 = blockIdx.x * kGatherRows, n = min(kGatherRows, rows - r0), tid = threadIdx.x;
     grid_wait();
     features = waited(features);
     targets = waited(targets);
-    int64_t s = waited(index)[z * rows + r];
-    if (s < 0 || s >= samples) s = 0;       // an index outside the data set reads sample 0
-    if (targets) {
-        const float4 *src = reinterpret_cast<const float4 *>(targets + s * nout);
-        float4 *dst = reinterpret_cast<float4 *>(t + (z * rows + r) * nout);
-        for (int j = threadIdx.x; j < nout / 4; j += blockDim.x) dst[j] = src[j];
+    if (tid < n) {
+        const int64_t s = waited(index)[z * rows + r0 + tid];
+        sample[tid] = s < 0 || s >= samples ? 0 : s;
     }
-    for (int f = threadIdx.x; f < width; f += blockDim.x) {
-        const uint16_t b = to_bf16(f < nfeat ? features[s * nfeat + f] : 0.f);
-        x[(z * rows + r) * width + f] = b;
-        xt[(z * width + f) * rows + r] = b;
+    __syncthreads();
+    for (int f0 = 0; f0 < width; f0 += 32) {
+        for (int i = tid; i < n * 32; i += 256) {
+            const int r = i >> 5, f = f0 + (i & 31);
+            if (f >= width) continue;
+            const uint16_t b = to_bf16(f < nfeat ? features[sample[r] * nfeat + f] : 0.f);
+            x[(z * rows + r0 + r) * width + f] = b;
+            tile[r][i & 31] = b;
+        }
+        __syncthreads();
+        for (int i = tid; i < 32 * 32; i += 256) {
+            const int r = i & 31, f = f0 + (i >> 5);
+            if (r < n && f < width) xt[(z * width + f) * rows + r0 + r] = tile[r][i >> 5];
+        }
+        __syncthreads();
     }
+    if (targets)
+        for (int r = 0; r < n; ++r) {
+            const float4 *src = reinterpret_cast<const float4 *>(targets + sample[r] * nout);
+            float4 *dst = reinterpret_cast<float4 *>(t + (z * rows + r0 + r) * nout);
+            for (int j = tid; j < nout / 4; j += 256) dst[j] = src[j];
+        }
 }
 
 // Rows of samples first, first + 1, ... (the last one beyond the data set) for every member alike, kPackCols
@@ -757,7 +785,7 @@ extern "C" int dm_mlp_softmax_xent(const float *logits, const float *targets, in
     DM_CHECK_ARG(logits && rows > 0 && members >= 1 && members <= 65535 && nout > 0);
     DM_CHECK_ARG(nout % kRowThreads == 0 && nout <= 16 * kRowThreads);
     DM_CHECK_ARG(targets ? (dz && dzt) : (probs != nullptr));
-    return launch_softmax(logits, targets, rows, members, nout, rows, rows, rows, grad_scale, probs, dz, dzt, loss_rows,
+    return launch_softmax(logits, targets, nullptr, 0, rows, members, nout, rows, rows, rows, grad_scale, probs, dz, dzt, loss_rows,
                           as_stream(stream));
 }
 
@@ -813,7 +841,7 @@ extern "C" int dm_mlp_gather(const float *features, int nfeat, const float *targ
     DM_CHECK_ARG(features && index && x && xt && nfeat > 0 && nfeat <= width && samples > 0);
     DM_CHECK_ARG(rows > 0 && members >= 1 && members <= 65535 && width % 8 == 0 && nout > 0 && nout % 4 == 0);
     DM_CHECK_ARG(!targets || (t && mlp::aligned16(targets) && mlp::aligned16(t)));
-    return launch_early(mlp::gather_kernel, dim3(rows, members), dim3(256), 0, as_stream(stream), features, nfeat, targets,
+    return launch_early(mlp::gather_kernel, dim3((rows + mlp::kGatherRows - 1) / mlp::kGatherRows, members), dim3(256), 0, as_stream(stream), features, nfeat, targets,
                         nout, samples, index, rows, width, x, xt, t);
 }
 
@@ -975,10 +1003,12 @@ static int backward(const dm_mlp_net &n, int rows, cudaStream_t s) {
     return launch_bias_grads(bg, n.members, s);
 }
 
-static int loss_and_grads(const dm_mlp_net &n, int rows, cudaStream_t s) {
+// targets: the batch's own (n.t), or rows index[] of a data set of `samples`
+static int loss_and_grads(const dm_mlp_net &n, int rows, const float *targets, const int32_t *index, int64_t samples,
+                          cudaStream_t s) {
     int rc = forward(n, rows, true, int64_t(n.batch) * kInput, s);
     if (rc) return rc;
-    if ((rc = launch_softmax(n.logits, n.t, rows, n.members, n.nout, n.batch, n.batch, n.batch, float(1.0 / rows), n.probs,
+    if ((rc = launch_softmax(n.logits, targets, index, samples, rows, n.members, n.nout, n.batch, n.batch, n.batch, float(1.0 / rows), n.probs,
                              n.dz, n.dzt, n.loss_rows, s)))
         return rc;
     return backward(n, rows, s);
@@ -999,7 +1029,7 @@ extern "C" int dm_mlp_backward(const dm_mlp_net *net, int rows, void *stream) {
 
 extern "C" int dm_mlp_loss_and_grads(const dm_mlp_net *net, int rows, void *stream) {
     const int rc = mlp::check_net(net, rows, true);
-    return rc ? rc : mlp::loss_and_grads(*net, rows, as_stream(stream));
+    return rc ? rc : mlp::loss_and_grads(*net, rows, net->t, nullptr, 0, as_stream(stream));
 }
 
 extern "C" int dm_mlp_train_step(const dm_mlp_net *net, const float *features, int nfeat, const float *targets,
@@ -1008,11 +1038,12 @@ extern "C" int dm_mlp_train_step(const dm_mlp_net *net, const float *features, i
     int rc = mlp::check_net(net, net ? net->batch : 0, true);
     if (rc) return rc;
     const dm_mlp_net &n = *net;
-    DM_CHECK_ARG(features && targets && index && n.m && n.v && step >= 1);
-    if ((rc = dm_mlp_gather(features, nfeat, targets, n.nout, samples, index, n.batch, n.members, mlp::kInput, n.x, n.xt,
-                            n.t, stream)))
+    DM_CHECK_ARG(features && targets && index && n.m && n.v && step >= 1 && mlp::aligned16(targets));
+    if ((rc = dm_mlp_gather(features, nfeat, nullptr, n.nout, samples, index, n.batch, n.members, mlp::kInput, n.x, n.xt,
+                            nullptr, stream)))
         return rc;
-    if ((rc = mlp::loss_and_grads(n, n.batch, as_stream(stream)))) return rc;
+    // the softmax reads its targets from the data set (gathering them took 12 us of a 150 us step)
+    if ((rc = mlp::loss_and_grads(n, n.batch, targets, index, samples, as_stream(stream)))) return rc;
     const int32_t shapes[2 * mlp::kLayers] = {mlp::kHidden, mlp::kInput,  mlp::kHidden, mlp::kHidden,
                                               mlp::kHidden, mlp::kHidden, n.nout,       mlp::kHidden};
     return dm_mlp_adam(n.params, n.grads, n.m, n.v, n.count, n.members, shapes, mlp::kLayers, lr, beta1, beta2, eps, step,
@@ -1033,7 +1064,7 @@ extern "C" int dm_mlp_predict(const dm_mlp_net *net, const float *features, int 
                           features, nfeat, samples, s0, padded, n.x);
         if (rc) return rc;
         if ((rc = mlp::forward(n, rows, false, 0, s))) return rc;
-        if ((rc = mlp::launch_softmax(n.logits, nullptr, rows, n.members, n.nout, n.batch, samples, 0, 1.f,
+        if ((rc = mlp::launch_softmax(n.logits, nullptr, nullptr, 0, rows, n.members, n.nout, n.batch, samples, 0, 1.f,
                                       out + s0 * n.nout, nullptr, nullptr, nullptr, s)))
             return rc;
     }

@@ -240,3 +240,44 @@ def test_gemm_launch_shapes(M, N_, K, members, epi):
         err = np.abs(_f(bf) - want)
         assert np.all(err <= 2.0 ** -8 * np.abs(want) + 1.13 * tol + 64 * U)
         assert np.array_equal(bf.cpu().numpy(), np.swapaxes(t.cpu().numpy(), 1, 2))
+
+
+@pytest.mark.parametrize('rows', [1, 31, 32, 33, 100])
+@pytest.mark.parametrize('nfeat,width', [(6, 64), (64, 64), (7, 8), (33, 40)])
+def test_gather(rows, nfeat, width):
+    """Blocks of 32 rows, ragged ends, widths that are no multiple of 32; indexes outside the data set read sample 0."""
+    torch = _torch()
+    members, nout, samples = 3, 12, 50
+    rng = np.random.default_rng(rows + nfeat)
+    f = rng.normal(size=(samples, nfeat)).astype(np.float32)
+    t = rng.normal(size=(samples, nout)).astype(np.float32)
+    idx = rng.integers(0, samples, (members, rows)).astype(np.int32)
+    idx[0, 0], idx[1, rows - 1] = -1, samples
+    used = np.where((idx < 0) | (idx >= samples), 0, idx)
+    x = torch.full((members, rows, width), 7, dtype=torch.int16, device='cuda')
+    xt = torch.full((members, width, rows), 7, dtype=torch.int16, device='cuda')
+    td = torch.zeros((members, rows, nout), device='cuda')
+    fd, tg, ix = (torch.from_numpy(a).cuda() for a in (f, t, idx))
+    vp = ctypes.c_void_p
+    N.call('dm_mlp_gather', vp(fd.data_ptr()), nfeat, vp(tg.data_ptr()), nout, ctypes.c_int64(samples), vp(ix.data_ptr()),
+           rows, members, width, vp(x.data_ptr()), vp(xt.data_ptr()), vp(td.data_ptr()), None)
+    want = np.zeros((members, rows, width), np.float32)
+    want[:, :, :nfeat] = MO.bf16(f)[used]
+    assert np.array_equal(_f(x), want)
+    assert np.array_equal(_f(xt), np.swapaxes(want, 1, 2))
+    assert np.array_equal(td.cpu().numpy(), t[used])
+
+
+def test_train_step_equals_its_parts():
+    """The step reads its targets from the data set; gathering them first gives the same parameters."""
+    torch = _torch()
+    g = torch.Generator('cuda').manual_seed(8)
+    f = torch.rand(300, 6, device='cuda', generator=g) * 2 - 1
+    t = torch.softmax(torch.randn(300, 256, device='cuda', generator=g), dim=1)
+    index = torch.randint(-2, 303, (2, 128), device='cuda', generator=g, dtype=torch.int32)
+    a, b = (S.MLPEnsemble(members=2, batch=128, nout=256, seed=3) for _ in range(2))
+    a.train_step(f, t, index, 1e-3)
+    b.gather(f, t, index, 128)
+    b.loss_and_grads(128)
+    b._adam(1, 1e-3)
+    assert torch.equal(a.params, b.params) and torch.equal(a.loss_rows, b.loss_rows) and torch.equal(a.grads, b.grads)
