@@ -474,7 +474,9 @@ struct Layers {
 };
 
 // One block per 32 x 32 tile of a weight matrix, so that the transposed BF16 copy leaves in rows too
-// (element by element it cost a sector per value: 26 us for 2 M parameters), then blocks of biases.
+// (element by element it cost a sector per value), then blocks of biases.  Vec: four
+// weights per thread at once, where every row of every matrix is 16-byte aligned (2 M parameters, 66 MB: 25 -> 12.6 us).
+template <bool Vec>
 __global__ void __launch_bounds__(256) adam_kernel(float *__restrict__ params, const float *__restrict__ grads,
                                                    float *__restrict__ m, float *__restrict__ v, int64_t P,
                                                    const __grid_constant__ Layers L, float lr, float b1, float b2,
@@ -483,15 +485,18 @@ __global__ void __launch_bounds__(256) adam_kernel(float *__restrict__ params, c
     __shared__ uint16_t tr[32][33];
     grid_wait();
     grads = waited(grads);
+    auto rule = [&](float p, float gr, float &mm, float &vv) {
+        mm = b1 * mm + (1.f - b1) * gr;
+        vv = b2 * vv + (1.f - b2) * gr * gr;
+        return p - lr * (mm / c1) / (sqrtf(vv / c2) + eps);
+    };
     auto update = [&](int64_t i) {
         float p = params[i];
         if (step > 0) {
-            const float gr = grads[i];
-            const float mm = b1 * m[i] + (1.f - b1) * gr;
-            const float vv = b2 * v[i] + (1.f - b2) * gr * gr;
+            float mm = m[i], vv = v[i];
+            p = rule(p, grads[i], mm, vv);
             m[i] = mm;
             v[i] = vv;
-            p -= lr * (mm / c1) / (sqrtf(vv / c2) + eps);
             params[i] = p;
         }
         return p;
@@ -511,14 +516,39 @@ __global__ void __launch_bounds__(256) adam_kernel(float *__restrict__ params, c
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     for (int64_t z = blockIdx.y; z < members; z += gridDim.y) {
         const int64_t w0 = z * P + L.w_off[l];
+        if constexpr (Vec) {
+            const int rr = threadIdx.x >> 3, cc = 4 * (threadIdx.x & 7);
+            if (r0 + rr < out && c0 + cc < in) {
+                const int64_t i = w0 + int64_t(r0 + rr) * in + c0 + cc;
+                float4 p = *reinterpret_cast<const float4 *>(params + i);
+                if (step > 0) {
+                    const float4 gr = *reinterpret_cast<const float4 *>(grads + i);
+                    float4 mm = *reinterpret_cast<const float4 *>(m + i), vv = *reinterpret_cast<const float4 *>(v + i);
+                    p.x = rule(p.x, gr.x, mm.x, vv.x);
+                    p.y = rule(p.y, gr.y, mm.y, vv.y);
+                    p.z = rule(p.z, gr.z, mm.z, vv.z);
+                    p.w = rule(p.w, gr.w, mm.w, vv.w);
+                    *reinterpret_cast<float4 *>(m + i) = mm;
+                    *reinterpret_cast<float4 *>(v + i) = vv;
+                    *reinterpret_cast<float4 *>(params + i) = p;
+                }
+                const uint32_t lo = pack2(p.x, p.y), hi = pack2(p.z, p.w);
+                *reinterpret_cast<uint2 *>(wb + i) = make_uint2(lo, hi);
+                tr[rr][cc] = uint16_t(lo);
+                tr[rr][cc + 1] = uint16_t(lo >> 16);
+                tr[rr][cc + 2] = uint16_t(hi);
+                tr[rr][cc + 3] = uint16_t(hi >> 16);
+            }
+        } else {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int r = r0 + ty + 8 * k, c = c0 + tx;
-            if (r < out && c < in) {
-                const int64_t i = w0 + int64_t(r) * in + c;
-                const uint16_t h = to_bf16(update(i));
-                wb[i] = h;
-                tr[ty + 8 * k][tx] = h;
+            for (int k = 0; k < 4; ++k) {
+                const int r = r0 + ty + 8 * k, c = c0 + tx;
+                if (r < out && c < in) {
+                    const int64_t i = w0 + int64_t(r) * in + c;
+                    const uint16_t h = to_bf16(update(i));
+                    wb[i] = h;
+                    tr[ty + 8 * k][tx] = h;
+                }
             }
         }
         __syncthreads();
@@ -831,7 +861,10 @@ extern "C" int dm_mlp_adam(float *params, const float *grads, float *m, float *v
     const double c1 = step > 0 ? 1.0 - pow(double(beta1), step) : 1.0;
     const double c2 = step > 0 ? 1.0 - pow(double(beta2), step) : 1.0;
     const dim3 grid(L.tiles[nlayers] + L.bias_blocks[nlayers], members < 65535 ? members : 65535);
-    return launch_early(mlp::adam_kernel, grid, dim3(256), 0, as_stream(stream), params, grads, m, v, count_per_member, L, lr,
+    bool vec = count_per_member % 4 == 0 && mlp::aligned16(params) && mlp::aligned16(grads) && mlp::aligned16(m) &&
+               mlp::aligned16(v) && (reinterpret_cast<uintptr_t>(w_bf16) & 7) == 0;
+    for (int l = 0; l < nlayers; ++l) vec = vec && L.w_off[l] % 4 == 0 && L.in[l] % 4 == 0;
+    return launch_early(vec ? mlp::adam_kernel<true> : mlp::adam_kernel<false>, grid, dim3(256), 0, as_stream(stream), params, grads, m, v, count_per_member, L, lr,
                         beta1, beta2, eps, float(c1), float(c2), step, members, w_bf16, wt_bf16);
 }
 

@@ -100,9 +100,10 @@ def test_softmax_rows(rows, nout):
     assert np.array_equal(dz.cpu().numpy(), np.swapaxes(dzt.cpu().numpy(), 1, 2))
 
 
-def test_adam_of_ragged_shapes():
+@pytest.mark.parametrize('shapes', [[(5, 7), (33, 64), (64, 33), (300, 32), (1, 1)],      # element by element
+                                    [(8, 4), (36, 64), (64, 36), (300, 32)]])             # four weights at once
+def test_adam_of_ragged_shapes(shapes):
     torch = _torch()
-    shapes = [(5, 7), (33, 64), (64, 33), (300, 32), (1, 1)]
     P = sum(o * i + o for o, i in shapes)
     Z = 3
     rng = np.random.default_rng(1)
