@@ -47,10 +47,10 @@ inline int launch_status() {
 // launches 654 and 528 us; the 16 passes of 20 layers on 10 qubits 356 us, and 244 us with this, a tile
 // per SM and one composition launch for all of them.
 template <typename... P, typename... A>
-int launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...args) {
+int launch_early_if(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...args) {
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
+    at.val.programmaticStreamSerializationAllowed = early ? 1 : 0;
     cudaLaunchConfig_t c{};
     c.gridDim = grid;
     c.blockDim = block;
@@ -61,6 +61,11 @@ int launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaS
     (void)cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);
     count_launch();
     return launch_status();
+}
+
+template <typename... P, typename... A>
+int launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...args) {
+    return launch_early_if(true, kernel, grid, block, smem, s, std::forward<A>(args)...);
 }
 
 #ifdef __CUDACC__

@@ -71,6 +71,7 @@ constexpr int kThreads = kTeams * kTeamThreads;
 constexpr int kMaxRounds = 16;                               // rounds of one pass
 constexpr int kUSlots = 6;                                   // round-image slots in shared memory
 constexpr int kStreamFrom = 4;                               // longer passes: rounds >= 4 streamed (slot 4 + team)
+constexpr int kEarlyTiles = 256;                             // tiles per SM up to which a pass starts early
 constexpr int kMaxDims = 5;                                  // tensor-map rank
 constexpr uint32_t kSlotBytes = 2 * kABytes;                 // 64 KB: AH | AL, or the FP32 tile
 constexpr uint32_t kUBytes = 2 * kBImage;                    // 16 KB per round: Uh | Ul (one 128-row operand)
@@ -564,7 +565,11 @@ extern "C" int dm_apply_pass_tma(void *state_dev, int n, const dm_tc_pass *pass,
     if (ensure_max_dynamic_smem(reinterpret_cast<const void *>(tma::pass_tma_kernel), int(tma::kSmemBytes)) !=
         cudaSuccess)
         return DM_ERR_CUDA;
-    return launch_early(tma::pass_tma_kernel, dim3(unsigned(grid)), dim3(tma::kThreads), tma::kSmemBytes, as_stream(stream),
+    // Blocks that waited for the previous pass all start at one moment and stream their tiles in step, which a
+    // long pass pays for: 84 passes on 16 qubits (1,725 tiles per SM) 882 ms early, 869 ms otherwise; 15 qubits
+    // (431) 77.6 both ways; 14 qubits (108) 50.0 and 50.4 ms; 10 qubits 243 and 266 us.
+    const bool early = p.ntiles <= int64_t(tma::kEarlyTiles) * sm_count();
+    return launch_early_if(early, tma::pass_tma_kernel, dim3(unsigned(grid)), dim3(tma::kThreads), tma::kSmemBytes, as_stream(stream),
                         map, p, static_cast<float *>(state_dev), umats_dev, status_dev);
 }
 
