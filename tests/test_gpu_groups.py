@@ -66,3 +66,15 @@ def test_template_of_many_slots():
     got = TP.TemplateRunner(tc).run(S.param_vectors(raw)).cpu().numpy()
     ref = TP.TemplateRunner(cc).run(S.param_vectors(raw)).cpu().numpy()
     assert np.abs(got - ref).max() < 4e-6
+
+
+@pytest.mark.parametrize('count', [1, 20, 310])
+def test_passes_of_many_rounds(count):
+    """Passes of 20 rounds (7 qubits, 30 layers): more than one CTA composes at a time, alone and in groups."""
+    specs = [_spec(7, 30, 700 + i) for i in range(count)]
+    got = _run(specs)
+    pick = sorted({0, count // 2, count - 1})
+    for i in pick:
+        assert np.array_equal(got[i], _run([specs[i]])[0]), i
+    for g, w in zip((got[i] for i in pick), _run([specs[i] for i in pick], 'double')):
+        assert np.abs(g - w).max() < 2e-6
