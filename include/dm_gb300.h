@@ -571,7 +571,8 @@ int dm_mlp_loss_and_grads(const dm_mlp_net *net, int rows, void *stream);
 int dm_mlp_train_step(const dm_mlp_net *net, const float *features, int nfeat, const float *targets,
                       int64_t samples, const int32_t *index, float lr, float beta1, float beta2, float eps,
                       int step, void *stream);
-/* Member distributions out[members][samples][nout] of every feature row. */
+/* Member distributions out[members][samples][nout] of every feature row (features
+ * and out may be NULL when samples == 0). */
 int dm_mlp_predict(const dm_mlp_net *net, const float *features, int nfeat, int64_t samples, float *out,
                    void *stream);
 

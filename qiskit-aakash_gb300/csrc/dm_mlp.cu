@@ -1088,7 +1088,8 @@ extern "C" int dm_mlp_predict(const dm_mlp_net *net, const float *features, int 
     int rc = mlp::check_net(net, net ? net->batch : 0, false);
     if (rc) return rc;
     const dm_mlp_net &n = *net;
-    DM_CHECK_ARG(features && out && nfeat > 0 && nfeat <= mlp::kInput && samples >= 0);
+    DM_CHECK_ARG(nfeat > 0 && nfeat <= mlp::kInput && samples >= 0);
+    DM_CHECK_ARG(samples == 0 || (features && out));      // an empty tensor has no address
     cudaStream_t s = as_stream(stream);
     for (int64_t s0 = 0; s0 < samples; s0 += n.batch) {
         const int rows = int(samples - s0 < n.batch ? samples - s0 : n.batch);

@@ -282,3 +282,13 @@ def test_train_step_equals_its_parts():
     b.loss_and_grads(128)
     b._adam(1, 1e-3)
     assert torch.equal(a.params, b.params) and torch.equal(a.loss_rows, b.loss_rows) and torch.equal(a.grads, b.grads)
+
+
+@pytest.mark.parametrize('members', [1, 3])
+def test_prediction_of_no_points(members):
+    """An empty set, whose tensors have no address, has an empty result; more points without one are refused."""
+    torch = _torch()
+    ens = S.MLPEnsemble(members=members, batch=128, nout=256)
+    got = ens.predict(torch.empty((0, 6), device='cuda'))
+    assert got.shape == (members, 0, 256) and got.dtype == torch.float32 and got.is_cuda
+    assert N.lib().dm_mlp_predict(ens._net(), None, 6, ctypes.c_int64(1), None, None) == N.DM_ERR_ARG
