@@ -277,7 +277,9 @@ int dm_plan_passes(int n, int kmax, int low, const dm_plan_op *ops, int count, i
 
 /* Descriptors and coefficients of planned passes for dm_apply_pass; host code.
  * coefs holds the ops' coefficients one after another (DM_OP_MAP1 and
- * DM_OP_DIAG2 16, DM_OP_CX 5, DM_OP_MAP2 256).  With width > 0 a pass's ops are
+ * DM_OP_DIAG2 16, DM_OP_CX 5, DM_OP_MAP2 256).  A pass's ops, in order, take its
+ * slots in order or share an earlier one, one-axis maps on one axis only
+ * (DM_ERR_ARG otherwise).  With width > 0 a pass's ops are
  * grouped into register rounds of width axes when it has width..max_axes
  * resident axes, qubit n-1 among them, no DM_OP_MAP2 and at most DM_MAX_ROUNDS
  * rounds.  mats (host memory of the state's type, mats_capacity values) gets

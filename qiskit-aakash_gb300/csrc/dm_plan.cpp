@@ -116,8 +116,10 @@ struct Composed {
     const double *data;
 };
 
-// Group the ops of one pass or round by slot; maps that share a slot are multiplied in order.
-void compose(const dm_plan_op *ops, const double *const *data, const std::vector<int32_t> &members,
+// Group the ops of one pass or round by slot; maps that share a slot are multiplied in order.  False where
+// the slots are not what a scan gives: taken in order, and shared by one-axis maps on one axis only (a slot
+// shared by a CX would read its 5 coefficients as 16).
+bool compose(const dm_plan_op *ops, const double *const *data, const std::vector<int32_t> &members,
              const int32_t *slot_of, std::vector<Composed> &body, std::vector<double> &products) {
     body.clear();
     products.clear();
@@ -125,15 +127,19 @@ void compose(const dm_plan_op *ops, const double *const *data, const std::vector
     for (const int32_t i : members) {
         const size_t slot = size_t(slot_of[i]);
         if (slot < body.size()) {
+            const dm_plan_op &first = body[slot].op;
+            if (first.kind != DM_OP_MAP1 || ops[i].kind != DM_OP_MAP1 || first.a != ops[i].a) return false;
             double c[16];
             multiply(data[i], body[slot].data, c);
             const size_t at = products.size();
             products.insert(products.end(), c, c + 16);
             body[slot].data = products.data() + at;
         } else {
+            if (slot != body.size()) return false;
             body.push_back({ops[i], data[i]});
         }
     }
+    return true;
 }
 
 }  // namespace
@@ -187,8 +193,8 @@ extern "C" int dm_encode_passes(int n, int dtype, int width, int max_axes, const
                 local_of[q] = dp.k;
                 dp.axes[dp.k++] = q;
             }
-        compose(ops, data.data(), members[size_t(p)], slot_of, body, products);
-        if (body.size() > DM_MAX_PASS_OPS) return DM_ERR_ARG;
+        if (!compose(ops, data.data(), members[size_t(p)], slot_of, body, products) || body.size() > DM_MAX_PASS_OPS)
+            return DM_ERR_ARG;
         bool map2 = false;
         local.clear();
         local_data.clear();
@@ -251,7 +257,8 @@ extern "C" int dm_encode_passes(int n, int dtype, int width, int max_axes, const
                     dp.round_axes[r][d++] = int8_t(a);
                 }
             for (; d < 4; ++d) dp.round_axes[r][d] = -1;
-            compose(local.data(), local_data.data(), by_round[r], round_slot.data(), regrouped, round_products);
+            if (!compose(local.data(), local_data.data(), by_round[r], round_slot.data(), regrouped, round_products))
+                return DM_ERR_PROGRAM;
             for (const Composed &c : regrouped) {
                 const int32_t digits = (at[c.op.a] << 8) | (c.op.kind == DM_OP_MAP1 ? 0 : at[c.op.b] << 12);
                 if (!emit(c, digits)) return DM_ERR_ARG;

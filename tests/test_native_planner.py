@@ -131,3 +131,30 @@ def test_full_pass_of_128_ops_and_what_is_refused():
     assert (mats == 7.0).all()
     with pytest.raises(ValueError):
         P.encode_plan(P.Plan([P.Op('map1', (0,), np.eye(3))], 1, 1, 0), 1, np.float64, None, mats.ctypes.data, 16)
+
+
+@pytest.mark.parametrize('kinds,axes,slots,ok', [
+    (('map1', 'map1', 'map1'), ((0,), (1,), (0,)), (0, 1, 0), True),
+    (('cx', 'cx'), ((0, 1), (0, 1)), (0, 0), False),              # 5 coefficients each
+    (('diag2', 'diag2'), ((0, 1), (0, 1)), (0, 0), False),
+    (('cx', 'map1'), ((0, 1), (0,)), (0, 0), False),
+    (('map1', 'cx'), ((0,), (0, 1)), (0, 0), False),
+    (('map1', 'map1'), ((0,), (1,)), (0, 0), False),              # two axes
+    (('map1', 'map1'), ((0,), (1,)), (0, 2), False),              # a gap
+    (('map1', 'map1'), ((0,), (1,)), (1, 0), False)])
+@pytest.mark.parametrize('width', [None, 2])
+def test_slots_that_no_scan_gives_are_refused(kinds, axes, slots, ok, width):
+    size = {'map1': (4, 4), 'cx': (5,), 'diag2': (16,)}
+    ops = [P.Op(k, a, np.ones(size[k])) for k, a in zip(kinds, axes)]
+    plan = P.Plan(ops, 2, 2, 2)
+    assert len(plan.resident) == 1
+    plan.slot_of = np.array(slots, dtype=np.int32)
+    mats = np.full(64, 7.0)
+    if ok:
+        _, used = P.encode_plan(plan, 2, np.float64, width, mats.ctypes.data, mats.size)
+        assert used == 32
+        return
+    with pytest.raises(N.NativeError) as e:
+        P.encode_plan(plan, 2, np.float64, width, mats.ctypes.data, mats.size)
+    assert e.value.code == N.DM_ERR_ARG
+    assert (mats == 7.0).all()
