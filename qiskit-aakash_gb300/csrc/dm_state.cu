@@ -156,6 +156,9 @@ __global__ void __launch_bounds__(256) max_abs_diff_kernel(const TA *__restrict_
 // 128-byte runs out).  Measured at n = 12 in FP64: 525 us (sweeps of 238, 108
 // and 179 us, the FP64 pipe 80 % busy), where one complex sweep per axis and a
 // de-interleaving gather took 1,157 us.
+//
+// An infinity or NaN in M would reach both parts of rho, and as inf - inf.  Tiles
+// that hold one are computed again by mat_exact, even and odd #Y apart.
 // ---------------------------------------------------------------------------
 
 constexpr int kMatLow = 6;        // axes of the first sweep
@@ -233,19 +236,76 @@ __device__ __forceinline__ uint32_t compact(uint32_t x) {
     return (x | (x >> 8)) & 0x0000ffffu;
 }
 
+// Where entry i (row-major) of tile t's part lies in rho; sr, sc: its tile row and column, bits spread apart.
+__device__ __forceinline__ int64_t mat_entry(int i, int n, int lowbits, int topbits, uint32_t t, int &sr, int &sc) {
+    const int bits = lowbits + topbits, c = i & ((1 << bits) - 1), r = i >> bits;
+    const uint32_t ro = compact(t >> 1) << lowbits, co = compact(t) << lowbits;
+    sc = spread6(c);
+    sr = spread6(r);
+    const uint32_t row = ro | uint32_t(r & ((1 << lowbits) - 1)) | (uint32_t(r >> lowbits) << (n - topbits));
+    const uint32_t col = co | uint32_t(c & ((1 << lowbits) - 1)) | (uint32_t(c >> lowbits) << (n - topbits));
+    return (int64_t(row) << n) | col;
+}
+
+__device__ __forceinline__ bool mat_nonfinite(double v) { return (__double2hiint(v) & 0x7ff00000) == 0x7ff00000; }
+
 // Tile t's part of rho, from the tile of M (a) and the tile of M holding the transposed entries (b).
 // lowbits: the matrix bits of the run axes; topbits: those of the top axes, at bit n - topbits.
-__device__ __forceinline__ void mat_write(const double *a, const double *b, int n, int lowbits, int topbits,
+// True where this thread met an infinity or a NaN.
+__device__ __forceinline__ bool mat_write(const double *a, const double *b, int n, int lowbits, int topbits,
                                           uint32_t t, double2 *__restrict__ out) {
-    const int bits = lowbits + topbits;
-    const uint32_t ro = compact(t >> 1) << lowbits, co = compact(t) << lowbits;
-    for (int i = threadIdx.x; i < 1 << (2 * bits); i += blockDim.x) {
-        const int c = i & ((1 << bits) - 1), r = i >> bits;
-        const int sc = spread6(c), sr = spread6(r);
+    bool bad = false;
+    for (int i = threadIdx.x; i < 1 << (2 * (lowbits + topbits)); i += blockDim.x) {
+        int sr, sc;
+        const int64_t at = mat_entry(i, n, lowbits, topbits, t, sr, sc);
         const double u = a[mat_swz(sc | (sr << 1))], w = b[mat_swz(sr | (sc << 1))];
-        const uint32_t row = ro | uint32_t(r & ((1 << lowbits) - 1)) | (uint32_t(r >> lowbits) << (n - topbits));
-        const uint32_t col = co | uint32_t(c & ((1 << lowbits) - 1)) | (uint32_t(c >> lowbits) << (n - topbits));
-        out[(int64_t(row) << n) | col] = make_double2(u + w, u - w);
+        bad = bad || mat_nonfinite(u) || mat_nonfinite(w);
+        out[at] = make_double2(u + w, u - w);
+    }
+    return bad;
+}
+
+// Tile t's part of rho again, straight from the state: the real part from the coefficients of even #Y,
+// the imaginary part from those of odd #Y, so that neither sees the other's infinities.  The digits
+// between the run and the top axes are summed (I and Z, or X and Y, as the tile's digit says), the
+// others run as butterflies in the tile.  2**(n - 6) loads per entry: for infinities and NaN only.
+template <typename T>
+__device__ __noinline__ void mat_exact(const T *__restrict__ st, double *tile, int n, int lowbits, int topbits,
+                                       uint32_t t, double2 *__restrict__ out) {
+    const int K = lowbits + topbits, tsize = 1 << (2 * K), mid = n - K;
+    for (int part = 0; part < 2; ++part) {
+        __syncthreads();
+        for (int e = threadIdx.x; e < tsize; e += blockDim.x) {
+            const uint64_t at =
+                uint64_t(e & ((1 << (2 * lowbits)) - 1)) | (uint64_t(e >> (2 * lowbits)) << (2 * (n - topbits)));
+            double sum = 0.0;
+            for (uint32_t m = 0; m < 1u << mid; ++m) {
+                uint64_t i = at;
+                uint32_t neg = 0;
+                for (int j = 0; j < mid; ++j) {
+                    const uint32_t d = (t >> (2 * j)) & 3, b = (m >> j) & 1;
+                    i |= uint64_t(d == 0 || d == 3 ? 3 * b : 1 + b) << (2 * (lowbits + j));
+                    neg ^= b & (d >> 1);
+                }
+                const int ys = __popcll((i >> 1) & ~i & 0x5555555555555555ull);
+                if ((ys & 1) != part) continue;
+                neg ^= uint32_t(ys + 1) >> 1 & 1;
+                const double v = double(st[i]);
+                sum += neg ? -v : v;
+            }
+            tile[mat_swz(e)] = sum;
+        }
+        __syncthreads();
+        mat_axes(tile, tsize, K, 0);
+        for (int i = threadIdx.x; i < tsize; i += blockDim.x) {
+            int sr, sc;
+            const int64_t o = mat_entry(i, n, lowbits, topbits, t, sr, sc);
+            const double v = tile[mat_swz(sc | (sr << 1))];
+            if (part == 0)
+                out[o].x = v;
+            else
+                out[o].y = v;
+        }
     }
 }
 
@@ -265,7 +325,7 @@ __global__ void __launch_bounds__(256) mat_low_kernel(const T *__restrict__ st, 
     __syncthreads();
     mat_axes(tile, tsize, L, 0);
     if (L == n) {
-        mat_write(tile, tile, n, n, 0, 0, out);
+        if (__syncthreads_or(mat_write(tile, tile, n, n, 0, 0, out))) mat_exact(st, tile, n, n, 0, 0, out);
         return;
     }
     for (int e = threadIdx.x; e < tsize; e += blockDim.x) w[base + e] = tile[mat_swz(e)];
@@ -288,8 +348,9 @@ __global__ void __launch_bounds__(256) mat_mid_kernel(double *__restrict__ w, in
 
 // The top K axes and rho: CTA t holds tile t (the digits between the run and the top axes) and the
 // tile t' of the transposed entries (row and column bits exchanged), and writes both.
-__global__ void __launch_bounds__(256) mat_top_kernel(const double *__restrict__ w, int n, int K,
-                                                      double2 *__restrict__ out) {
+template <typename T>
+__global__ void __launch_bounds__(256) mat_top_kernel(const T *__restrict__ st, const double *__restrict__ w, int n,
+                                                      int K, double2 *__restrict__ out) {
     extern __shared__ __align__(16) unsigned char mat_smem[];
     double *a = reinterpret_cast<double *>(mat_smem);
     const uint32_t t = blockIdx.x;
@@ -305,8 +366,12 @@ __global__ void __launch_bounds__(256) mat_top_kernel(const double *__restrict__
     __syncthreads();
     mat_axes(a, tsize, K, 2 * kMatRun);
     if (tt != t) mat_axes(b, tsize, K, 2 * kMatRun);
-    mat_write(a, b, n, kMatRun, K, t, out);
-    if (tt != t) mat_write(b, a, n, kMatRun, K, tt, out);
+    bool bad = mat_write(a, b, n, kMatRun, K, t, out);
+    if (tt != t) bad = mat_write(b, a, n, kMatRun, K, tt, out) || bad;
+    if (__syncthreads_or(bad)) {
+        mat_exact(st, a, n, kMatRun, K, t, out);
+        if (tt != t) mat_exact(st, b, n, kMatRun, K, tt, out);
+    }
 }
 
 }  // namespace dmg
@@ -475,6 +540,17 @@ extern "C" size_t dm_pauli_to_matrix_scratch_bytes(int n) {
     return size_t(pow4(n)) * sizeof(double2);
 }
 
+template <typename T>
+static int launch_mat_top(const T *st, const double *w, int n, int top, double2 *out, cudaStream_t s) {
+    const int smem = 2 * (1 << (2 * (top + kMatRun))) * int(sizeof(double));
+    if (ensure_max_dynamic_smem(reinterpret_cast<const void *>(mat_top_kernel<T>),
+                                2 * (1 << (2 * (kMatTop + kMatRun))) * int(sizeof(double))) != cudaSuccess)
+        return DM_ERR_CUDA;
+    mat_top_kernel<T><<<unsigned(pow4(n - top - kMatRun)), 256, smem, s>>>(st, w, n, top, out);
+    count_launch();
+    return launch_status();
+}
+
 extern "C" int dm_pauli_to_matrix(const void *state_dev, int n, int dtype, double *out_dev, void *scratch_dev,
                                   void *stream) {
     DM_CHECK_ARG(state_dev && out_dev && scratch_dev && valid_n(n) && valid_dtype(dtype));
@@ -501,13 +577,8 @@ extern "C" int dm_pauli_to_matrix(const void *state_dev, int n, int dtype, doubl
         if ((rc = launch_status())) return rc;
         lo += K;
     }
-    const int smem = 2 * (1 << (2 * (top + kMatRun))) * int(sizeof(double));
-    if (ensure_max_dynamic_smem(reinterpret_cast<const void *>(mat_top_kernel),
-                                2 * (1 << (2 * (kMatTop + kMatRun))) * int(sizeof(double))) != cudaSuccess)
-        return DM_ERR_CUDA;
-    mat_top_kernel<<<unsigned(pow4(n - top - kMatRun)), 256, smem, s>>>(w, n, top, out);
-    count_launch();
-    return launch_status();
+    return dtype == DM_F64 ? launch_mat_top(static_cast<const double *>(state_dev), w, n, top, out, s)
+                           : launch_mat_top(static_cast<const float *>(state_dev), w, n, top, out, s);
 }
 
 extern "C" int dm_max_abs_diff(const void *a_dev, int dtype_a, const void *b_dev, int dtype_b, int n, double *out_dev,

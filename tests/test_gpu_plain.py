@@ -154,3 +154,34 @@ def test_partial_read_out_sweeps(m):
     w = w.reshape(-1)
     np.testing.assert_allclose(out.cpu().numpy(), w, rtol=0,
                                atol=4 * EPS[N.DM_F64] * (m + 4) * 2 ** n * 8)
+
+
+def _matrix_parts(a, n):
+    """Real and imaginary part of the matrix by additions alone (a product 0 * inf would be NaN)."""
+    re, im = a.reshape([4] * n), np.zeros([4] * n)
+    with np.errstate(invalid='ignore'):
+        for q in range(n):
+            (i, x, y, z), (ii, xi, yi, zi) = np.moveaxis(re, q, 0), np.moveaxis(im, q, 0)
+            re = np.moveaxis(np.stack([i + z, x + yi, x - yi, i - z]), 0, q)
+            im = np.moveaxis(np.stack([ii + zi, xi - y, xi + y, ii - zi]), 0, q)
+    order = [2 * j for j in range(n)] + [2 * j + 1 for j in range(n)]
+    return tuple(np.transpose(p.reshape([2] * (2 * n)), order).reshape(2 ** n, 2 ** n) for p in (re, im))
+
+
+@pytest.mark.parametrize('dtype', [N.DM_F64, N.DM_F32])
+@pytest.mark.parametrize('n', [1, 2, 5, 6, 7, 8, 9, 10])
+def test_matrix_of_infinities_and_nan(n, dtype):
+    """An entry's part is infinite or NaN only where a coefficient that it sums is."""
+    torch = _torch()
+    rng = np.random.default_rng(n)
+    for values in ([np.inf], [-np.inf], [np.nan], [np.inf, np.inf, -np.inf, np.nan], [np.nan] * 4 ** n):
+        a = _rand(n, dtype, n)
+        finite = np.abs(a).max()
+        a[rng.choice(4 ** n, size=min(len(values), 4 ** n), replace=False)] = values[:4 ** n]
+        t = _state(a, dtype, 1)
+        out = torch.empty((2 ** n, 2 ** n), dtype=torch.complex128, device='cuda')
+        scratch = torch.empty(N.lib().dm_pauli_to_matrix_scratch_bytes(n), dtype=torch.uint8, device='cuda')
+        N.call('dm_pauli_to_matrix', _vp(t), n, dtype, _vp(out), _vp(scratch), _stream())
+        got = out.cpu().numpy()
+        for g, w in zip((got.real, got.imag), _matrix_parts(a, n)):
+            np.testing.assert_allclose(g, w, rtol=0, atol=2 * EPS[N.DM_F64] * (n + 2) * 2 ** n * finite)
