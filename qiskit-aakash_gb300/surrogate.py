@@ -271,20 +271,30 @@ class MLPEnsemble:
         import torch
         S = feats.shape[0]
         out = torch.empty((self.M, S, self.nout), dtype=torch.float32, device=self.device)
-        net, work = self._net(), []
-        rows = self._predict_rows(S)
-        if rows > self.bufB:
+        net, work = self._net(), self._predict_work(S)
+        if work:
             n = net._obj
-            n.batch = rows
-            work = [torch.empty((m, rows, w), dtype=t, device=self.device)
-                    for m, w, t in ((1, 64, torch.int16), (self.M, 256, torch.int16), (self.M, 256, torch.int16),
-                                    (self.M, 256, torch.int16), (self.M, self.nout, torch.float32))]
+            n.batch = work[0].shape[1]
             n.x, n.logits = work[0].data_ptr(), work[4].data_ptr()
             n.h = (ctypes.c_void_p * 3)(*[b.data_ptr() for b in work[1:4]])
         vp = ctypes.c_void_p
         N.call('dm_mlp_predict', net, vp(feats.data_ptr()), N_FEATURES, ctypes.c_int64(S), vp(out.data_ptr()),
                self._stream())
         return out
+
+    def _predict_work(self, S):
+        """Activations of a prediction's passes (x, three layers, logits) where they are larger than a batch's;
+        None where a batch's buffers do, also when the device has no room for more."""
+        import torch
+        rows = self._predict_rows(S)
+        if rows <= self.bufB:
+            return None
+        try:
+            return [torch.empty((m, rows, w), dtype=t, device=self.device)
+                    for m, w, t in ((1, 64, torch.int16), (self.M, 256, torch.int16), (self.M, 256, torch.int16),
+                                    (self.M, 256, torch.int16), (self.M, self.nout, torch.float32))]
+        except torch.OutOfMemoryError:
+            return None
 
     def _predict_rows(self, S):
         """Points per pass through the network: the batch, or as many as PREDICT_WORKSPACE holds activations of,

@@ -292,3 +292,23 @@ def test_prediction_of_no_points(members):
     got = ens.predict(torch.empty((0, 6), device='cuda'))
     assert got.shape == (members, 0, 256) and got.dtype == torch.float32 and got.is_cuda
     assert N.lib().dm_mlp_predict(ens._net(), None, 6, ctypes.c_int64(1), None, None) == N.DM_ERR_ARG
+
+
+def test_predictions_where_no_workspace_fits():
+    """With room for the result alone, the passes run in a batch's buffers."""
+    torch = _torch()
+    ens = S.MLPEnsemble(members=2, batch=128, nout=1024, seed=5)
+    f = torch.rand(4000, 6, device='cuda', generator=torch.Generator('cuda').manual_seed(1)) * 2 - 1
+    want = ens.predict(f).cpu()
+    assert ens._predict_rows(4000) == 4096          # its workspace: 47 MB beside 33 MB of results
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    try:
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (48 << 20)) / total)
+        got = ens.predict(f)
+        with pytest.raises(torch.OutOfMemoryError):   # a result that does not fit is refused as ever
+            ens.predict(torch.rand(20000, 6, device='cuda'))
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert torch.equal(got.cpu(), want)
