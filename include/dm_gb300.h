@@ -38,7 +38,8 @@ enum dm_status {
     DM_ERR_ARG = -1,      /* invalid argument (qubit index, size, dtype, pointer) */
     DM_ERR_CUDA = -2,     /* a CUDA runtime call failed (launch, copy) */
     DM_ERR_RANGE = -3,    /* size beyond a documented limit */
-    DM_ERR_PROGRAM = -4   /* malformed fused-pass program */
+    DM_ERR_PROGRAM = -4,  /* malformed fused-pass program */
+    DM_ERR_MEMORY = -5    /* planning found no host memory */
 };
 
 /* Limits of the fused-pass kernel. */

@@ -24,7 +24,7 @@ ARCH = ['-gencode', 'arch=compute_103a,code=sm_103a']
 NVCC_FLAGS = ['-O3', '-std=c++17', '-lineinfo', '-Xcompiler', '-fPIC', '-Xptxas', '-warn-spills',
               '--expt-relaxed-constexpr']
 
-DM_OK, DM_ERR_ARG, DM_ERR_CUDA, DM_ERR_RANGE, DM_ERR_PROGRAM = 0, -1, -2, -3, -4
+DM_OK, DM_ERR_ARG, DM_ERR_CUDA, DM_ERR_RANGE, DM_ERR_PROGRAM, DM_ERR_MEMORY = 0, -1, -2, -3, -4, -5
 DM_F64, DM_F32 = 0, 1
 DM_MAX_QUBITS = 17
 DM_MAX_TILE_AXES = 7

@@ -155,6 +155,7 @@ extern "C" const char *dm_error_string(int code) {
         case DM_ERR_CUDA: return "CUDA runtime error";
         case DM_ERR_RANGE: return "size beyond a documented limit";
         case DM_ERR_PROGRAM: return "malformed fused-pass program";
+        case DM_ERR_MEMORY: return "out of host memory";
         default: return "unknown error";
     }
 }

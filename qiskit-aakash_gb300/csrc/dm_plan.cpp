@@ -20,6 +20,7 @@
 #include <stdint.h>
 #include <string.h>
 
+#include <exception>
 #include <vector>
 
 #include "dm_gb300.h"
@@ -142,10 +143,8 @@ bool compose(const dm_plan_op *ops, const double *const *data, const std::vector
     return true;
 }
 
-}  // namespace
-
-extern "C" int dm_plan_passes(int n, int kmax, int low, const dm_plan_op *ops, int count, int partial,
-                              int32_t *pass_of, int32_t *slot_of, uint32_t *resident, int32_t *npasses) {
+int plan(int n, int kmax, int low, const dm_plan_op *ops, int count, int partial, int32_t *pass_of, int32_t *slot_of,
+         uint32_t *resident, int32_t *npasses) {
     if (n < 1 || n > 30 || kmax < 0 || low < 0 || count < 0 || !npasses) return DM_ERR_ARG;
     if (count > 0 && (!ops || !pass_of || !slot_of || !resident)) return DM_ERR_ARG;
     if (!valid(ops, count, n)) return DM_ERR_ARG;
@@ -159,10 +158,9 @@ extern "C" int dm_plan_passes(int n, int kmax, int low, const dm_plan_op *ops, i
     return DM_OK;
 }
 
-extern "C" int dm_encode_passes(int n, int dtype, int width, int max_axes, const dm_plan_op *ops, int count,
-                                const double *coefs, const int32_t *pass_of, const int32_t *slot_of,
-                                const uint32_t *resident, int npasses, size_t mats_off, dm_pass *passes, void *mats,
-                                size_t mats_capacity, size_t *mats_used) {
+int encode(int n, int dtype, int width, int max_axes, const dm_plan_op *ops, int count, const double *coefs,
+           const int32_t *pass_of, const int32_t *slot_of, const uint32_t *resident, int npasses, size_t mats_off,
+           dm_pass *passes, void *mats, size_t mats_capacity, size_t *mats_used) {
     if (n < 1 || n > 30 || (dtype != DM_F32 && dtype != DM_F64) || count < 0 || npasses < 0 || !mats_used ||
         width < 0 || width > 4)
         return DM_ERR_ARG;
@@ -268,4 +266,31 @@ extern "C" int dm_encode_passes(int n, int dtype, int width, int max_axes, const
     }
     *mats_used = used;
     return DM_OK;
+}
+
+// No exception leaves the C entry points: what the standard library throws is memory it did not get.
+template <typename F>
+int guarded(F f) {
+    try {
+        return f();
+    } catch (const std::exception &) {
+        return DM_ERR_MEMORY;
+    }
+}
+
+}  // namespace
+
+extern "C" int dm_plan_passes(int n, int kmax, int low, const dm_plan_op *ops, int count, int partial,
+                              int32_t *pass_of, int32_t *slot_of, uint32_t *resident, int32_t *npasses) {
+    return guarded([&] { return plan(n, kmax, low, ops, count, partial, pass_of, slot_of, resident, npasses); });
+}
+
+extern "C" int dm_encode_passes(int n, int dtype, int width, int max_axes, const dm_plan_op *ops, int count,
+                                const double *coefs, const int32_t *pass_of, const int32_t *slot_of,
+                                const uint32_t *resident, int npasses, size_t mats_off, dm_pass *passes, void *mats,
+                                size_t mats_capacity, size_t *mats_used) {
+    return guarded([&] {
+        return encode(n, dtype, width, max_axes, ops, count, coefs, pass_of, slot_of, resident, npasses, mats_off, passes,
+                      mats, mats_capacity, mats_used);
+    });
 }

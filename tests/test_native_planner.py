@@ -1,6 +1,9 @@
 """The compiled planner against the same scan written over sets of axes, and its descriptors against program order."""
 import ctypes
 import importlib
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -158,3 +161,32 @@ def test_slots_that_no_scan_gives_are_refused(kinds, axes, slots, ok, width):
         P.encode_plan(plan, 2, np.float64, width, mats.ctypes.data, mats.size)
     assert e.value.code == N.DM_ERR_ARG
     assert (mats == 7.0).all()
+
+
+_NO_MEMORY = """
+import ctypes, importlib, resource
+import numpy as np
+N = importlib.import_module('qiskit-aakash_gb300._native')
+L, count = N.lib(), 1 << 21
+vp = lambda a: ctypes.c_void_p(a.ctypes.data)
+table = np.zeros((count, 4), np.int16)
+table[:, 0] = N.DM_OP_MAP1
+pass_of, slot_of, mats = np.zeros(count, np.int32), np.zeros(count, np.int32), np.zeros(16)
+resident, coefs, descs = np.ones(count, np.uint32), np.zeros((count, 16)), (N.DmPass * 1)()
+npasses, used = ctypes.c_int32(), ctypes.c_size_t()
+pages = int(open('/proc/self/statm').read().split()[0])
+limit = pages * resource.getpagesize() + (4 << 20)          # the calls' lists take 8 and 16 MB
+resource.setrlimit(resource.RLIMIT_AS, (limit, limit))
+print(L.dm_plan_passes(1, 1, 0, vp(table), count, 0, vp(pass_of), vp(slot_of), vp(resident), ctypes.byref(npasses)),
+      L.dm_encode_passes(1, N.DM_F64, 0, 6, vp(table), count, vp(coefs), vp(pass_of), vp(slot_of), vp(resident), 1, 0,
+                         ctypes.cast(descs, ctypes.c_void_p), vp(mats), 16, ctypes.byref(used)))
+"""
+
+
+@pytest.mark.skipif(not sys.platform.startswith('linux'), reason='limits its own address space')
+def test_no_memory_is_an_error_code():
+    """An allocation that fails in the planner comes back as a status, not as an exception through the C ABI."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(P.__file__)))
+    r = subprocess.run([sys.executable, '-c', _NO_MEMORY], cwd=root, capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stderr
+    assert r.stdout.split() == [str(N.DM_ERR_MEMORY)] * 2
