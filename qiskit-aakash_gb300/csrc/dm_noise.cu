@@ -14,7 +14,8 @@
 // from a table as the last sweep writes back.  That is n/4 + 1 FP64
 // operations per coefficient instead of n.  Defer needs c to stay small (the
 // unscaled Z grows like g**-n), so it is used for g >= 1/2, which every
-// physical decay factor per cycle is; below that each axis is scaled at once.
+// physical decay factor per cycle is; below that, and on a few qubits, each
+// axis is scaled at once.
 // Measured for all qubits: n = 13 FP64 672 us in three sweeps (6.8 ms as 13),
 // n = 14 FP32 1.32 ms in three (4.5 ms as 14, each at the HBM roof).
 #include <math.h>
@@ -29,11 +30,19 @@ constexpr int kThreads = 256;
 constexpr int kMaxLow = 6;         // axes of a sweep over the lowest axes: 16 / 32 KB tiles
 constexpr int kMaxHigh = 4;        // axes of a sweep above them: 256 rows of 16 contiguous elements and more
 constexpr int kMaxTile = 1 << (2 * kMaxLow);
+// Up to this many qubits each axis is scaled at once: the call is host time, and the table of factors (324
+// values, 2.6 KB of kernel parameters in FP64) is more of it than the few FP64 operations it saves.  One
+// qubit: 9.8 us a call with the table from 648 calls of pow, 4.1 with it from 2 n + 2, 3.3 without it.
+constexpr int kFewQubits = 4;
 
-template <typename T>
+template <typename T, bool Defer>
 struct Args {
-    T k, g, d, c;
-    T scale[DM_MAX_QUBITS + 1][DM_MAX_QUBITS + 1];   // Defer: k**a g**b for a X/Y and b Z digits
+    T k, g, d;
+};
+template <typename T>
+struct Args<T, true> {
+    T c;
+    T scale[DM_MAX_QUBITS + 1][DM_MAX_QUBITS + 1];   // k**a g**b for a X/Y and b Z digits
 };
 
 // Position of tile element e in shared memory: 16-byte chunks stay whole, the chunk index inside
@@ -53,8 +62,8 @@ __device__ __forceinline__ void count_digits(uint64_t i, int &xy, int &z) {
 
 // One axis of four coefficients
 template <typename T, bool Defer>
-__device__ __forceinline__ void axis(const Args<T> &a, T &x0, T &x1, T &x2, T &x3) {
-    if (Defer) {
+__device__ __forceinline__ void axis(const Args<T, Defer> &a, T &x0, T &x1, T &x2, T &x3) {
+    if constexpr (Defer) {
         x3 = fma(a.c, x0, x3);
     } else {
         x1 *= a.k;
@@ -70,7 +79,7 @@ __device__ __forceinline__ void axis(const Args<T> &a, T &x0, T &x1, T &x2, T &x
 // 16-byte access holds axis 0 whole, applied on load too.  Vec: 16-byte global accesses.
 template <typename T, bool Defer, bool Vec>
 __global__ void __launch_bounds__(kThreads) sweep_kernel(T *__restrict__ st, int K, int lo, int rlog, int last,
-                                                         const __grid_constant__ Args<T> a) {
+                                                         const __grid_constant__ Args<T, Defer> a) {
     __shared__ __align__(16) T tile[kMaxTile];
     __shared__ T scale[DM_MAX_QUBITS + 1][DM_MAX_QUBITS + 1];
     constexpr int V = Vec ? 16 / int(sizeof(T)) : 1;
@@ -84,10 +93,11 @@ __global__ void __launch_bounds__(kThreads) sweep_kernel(T *__restrict__ st, int
     const int64_t b = blockIdx.x;
     const int64_t base = ((b >> runs_log) << (2 * (lo + K))) + ((b & ((int64_t(1) << runs_log) - 1)) << rlog);
     auto offset = [&](int e) { return base + (int64_t(e >> rlog) << (2 * lo)) + (e & ((1 << rlog) - 1)); };
-    if (Defer && last)
-        for (int i = tid; i < (DM_MAX_QUBITS + 1) * (DM_MAX_QUBITS + 1); i += kThreads)
-            scale[i / (DM_MAX_QUBITS + 1)][i % (DM_MAX_QUBITS + 1)] =
-                a.scale[i / (DM_MAX_QUBITS + 1)][i % (DM_MAX_QUBITS + 1)];
+    if constexpr (Defer)
+        if (last)
+            for (int i = tid; i < (DM_MAX_QUBITS + 1) * (DM_MAX_QUBITS + 1); i += kThreads)
+                scale[i / (DM_MAX_QUBITS + 1)][i % (DM_MAX_QUBITS + 1)] =
+                    a.scale[i / (DM_MAX_QUBITS + 1)][i % (DM_MAX_QUBITS + 1)];
     // over the lowest axes a pack lies along axis 0: all of it in FP32, half of it in FP64
     const bool along = V > 1 && rlog == 0;
     const bool low_pack = V == 4 && along;
@@ -184,7 +194,7 @@ __global__ void __launch_bounds__(kThreads) sweep_kernel(T *__restrict__ st, int
 }
 
 template <typename T, bool Defer>
-static int run(T *st, int n, const Args<T> &a, cudaStream_t s) {
+static int run(T *st, int n, const Args<T, Defer> &a, cudaStream_t s) {
     const bool vec = (reinterpret_cast<uintptr_t>(st) & 15) == 0;
     // the fewest sweeps (kMaxLow axes in the first, kMaxHigh in each further one), the axes spread evenly
     const int sweeps = n <= kMaxLow ? 1 : 1 + (n - kMaxLow + kMaxHigh - 1) / kMaxHigh;
@@ -214,15 +224,16 @@ static int run(T *st, int n, const Args<T> &a, cudaStream_t s) {
 template <typename T>
 static int apply(T *st, int n, double f, double p, double g, cudaStream_t s) {
     const double k = sqrt(g) * f, d = (1 - g) * (2 * p - 1);
-    const bool defer = g >= 0.5 && fabs(d) <= g;
-    Args<T> a;
-    a.k = T(k);
-    a.g = T(g);
-    a.d = T(d);
-    a.c = defer ? T(d / g) : T(0);
-    for (int i = 0; i <= DM_MAX_QUBITS; ++i)
-        for (int j = 0; j <= DM_MAX_QUBITS; ++j) a.scale[i][j] = T(pow(k, i) * pow(g, j));
-    return defer ? run<T, true>(st, n, a, s) : run<T, false>(st, n, a, s);
+    if (n <= kFewQubits || !(g >= 0.5 && fabs(d) <= g)) return run<T, false>(st, n, {T(k), T(g), T(d)}, s);
+    Args<T, true> a{};
+    a.c = T(d / g);
+    double gp[DM_MAX_QUBITS + 1];
+    for (int j = 0; j <= n; ++j) gp[j] = pow(g, j);
+    for (int i = 0; i <= n; ++i) {
+        const double kp = pow(k, i);
+        for (int j = 0; i + j <= n; ++j) a.scale[i][j] = T(kp * gp[j]);
+    }
+    return run<T, true>(st, n, a, s);
 }
 
 }  // namespace noise

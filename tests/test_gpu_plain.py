@@ -185,3 +185,34 @@ def test_matrix_of_infinities_and_nan(n, dtype):
         got = out.cpu().numpy()
         for g, w in zip((got.real, got.imag), _matrix_parts(a, n)):
             np.testing.assert_allclose(g, w, rtol=0, atol=2 * EPS[N.DM_F64] * (n + 2) * 2 ** n * finite)
+
+
+@pytest.mark.parametrize('dtype', [N.DM_F64, N.DM_F32])
+@pytest.mark.parametrize('n', [1, 2, 3])
+def test_memory_noise_of_few_qubits_costs_no_more_than_its_maps(n, dtype):
+    """One call against the n one-qubit maps it stands for, host time included."""
+    import time
+    torch = _torch()
+    f, p, g = 0.97, 0.2, 0.93
+    k, d = np.sqrt(g) * f, (1 - g) * (2 * p - 1)
+    m = N.f64_array([1, 0, 0, 0, 0, k, 0, 0, 0, 0, k, 0, d, 0, 0, g])
+    t = _state(_rand(n, dtype, n), dtype)
+    s = _stream()
+
+    def noise():
+        N.call('dm_apply_memory_noise', _vp(t), n, dtype, f, p, g, s)
+
+    def maps():
+        for q in range(n):
+            N.call('dm_apply_map1', _vp(t), n, dtype, q, m, s)
+
+    best = {noise: np.inf, maps: np.inf}
+    for _ in range(20):
+        for call in best:
+            torch.cuda.synchronize()
+            t0 = time.perf_counter()
+            for _ in range(100):
+                call()
+            torch.cuda.synchronize()
+            best[call] = min(best[call], time.perf_counter() - t0)
+    assert best[noise] < 1.25 * best[maps]
