@@ -327,10 +327,12 @@ ROUND_MAX_AXES = {np.dtype(np.float32): 7, np.dtype(np.float64): 6}
 
 def _encode(plan, n, dtype_np, round_width, mats_off, mats_ptr, capacity):
     """(dm_pass descriptors, coefficients written) of a plan: dm_encode_passes."""
-    coefs = np.concatenate([op.data for op in plan.ops], axis=None).astype(np.float64, copy=False) \
-        if plan.ops else np.zeros(0)
-    if coefs.size != plan.coefficients():
-        raise ValueError('an operation holds %d coefficients more than its kind has' % (coefs.size - plan.coefficients()))
+    data = [np.asarray(op.data) for op in plan.ops]
+    expected = _OP_COEFFICIENTS[plan.table[::4]].tolist()
+    if [d.size for d in data] != expected:            # each: the errors of two could add up to nothing
+        i = next(i for i, d in enumerate(data) if d.size != expected[i])
+        raise ValueError('%r holds %d coefficients, not %d' % (plan.ops[i], data[i].size, expected[i]))
+    coefs = np.concatenate(data, axis=None).astype(np.float64, copy=False) if data else np.zeros(0)
     descs = (N.DmPass * len(plan.resident))()
     used = ctypes.c_size_t()
     dtype_np = np.dtype(dtype_np)

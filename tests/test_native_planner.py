@@ -163,6 +163,22 @@ def test_slots_that_no_scan_gives_are_refused(kinds, axes, slots, ok, width):
     assert (mats == 7.0).all()
 
 
+@pytest.mark.parametrize('data', [
+    [np.ones(4), np.ones(28)],                        # two maps whose lengths add up to two maps'
+    [np.eye(4), np.ones(17)], [np.eye(4), np.ones(15)]])
+def test_operations_of_the_wrong_length_are_refused(data):
+    plan = P.Plan([P.Op('map1', (q,), d) for q, d in enumerate(data)], 2, 2, 2)
+    mats = np.full(64, 7.0)
+    with pytest.raises(ValueError):
+        P.encode_plan(plan, 2, np.float64, None, mats.ctypes.data, mats.size)
+    cx = P.Op('cx', (0, 1), np.ones(16))
+    diag = P.Op('diag2', (0, 1), np.ones(5))          # 16 and 5 the wrong way round
+    with pytest.raises(ValueError):
+        P.encode_plan(P.Plan([cx, diag], 2, 2, 2), 2, np.float64, None, mats.ctypes.data, mats.size)
+    assert (mats == 7.0).all()
+    P.encode_plan(P.Plan([P.Op('map1', (0,), np.eye(4).tolist())], 2, 2, 2), 2, np.float64, None, mats.ctypes.data, 64)
+
+
 _NO_MEMORY = """
 import ctypes, importlib, resource
 import numpy as np
