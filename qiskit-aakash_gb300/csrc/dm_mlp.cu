@@ -484,7 +484,10 @@ __global__ void __launch_bounds__(256) adam_kernel(float *__restrict__ params, c
                                                    uint16_t *__restrict__ wb, uint16_t *__restrict__ wtb) {
     __shared__ uint16_t tr[32][33];
     grid_wait();
+    params = waited(params);      // restrict alone allows loads above the wait: an earlier step's are in it
     grads = waited(grads);
+    m = waited(m);
+    v = waited(v);
     auto rule = [&](float p, float gr, float &mm, float &vv) {
         mm = b1 * mm + (1.f - b1) * gr;
         vv = b2 * vv + (1.f - b2) * gr * gr;

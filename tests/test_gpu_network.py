@@ -312,3 +312,58 @@ def test_predictions_where_no_workspace_fits():
     finally:
         torch.cuda.set_per_process_memory_fraction(1.0)
     assert torch.equal(got.cpu(), want)
+
+
+@pytest.mark.parametrize('shift', [0, 1])
+@pytest.mark.parametrize('shapes', [[(5, 7), (33, 64), (64, 33), (300, 32), (1, 1)],
+                                    [(8, 4), (36, 64), (64, 36), (300, 32)]])
+def test_adam_steps_follow_the_rule(shapes, shift):
+    """Three steps in a row, a new gradient each, from moments that are not zero, against the rule in FP64;
+    with the state off 16-byte alignment (element by element) as well."""
+    torch = _torch()
+    P = sum(o * i + o for o, i in shapes)
+    Z = 2
+    rng = np.random.default_rng(3)
+
+    def place(a):
+        t = torch.zeros(a.size + 8, dtype=torch.float32, device='cuda')[shift:shift + a.size]
+        t.copy_(torch.from_numpy(a.reshape(-1)))
+        return t
+
+    lr, b1, b2, eps = (float(np.float32(x)) for x in (1e-2, 0.9, 0.999, 1e-8))
+    p = rng.normal(size=(Z, P)).astype(np.float32)
+    m = (0.3 * rng.normal(size=(Z, P))).astype(np.float32)
+    v = rng.uniform(0.01, 0.1, size=(Z, P)).astype(np.float32)
+    dp, dm, dv = place(p), place(m), place(v)
+    grads = [rng.normal(size=(Z, P)).astype(np.float32) for _ in range(3)]
+    dg = [place(g) for g in grads]
+    wb, wtb = (torch.zeros((Z, P), dtype=torch.int16, device='cuda') for _ in range(2))
+    flat = (ctypes.c_int32 * (2 * len(shapes)))(*[x for s in shapes for x in s])
+    vp = ctypes.c_void_p
+    for step in (1, 2, 3):
+        N.call('dm_mlp_adam', vp(dp.data_ptr()), vp(dg[step - 1].data_ptr()), vp(dm.data_ptr()), vp(dv.data_ptr()),
+               ctypes.c_int64(P), Z, flat, len(shapes), ctypes.c_float(lr), ctypes.c_float(b1), ctypes.c_float(b2),
+               ctypes.c_float(eps), step, vp(wb.data_ptr()), vp(wtb.data_ptr()), None)
+    # FP64, with a running bound of the FP32 roundings: three per moment, eight in the update, one on p
+    p, m, v = (a.astype(np.float64) for a in (p, m, v))
+    em, ev, ep = np.zeros_like(m), np.zeros_like(v), np.zeros_like(p)
+    for step, g in enumerate(grads, 1):
+        g = g.astype(np.float64)
+        em = b1 * em + 4 * U * (b1 * np.abs(m) + (1 - b1) * np.abs(g))
+        ev = b2 * ev + 4 * U * (b2 * v + (1 - b2) * g * g)
+        # 1 - beta in FP32 is exact to U of 1
+        em, ev = em + U * np.abs(g), ev + U * g * g
+        m, v = b1 * m + (1 - b1) * g, b2 * v + (1 - b2) * g * g
+        mh, vh = m / (1 - b1 ** step), np.sqrt(v / (1 - b2 ** step)) + eps
+        ep = ep + lr / vh * (em / (1 - b1 ** step) + np.abs(mh) * (0.5 * ev / v + 8 * U)) + U * (np.abs(p) + 1)
+        p = p - lr * mh / vh
+    for got, want, bound in ((dp, p, ep), (dm, m, em), (dv, v, ev)):
+        assert np.all(np.abs(got.cpu().numpy().reshape(Z, P) - want) <= 1.01 * bound)
+    off = 0
+    bits = (MO.bf16(dp.cpu().numpy().reshape(Z, P)).view(np.uint32) >> 16).astype(np.uint16).view(np.int16)
+    for o, i in shapes:
+        w = bits[:, off:off + o * i]
+        assert np.array_equal(wb[:, off:off + o * i].cpu().numpy(), w)
+        assert np.array_equal(wtb[:, off:off + o * i].cpu().numpy().reshape(Z, i, o),
+                              np.swapaxes(w.reshape(Z, o, i), 1, 2))
+        off += o * i + o
