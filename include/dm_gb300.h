@@ -309,14 +309,14 @@ typedef struct dm_batch_pass {
 
 /* The round images of one tensor-core pass, composed in FP64 on the device:
  * round r's 64x64 transfer matrix U (input and output index j = d0 + 4 d1
- * + 16 d2 over the round's local axes pass->round_axes[r][0..2]) is ops
- * [round_end[r-1], round_end[r]) applied to the 64 unit vectors, written at
- * images_dev + r * (values per round) as Uh = fp16(U) and
- * Ul = fp16(2**11 (U - Uh)) in the K-major core-matrix order the passes
- * read.  Op coefficients (moff in doubles) come from mats_dev; ops may be
+ * + 16 d2 over the round's local axes pass->round_axes[r][0..2]) is the
+ * product of the maps of ops [round_end[r-1], round_end[r]), the first one
+ * applied first, written at images_dev + r * (values per round) as
+ * Uh = fp16(U) and Ul = fp16(2**11 (U - Uh)) in the K-major core-matrix order
+ * the passes read.  Op coefficients (moff in doubles) come from mats_dev; ops may be
  * DM_OP_MAP1, DM_OP_MAP2, DM_OP_DIAG2 and DM_OP_CX, with their digit
  * positions in the flags as in the register rounds.  pass->k and
- * pass->axes are not read.  One launch of nrounds CTAs, stream-ordered
+ * pass->axes are not read.  One launch of 8 CTAs per round, stream-ordered
  * before the pass that reads the images.  The reference multiplies the
  * same per-gate maps one gate at a time on the host (dm_simulator.py:1005-1177);
  * here they are folded into one matrix per round. */
@@ -390,11 +390,13 @@ size_t dm_batch_tc_scratch_bytes(void);
 /* dm_batch_run for FP32 instances of 7..12 qubits with every pass on the
  * tensor cores (the dm_apply_pass_tc kernel): at the start of each pass a
  * CTA composes the pass's round matrices from the instance's FP64
- * coefficient block (the ops applied to the 64 unit vectors, in FP64) into
- * its slice of scratch_dev as the 3-way FP16 split images, then streams the
- * instance's tiles.  Large instances of an uneven batch, and batches too small
- * for the chip, run on several CTAs each (one or two launches).  status_dev is set to 1 if a bounded tensor-core wait
- * gives up. */
+ * coefficient block (as dm_compose_rounds, in FP64) into its slice of
+ * scratch_dev as the 3-way FP16 split images, then streams the instance's
+ * tiles.  Large instances of an uneven batch, and batches too small for the
+ * chip, run on several CTAs each (one or two launches).  Order the instances
+ * largest first (4**n x passes): the large ones are taken from the front of the
+ * list, and those behind a smaller one run on one CTA each.  status_dev is set
+ * to 1 if a bounded wait gives up. */
 int dm_batch_run_tc(float *states_dev, size_t states_count, double *probs_dev, size_t probs_count,
                     const double *mats_dev, size_t mats_count, const dm_batch_instance *insts_host,
                     const dm_batch_instance *insts_dev, int ninst, const dm_batch_tc_pass *passes_host,

@@ -12,15 +12,15 @@
 // memory so that global accesses are whole rows; it writes the row-major result
 // plus, where the next product needs it, its transpose, so that every later
 // product is again of the A B^T form with K contiguous.  Several independent
-// products of one epilogue can share a launch.  These products are small, 2.7
-// GFLOP at most, and bound by latencies: of a chunk's load, multiply and wait,
-// and of the epilogue's chains.  With 4 warps per CTA (64 columns and 64 tanhf a
-// thread), 16-byte cp.async loads and a wait per chunk the ten products of a
-// training step of 5 x 1,024 rows, 1,024 outcomes took 260 us; with TMA, stages
-// and the work spread over more warps the eight launches take 95 us (11 us for
-// 1,024 x 256 x 256, 13 us for 1,024 x 1,024 x 256).  The whole step went from
-// 402 to 150 us, the prediction of 10,233 points with the ensemble's spread from
-// 1,670 to 283 us.
+// products of one epilogue can share a launch.  A training step's products are
+// small, 2.7 GFLOP at most (a prediction's output layer has 27), and bound by
+// latencies: of a chunk's load, multiply and wait, and of the epilogue's chains.
+// With 4 warps per CTA (64 columns and 64 tanhf a thread), 16-byte cp.async
+// loads and a wait per chunk the ten products of a training step of 5 x 1,024
+// rows, 1,024 outcomes took 260 us; with TMA, stages and the work spread over
+// more warps the eight launches take 97 us (11 us for 1,024 x 256 x 256, 13 us
+// for 1,024 x 1,024 x 256).  The whole step went from 405 to 132 us, the
+// prediction of 10,233 points with the ensemble's spread from 1,640 to 283 us.
 // Waits on an mbarrier are bounded and record an error in *status.
 //
 // The other kernels are memory-light helpers: softmax with the KL loss and
@@ -82,7 +82,7 @@ struct GemmGroup {
     int count;
     int first[kMaxGroup + 1];                      // tiles before product i
     dm_mlp_gemm g[kMaxGroup];
-    CUtensorMap a[kMaxGroup], b[kMaxGroup];        // K x rows x members, boxes of 64 x 128 (A) and 64 x 64 (B)
+    CUtensorMap a[kMaxGroup], b[kMaxGroup];        // K x rows x members, boxes of 64 x 128 (A) and 64 x kBN (B)
 };
 
 // K-major operand of 128-byte rows with the 128-byte swizzle: 8 rows are 1024 bytes (the stride
@@ -625,12 +625,12 @@ __global__ void pack_kernel(const float *__restrict__ features, int nfeat, int64
         make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
 }
 
-// One CTA per row: every member's deviation is reduced within the warps, the CTA meets once, and one lane
-// per member adds its warps' sums (thread 0 alone over all of them was a chain of 48 shared-memory reads).
-// 5 members x 10,233 rows x 1,024 columns, 252 MB: 139 -> 75 us, with four columns per load 49 us.
 static bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-// Four columns per load where the rows are 16-byte aligned.
+// One CTA per row: every member's deviation is reduced within the warps, the CTA meets once, and one lane
+// per member adds its warps' sums (thread 0 alone over all of them was a chain of 48 shared-memory reads).
+// Four columns per load where the rows are 16-byte aligned.  5 members x 10,233 rows x 1,024 columns, 252 MB:
+// 139 -> 75 us, with four columns per load 49 us.
 template <int Members, bool Vec>
 __global__ void __launch_bounds__(kRowThreads) ensemble_kernel(const float *__restrict__ probs, int rows, int nout,
                                                                const float *__restrict__ ref, float *__restrict__ mean,
