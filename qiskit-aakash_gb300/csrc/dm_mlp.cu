@@ -257,7 +257,8 @@ __global__ void __launch_bounds__(Sh::kThreads, Sh::kPerSm) gemm_kernel(const __
 #pragma unroll
             for (int q = 0; q < kPre; ++q) {
                 const int i = tid + q * kThreads;
-                *reinterpret_cast<float4 *>(st + (i / kF4) * kF32Row + 4 * (i % kF4)) = early ? pre[early ? q : 0] : load_pre(q);
+                *reinterpret_cast<float4 *>(st + (i / kF4) * kF32Row + 4 * (i % kF4)) =
+                    early ? pre[early ? q : 0] : load_pre(q);
             }
             __syncthreads();
 #pragma unroll
@@ -341,8 +342,9 @@ __device__ __forceinline__ float slice_sum(const float (&part)[kSoftSlices]) {
 template <int Per>
 __global__ void __launch_bounds__(32 * kSoftRows, 2)
     softmax_kernel(const float *__restrict__ logits, const float *__restrict__ targets,
-                   const int32_t *__restrict__ index, int64_t samples, int rows, int nout, int64_t row_ms, int64_t out_ms, int64_t ld_t, float grad_scale, float *__restrict__ probs,
-                   uint16_t *__restrict__ dz, uint16_t *__restrict__ dzt, float *__restrict__ loss_rows) {
+                   const int32_t *__restrict__ index, int64_t samples, int rows, int nout, int64_t row_ms,
+                   int64_t out_ms, int64_t ld_t, float grad_scale, float *__restrict__ probs, uint16_t *__restrict__ dz,
+                   uint16_t *__restrict__ dzt, float *__restrict__ loss_rows) {
     __shared__ __align__(4) uint16_t tr[kRowThreads * kSoftStride];
     const int lane = threadIdx.x & 31, rl = threadIdx.x >> 5;
     const int64_t r0 = int64_t(blockIdx.x) * kSoftRows, r = r0 + rl, z = blockIdx.y;
@@ -421,16 +423,16 @@ __global__ void __launch_bounds__(32 * kSoftRows, 2)
     }
 }
 
-static int launch_softmax(const float *logits, const float *targets, const int32_t *index, int64_t samples, int rows, int members, int nout, int64_t row_ms,
-                          int64_t out_ms, int64_t ld_t, float grad_scale, float *probs, uint16_t *dz, uint16_t *dzt,
-                          float *loss_rows, cudaStream_t s) {
+static int launch_softmax(const float *logits, const float *targets, const int32_t *index, int64_t samples, int rows,
+                          int members, int nout, int64_t row_ms, int64_t out_ms, int64_t ld_t, float grad_scale,
+                          float *probs, uint16_t *dz, uint16_t *dzt, float *loss_rows, cudaStream_t s) {
     const dim3 grid((rows + kSoftRows - 1) / kSoftRows, members), block(32 * kSoftRows);
     auto kernel = nout == 256 ? softmax_kernel<1>
                 : nout == 512 ? softmax_kernel<2>
                 : nout == 768 ? softmax_kernel<3>
                 : nout == 1024 ? softmax_kernel<4> : softmax_kernel<0>;
-    return launch_early(kernel, grid, block, 0, s, logits, targets, index, samples, rows, nout, row_ms, out_ms, ld_t, grad_scale, probs,
-                        dz, dzt, loss_rows);
+    return launch_early(kernel, grid, block, 0, s, logits, targets, index, samples, rows, nout, row_ms, out_ms, ld_t,
+                        grad_scale, probs, dz, dzt, loss_rows);
 }
 
 // db[n] = sum_b d_t[n][b] for up to four layers: one warp per (layer, n, member)
@@ -818,8 +820,8 @@ extern "C" int dm_mlp_softmax_xent(const float *logits, const float *targets, in
     DM_CHECK_ARG(logits && rows > 0 && members >= 1 && members <= 65535 && nout > 0);
     DM_CHECK_ARG(nout % kRowThreads == 0 && nout <= 16 * kRowThreads);
     DM_CHECK_ARG(targets ? (dz && dzt) : (probs != nullptr));
-    return launch_softmax(logits, targets, nullptr, 0, rows, members, nout, rows, rows, rows, grad_scale, probs, dz, dzt, loss_rows,
-                          as_stream(stream));
+    return launch_softmax(logits, targets, nullptr, 0, rows, members, nout, rows, rows, rows, grad_scale, probs, dz, dzt,
+                          loss_rows, as_stream(stream));
 }
 
 extern "C" int dm_mlp_bias_grad(const uint16_t *d_t, int64_t ld, int64_t d_ms, int N, int rows, int members,
@@ -867,8 +869,9 @@ extern "C" int dm_mlp_adam(float *params, const float *grads, float *m, float *v
     bool vec = count_per_member % 4 == 0 && mlp::aligned16(params) && mlp::aligned16(grads) && mlp::aligned16(m) &&
                mlp::aligned16(v) && (reinterpret_cast<uintptr_t>(w_bf16) & 7) == 0;
     for (int l = 0; l < nlayers; ++l) vec = vec && L.w_off[l] % 4 == 0 && L.in[l] % 4 == 0;
-    return launch_early(vec ? mlp::adam_kernel<true> : mlp::adam_kernel<false>, grid, dim3(256), 0, as_stream(stream), params, grads, m, v, count_per_member, L, lr,
-                        beta1, beta2, eps, float(c1), float(c2), step, members, w_bf16, wt_bf16);
+    return launch_early(vec ? mlp::adam_kernel<true> : mlp::adam_kernel<false>, grid, dim3(256), 0, as_stream(stream),
+                        params, grads, m, v, count_per_member, L, lr, beta1, beta2, eps, float(c1), float(c2), step,
+                        members, w_bf16, wt_bf16);
 }
 
 extern "C" int dm_mlp_gather(const float *features, int nfeat, const float *targets, int nout, int64_t samples,
@@ -877,8 +880,8 @@ extern "C" int dm_mlp_gather(const float *features, int nfeat, const float *targ
     DM_CHECK_ARG(features && index && x && xt && nfeat > 0 && nfeat <= width && samples > 0);
     DM_CHECK_ARG(rows > 0 && members >= 1 && members <= 65535 && width % 8 == 0 && nout > 0 && nout % 4 == 0);
     DM_CHECK_ARG(!targets || (t && mlp::aligned16(targets) && mlp::aligned16(t)));
-    return launch_early(mlp::gather_kernel, dim3((rows + mlp::kGatherRows - 1) / mlp::kGatherRows, members), dim3(256), 0, as_stream(stream), features, nfeat, targets,
-                        nout, samples, index, rows, width, x, xt, t);
+    return launch_early(mlp::gather_kernel, dim3((rows + mlp::kGatherRows - 1) / mlp::kGatherRows, members), dim3(256), 0,
+                        as_stream(stream), features, nfeat, targets, nout, samples, index, rows, width, x, xt, t);
 }
 
 extern "C" int dm_mlp_ensemble(const float *probs, int rows, int members, int nout, const float *ref, float *mean,
@@ -1044,8 +1047,8 @@ static int loss_and_grads(const dm_mlp_net &n, int rows, const float *targets, c
                           cudaStream_t s) {
     int rc = forward(n, rows, true, int64_t(n.batch) * kInput, s);
     if (rc) return rc;
-    if ((rc = launch_softmax(n.logits, targets, index, samples, rows, n.members, n.nout, n.batch, n.batch, n.batch, float(1.0 / rows), n.probs,
-                             n.dz, n.dzt, n.loss_rows, s)))
+    if ((rc = launch_softmax(n.logits, targets, index, samples, rows, n.members, n.nout, n.batch, n.batch, n.batch,
+                             float(1.0 / rows), n.probs, n.dz, n.dzt, n.loss_rows, s)))
         return rc;
     return backward(n, rows, s);
 }

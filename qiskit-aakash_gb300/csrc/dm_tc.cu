@@ -74,7 +74,8 @@ struct Pass {
     int64_t nonres_stride[DM_MAX_QUBITS];
     alignas(16) uint32_t natrow[8];
     alignas(16) uint32_t natk[8];
-    alignas(16) int64_t lastg[14];               // direct: global element offsets of the last round's row bits 0-7, K bits 0-5
+    // direct: global element offsets of the last round's row bits 0-7, K bits 0-5
+    alignas(16) int64_t lastg[14];
     Round rounds[DM_MAX_ROUNDS];
 };
 
@@ -1493,8 +1494,8 @@ extern "C" int dm_batch_run_params_tc(const dm_param_program *host, const dm_par
         if (count == 0) continue;
         const int G = part ? tc::spread_group(ctas, count) : 1;
         const int e = launch_groups(
-            G > 1 ? tc::batch_param_tc_kernel<true> : tc::batch_param_tc_kernel<false>, G, ctas, counter_dev, scratch_dev, as_stream(stream),
-            states_dev + (int64_t(begin) << (2 * P.n)), probs_dev + (int64_t(begin) << P.n), *dev, passes_dev,
+            G > 1 ? tc::batch_param_tc_kernel<true> : tc::batch_param_tc_kernel<false>, G, ctas, counter_dev, scratch_dev,
+            as_stream(stream), states_dev + (int64_t(begin) << (2 * P.n)), probs_dev + (int64_t(begin) << P.n), *dev, passes_dev,
             params_dev + int64_t(begin) * params_stride, params_stride, count, counter_dev,
             static_cast<unsigned char *>(scratch_dev), ctas, G, status_dev);
         if (e) return e;

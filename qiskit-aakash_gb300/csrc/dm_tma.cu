@@ -569,8 +569,8 @@ extern "C" int dm_apply_pass_tma(void *state_dev, int n, const dm_tc_pass *pass,
     // long pass pays for: 84 passes on 16 qubits (1,725 tiles per SM) 882 ms early, 869 ms otherwise; 15 qubits
     // (431) 77.6 both ways; 14 qubits (108) 50.0 and 50.4 ms; 10 qubits 243 and 266 us.
     const bool early = p.ntiles <= int64_t(tma::kEarlyTiles) * sm_count();
-    return launch_early_if(early, tma::pass_tma_kernel, dim3(unsigned(grid)), dim3(tma::kThreads), tma::kSmemBytes, as_stream(stream),
-                        map, p, static_cast<float *>(state_dev), umats_dev, status_dev);
+    return launch_early_if(early, tma::pass_tma_kernel, dim3(unsigned(grid)), dim3(tma::kThreads), tma::kSmemBytes,
+                           as_stream(stream), map, p, static_cast<float *>(state_dev), umats_dev, status_dev);
 }
 
 // ---------------------------------------------------------------------------
